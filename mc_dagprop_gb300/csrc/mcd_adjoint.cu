@@ -180,7 +180,7 @@ static void (*forward_kernel(const KArgs &a))(const KArgs) {
 // The forward half over stages [a.stage_begin, a.stage_end).
 cudaError_t launch_adjoint_forward(const KArgs &a, cudaStream_t st) {
     if (a.n <= 0) return cudaSuccess;
-    const dim3 grid((unsigned)((a.n + kTile - 1) / kTile)), block((unsigned)(a.n_warps * 32));
+    const dim3 grid((unsigned)((a.n + kTile - 1) / kTile)), block((unsigned)(pick_warps(a, (int64_t)grid.x) * 32));
     const size_t smem = (size_t)a.smem_total;
     void (*fwd)(const KArgs) = a.win_smem ? forward_kernel<true>(a) : forward_kernel<false>(a);
     cudaError_t e = raise_smem_limit((const void *)fwd, smem);
@@ -192,7 +192,7 @@ cudaError_t launch_adjoint_forward(const KArgs &a, cudaStream_t st) {
 // The backward half over stages [a.stage_begin, a.stage_end), last stage first.
 cudaError_t launch_adjoint_backward(const KArgs &a, cudaStream_t st) {
     if (a.n <= 0) return cudaSuccess;
-    const dim3 grid((unsigned)((a.n + kTile - 1) / kTile)), block((unsigned)(a.n_warps * 32));
+    const dim3 grid((unsigned)((a.n + kTile - 1) / kTile)), block((unsigned)(pick_warps(a, (int64_t)grid.x) * 32));
     const size_t smem = (size_t)a.smem_total;
     void (*bwd)(const KArgs) = a.win_smem ? k_adjoint<true> : k_adjoint<false>;
     cudaError_t e = raise_smem_limit((const void *)bwd, smem);

@@ -37,6 +37,9 @@ namespace mcd {
 // keep the limit they were recorded with.
 cudaError_t raise_smem_limit(const void *fn, size_t smem);
 
+// Warps per CTA of a single-DAG launch over `tiles` tiles.
+int pick_warps(const KArgs &a, int64_t tiles);
+
 // ---------------------------------------------------------------- Philox4x32-10
 // Counter mode under one fixed key: the 128-bit counter is (seed low, seed high,
 // link, salt ^ attempt), so a draw depends only on (sample seed, link, attempt)
@@ -639,7 +642,7 @@ __device__ __forceinline__ bool propagate_tile(const KArgs &a, int64_t tile, dou
     TileCtx t;
     t.lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    const int NW = a.n_warps;
+    const int NW = blockDim.x >> 5;
     t.s = tile * kTile + t.lane;
     t.active = t.s < a.n;
     t.active_mask = __ballot_sync(0xFFFFFFFFu, t.active);

@@ -60,6 +60,7 @@ struct HostDag {
     bool positive = false;        // all times non-negative and finite
     int64_t max_preds = 0;        // largest predecessor list
     bool tables_in_smem = true;
+    int32_t max_units = 0;        // most work units of a stage (0: warps per CTA fixed by the caller)
     int32_t n_stages = 0, stage_bytes = 0;
     int32_t smem_stage_off = 0, smem_tables_off = 0, smem_bar_off = 0, smem_total = 0;
     std::vector<int32_t> stage_meta;  // kStageMetaInts ints per stage (KArgs::stage_meta)
