@@ -64,6 +64,9 @@ KArgs base_args(const mcd_dag *g) {
     a.aux = g->d_aux;
     a.dist = g->d_dist;
     a.vals = g->d_vals;
+    a.groups = g->d_groups;
+    a.draws = g->d_draws;
+    a.n_groups = (int32_t)g->h.groups.size();
     a.wk_off = g->d_wk;
     a.stage_meta = g->d_stage_meta;
     a.n_stages = g->h.n_stages;
@@ -365,10 +368,12 @@ void upload_image(DagImage &im) {
                  s_aux = align_up(h.aux.size() * sizeof(LinkRec), 256),
                  s_tables = align_up(tables_bytes(h), 256),
                  s_vals = align_up(h.vals.size() * sizeof(double), 256),
+                 s_groups = align_up(h.groups.size() * sizeof(DrawGroup), 256),
+                 s_draws = align_up(h.draws.size() * sizeof(DrawRec), 256),
                  s_wk = align_up(h.wk_off.size() * sizeof(int32_t), 256),
                  s_meta = align_up(h.stage_meta.size() * sizeof(int32_t), 256),
                  s_times = align_up(h.earliest.size() * sizeof(double), 256);
-    im.dbytes = s_ev + s_pred + s_aux + s_tables + s_vals + s_wk + s_meta + 2 * s_times;
+    im.dbytes = s_ev + s_pred + s_aux + s_tables + s_vals + s_groups + s_draws + s_wk + s_meta + 2 * s_times;
     cuda_check(cudaMalloc(&im.dmem, std::max<size_t>(im.dbytes, 256)), "compiled DAG allocation");
     char *p = im.dmem;
     auto place = [&](auto *&dst, const auto &vec, size_t sz) {
@@ -386,6 +391,8 @@ void upload_image(DagImage &im) {
         place(im.d_dist, tb, s_tables);
     }
     place(im.d_vals, h.vals, s_vals);
+    place(im.d_groups, h.groups, s_groups);
+    place(im.d_draws, h.draws, s_draws);
     place(im.d_wk, h.wk_off, s_wk);
     place(im.d_stage_meta, h.stage_meta, s_meta);
     place(im.d_earliest, h.earliest, s_times);

@@ -167,6 +167,32 @@ static void verify_layout(const HostDag &H) {
         pred_next = pfirst + npred;
     }
     if (ev_next != E || pred_next != P || val_next != (int64_t)H.vals.size()) fail("stage coverage");
+    // drawing groups: every link once, a group's words within its block, tables within vals
+    {
+        std::vector<char> drawn((size_t)H.L, 0);
+        int64_t next = 0;
+        for (size_t k = 0; k < H.groups.size(); ++k) {
+            const DrawGroup &q = H.groups[k];
+            if (q.first != next || q.n < 1 || q.n > kGroupLinks || (q.block >= 0) != ((int64_t)k < H.n_draw_groups))
+                fail("drawing groups");
+            next += q.n;
+            for (int32_t j = q.first; j < q.first + q.n; ++j) {
+                const DrawRec &r = H.draws[(size_t)j];
+                if (r.link < 0 || r.link >= H.L || drawn[(size_t)r.link] || H.link_block[(size_t)r.link] != q.block)
+                    fail("drawing record");
+                drawn[(size_t)r.link] = 1;
+                const int kind = r.kd & KD_KIND_MASK;
+                if ((kind == K_FIXED) != (q.block < 0)) fail("drawing kind");
+                if (kind == K_FIXED) continue;
+                if (r.kd >> 8 >= (int32_t)H.dist.size()) fail("drawing distribution");
+                const DistParam &dp = H.dist[(size_t)(r.kd >> 8)];
+                const int words = kind == K_GAMMA ? dp.erlang : 1;
+                if (((r.kd >> KD_WORD_SHIFT) & 3) + words > 4) fail("drawing words");
+                if (r.vt >= 0 && (int64_t)r.vt + dp.tab_n > (int64_t)H.vals.size()) fail("drawing table");
+            }
+        }
+        if (next != (int64_t)H.draws.size() || next != H.L) fail("drawing coverage");
+    }
     // sources and window slots, in execution order
     std::vector<int32_t> slot_of((size_t)E, -1), tenant((size_t)std::max(H.window_slots, 1), -1),
         last_read((size_t)std::max(H.window_slots, 1), -1);
@@ -765,6 +791,7 @@ void compile_dag(const mcd_dag_desc &d, const mcd_generator &g, HostDag &H, int3
         if ((int64_t)H.vals.size() - vbase > m[5]) throw McdError(MCD_ERR_RUNTIME, "value region overflow");
         while ((int64_t)H.vals.size() < vbase + m[5]) H.vals.push_back(0.0);
     };
+    std::vector<int32_t> link_vt((size_t)L, -1);  // a link's (first) duration table in vals
     int32_t group = -1, group_n = 0;  // the work unit's open Philox block of one-word links
     int32_t last_block = -1;          // block its last non-gamma random reference drew (in registers)
     for (int32_t i = 0; i < E; ++i) {
@@ -850,6 +877,7 @@ void compile_dag(const mcd_dag_desc &d, const mcd_generator &g, HostDag &H, int3
                     const int64_t local = (int64_t)H.vals.size() - vbase;
                     if (sm[1] >= 0) p.dvo = (int32_t)(sm[7] + local * (int64_t)sizeof(double));  // staged: byte offset
                     else p.dvo = kVtGlobal | (int32_t)(vbase + local);                           // index in vals
+                    if (link_vt[l] < 0) link_vt[l] = (int32_t)(vbase + local);
                     const std::vector<double> &vv = dist_values[di];
                     for (int32_t k = 0; k < nb; ++k)
                         H.vals.push_back(rel ? base + vv[(size_t)k] * base : base + vv[(size_t)k]);  // _core.cpp:140, 328
@@ -891,6 +919,47 @@ void compile_dag(const mcd_dag_desc &d, const mcd_generator &g, HostDag &H, int3
             else if ((kd & KD_KIND_MASK) != K_GAMMA) kd |= KD_TWO_WORD;
         }
         H.aux.push_back(LinkRec{l, kd, H.link_v[l]});
+    }
+    // ---- 13) the links by Philox block, for the kernel that draws durations alone:
+    // the same (block, word) of every link as the work units' draws
+    {
+        H.groups.clear();
+        H.draws.clear();
+        std::vector<int32_t> members((size_t)L, 0), at((size_t)L, -1);  // per block: links, its group
+        for (int32_t l = 0; l < L; ++l)
+            if (H.link_block[l] >= 0) ++members[(size_t)H.link_block[l]];
+        auto rec = [&](int32_t l) {
+            DrawRec r{};
+            r.link = l;
+            r.kd = H.link_kd[l];
+            if (H.link_word[l] >= 0) r.kd |= (int32_t)H.link_word[l] << KD_WORD_SHIFT;
+            else if ((r.kd & KD_KIND_MASK) != K_FIXED && (r.kd & KD_KIND_MASK) != K_GAMMA) r.kd |= KD_TWO_WORD;
+            r.v = H.link_v[l];
+            r.vt = link_vt[l];
+            return r;
+        };
+        int32_t n_rec = 0;
+        for (int32_t l = 0; l < L; ++l) {
+            const int32_t b = H.link_block[l];
+            if (b < 0 || at[(size_t)b] >= 0) continue;
+            at[(size_t)b] = (int32_t)H.groups.size();
+            H.groups.push_back(DrawGroup{b, n_rec, 0, 0});
+            n_rec += members[(size_t)b];
+        }
+        H.draws.resize((size_t)n_rec);
+        for (int32_t l = 0; l < L; ++l)
+            if (H.link_block[l] >= 0) {
+                DrawGroup &q = H.groups[(size_t)at[(size_t)H.link_block[l]]];
+                H.draws[(size_t)(q.first + q.n++)] = rec(l);
+            }
+        H.n_draw_groups = (int32_t)H.groups.size();
+        for (int32_t l = 0; l < L; ++l) {
+            if (H.link_block[l] >= 0) continue;
+            if ((int32_t)H.groups.size() == H.n_draw_groups || H.groups.back().n == kGroupLinks)
+                H.groups.push_back(DrawGroup{-1, (int32_t)H.draws.size(), 0, 0});
+            ++H.groups.back().n;
+            H.draws.push_back(rec(l));
+        }
     }
     // what the work units save: Philox blocks a sample's propagation draws
     H.n_pairs = 0;

@@ -205,17 +205,23 @@ static __device__ __forceinline__ double draw_gamma(const DistParam &p, double b
 // atoms and any last-bit difference would separate the two discrete
 // distributions: read from the link's own table (vt, kLinkTableBins) or, for
 // larger tables and links without one, evaluated here in FP64.
+__device__ __forceinline__ int pick_bin(const DistParam &p, const AliasPick *picks, uint32_t r, uint32_t r2,
+                                        bool two_word) {
+    const uint32_t j = __umulhi(r, (uint32_t)p.tab_n);
+    const uint32_t u = two_word ? r2 : r * (uint32_t)p.tab_n;
+    const AliasPick pk = picks[p.tab_off + j];
+    return u < pk.thresh ? (int)j : pk.alias;
+}
 __device__ __forceinline__ double draw_empirical(const DistParam &p, const AliasEntry *alias, const AliasPick *picks,
                                                  const double *vt, double base, bool relative, uint32_t r,
                                                  uint32_t r2, bool two_word, float &dfac) {
-    const uint32_t j = __umulhi(r, (uint32_t)p.tab_n);
-    const uint32_t u = two_word ? r2 : r * (uint32_t)p.tab_n;
     if (vt) {
-        const AliasPick pk = picks[p.tab_off + j];
-        const int k = u < pk.thresh ? (int)j : pk.alias;
+        const int k = pick_bin(p, picks, r, r2, two_word);
         dfac = relative ? 1.0f + (float)alias[p.tab_off + k].v_self : 1.0f;
         return vt[k];
     }
+    const uint32_t j = __umulhi(r, (uint32_t)p.tab_n);
+    const uint32_t u = two_word ? r2 : r * (uint32_t)p.tab_n;
     const AliasEntry &e = alias[p.tab_off + j];
     const double val = u < e.thresh ? e.v_self : e.v_alias;
     dfac = relative ? 1.0f + (float)val : 1.0f;

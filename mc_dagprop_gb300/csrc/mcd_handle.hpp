@@ -25,6 +25,8 @@ struct DagImage {
     LinkRec *d_aux = nullptr;
     DistParam *d_dist = nullptr;  // tables block: distributions, alias entries, alias picks
     double *d_vals = nullptr;
+    DrawGroup *d_groups = nullptr;
+    DrawRec *d_draws = nullptr;
     int32_t *d_wk = nullptr;
     int32_t *d_stage_meta = nullptr;
     double *d_earliest = nullptr;  // caller order, for the statistics finish
@@ -52,6 +54,8 @@ struct mcd_dag {
     const mcd::LinkRec *d_aux = nullptr;
     const mcd::DistParam *d_dist = nullptr;
     const double *d_vals = nullptr;
+    const mcd::DrawGroup *d_groups = nullptr;
+    const mcd::DrawRec *d_draws = nullptr;
     const int32_t *d_wk = nullptr;
     const int32_t *d_stage_meta = nullptr;
     const double *d_earliest = nullptr;
@@ -62,8 +66,9 @@ struct mcd_dag {
     int64_t last_adj_plan[3] = {0, 0, 0};  // the last gradient's samples per chunk, level blocks, buffer bytes
     explicit mcd_dag(std::shared_ptr<const mcd::DagImage> image)
         : img(std::move(image)), h(img->h), device(img->device), dbytes(img->dbytes), d_ev(img->d_ev),
-          d_pred(img->d_pred), d_aux(img->d_aux), d_dist(img->d_dist), d_vals(img->d_vals), d_wk(img->d_wk),
-          d_stage_meta(img->d_stage_meta), d_earliest(img->d_earliest), d_ub(img->d_ub) {}
+          d_pred(img->d_pred), d_aux(img->d_aux), d_dist(img->d_dist), d_vals(img->d_vals),
+          d_groups(img->d_groups), d_draws(img->d_draws), d_wk(img->d_wk), d_stage_meta(img->d_stage_meta),
+          d_earliest(img->d_earliest), d_ub(img->d_ub) {}
     mcd_dag(const mcd_dag &) = delete;
     mcd_dag &operator=(const mcd_dag &) = delete;
 };

@@ -67,6 +67,9 @@ struct HostDag {
     std::vector<EvRec> ev;
     std::vector<PredRec> pred;
     std::vector<LinkRec> aux;  // links stored by the aux pass
+    std::vector<DrawGroup> groups;  // the links by Philox block: drawing groups, then fixed links
+    std::vector<DrawRec> draws;
+    int32_t n_draw_groups = 0;
     int32_t n_orphan = 0;      // sampled links no precedence entry references
     int32_t n_pairs = 0;       // event pairs over all stages (KArgs::stage_meta)
     int64_t block_draws = 0;   // Philox blocks a sample draws on first attempts

@@ -103,6 +103,26 @@ struct alignas(16) LinkRec {
     double v;
 };
 
+// One link as a kernel that draws without propagating (k_delay_hist) sees it.  32 bytes.
+struct alignas(16) DrawRec {
+    int32_t link;  // link index; Philox key of the link's redraws
+    int32_t kd;    // kind, first word and distribution (KD_REUSE and KD_WRITE unused)
+    double v;      // FIXED: the duration; otherwise the base (minimal_duration)
+    int32_t vt;    // empirical kinds: the link's duration table as an index into KArgs::vals, -1 without one
+    int32_t pad[3];
+};
+
+// The links that draw from one Philox block, recs [first, first + n): at most
+// four (a block has four words).  Fixed links come in groups of four, block -1,
+// after all drawing groups.
+struct alignas(16) DrawGroup {
+    int32_t block;
+    int32_t first;
+    int32_t n;
+    int32_t pad;
+};
+constexpr int kGroupLinks = 4;
+
 // Per-distribution constants, single precision where the sampler works in FP32.
 struct alignas(16) DistParam {
     int32_t kind;
@@ -179,6 +199,9 @@ struct KArgs {
                                 //  first pred, preds, first value, values, byte offsets of the predecessor
                                 //  records and of the value region inside a staging buffer, event pairs, 0, 0, 0}
     const double *vals;         // per-link duration tables, stage by stage (value regions)
+    const DrawGroup *groups;    // the links by Philox block (single-DAG handles only)
+    const DrawRec *draws;
+    int32_t n_groups;
     int32_t n_stages;
     int32_t n_warps;
     int32_t max_units;        // most work units of a stage: the single-DAG launches choose their warps per
