@@ -40,18 +40,16 @@ def _links(activities, n_links: int):
         typ = np.asarray(activities["act_type"])
     else:
         acts = list(activities.values())
-        idx = np.array([a.idx for a in acts])
+        idx = np.array([a.idx for a in acts], dtype=None if acts else int)
         dur = np.array([a.minimal_duration for a in acts], float)
         typ = np.array([a.activity_type for a in acts])
-    types = sorted(set(int(t) for t in typ))
+    types, pos = np.unique(typ.astype(np.int64), return_inverse=True)
     cls = np.full(n_links, -1, np.int32)
     base = np.zeros(n_links)
-    pos = {t: i for i, t in enumerate(types)}
-    for i, d, t in zip(idx, dur, typ):
-        if 0 <= i < n_links:
-            cls[i] = pos[int(t)]
-            base[i] = d
-    return cls, base, types
+    ok = (idx >= 0) & (idx < n_links)  # (a link listed twice takes its last entry)
+    cls[idx[ok]] = pos[ok]
+    base[idx[ok]] = dur[ok]
+    return cls, base, types.tolist()
 
 
 def delay_histograms(propagator, activities, seeds, bins: int = 64, ranges: dict | None = None):
@@ -70,13 +68,16 @@ def delay_histograms(propagator, activities, seeds, bins: int = 64, ranges: dict
     missing = [c for c, t in enumerate(types) if not ranges or t not in ranges]
     if missing:
         _, dur, _ = propagator.run_many_arrays(seeds[:256])
+        # a class's extremes from its links' extremes: subtracting or dividing by a
+        # link's base is monotone, rounding included, so they are those of every delay
+        some = len(dur) > 0
+        d_lo, d_hi = (dur.min(axis=0) - base, dur.max(axis=0) - base) if some else (base, base)
         for c in missing:
             sel = cls == c
-            d = dur[:, sel] - base[sel]
-            b = base[sel]
-            rel = (d / np.where(b != 0.0, b, 1.0))[:, b != 0.0]
-            a_lo, a_hi = (float(d.min()), float(d.max())) if d.size else (0.0, 1.0)
-            r_lo, r_hi = (float(rel.min()), float(rel.max())) if rel.size else (0.0, 1.0)
+            a_lo, a_hi = (float(d_lo[sel].min()), float(d_hi[sel].max())) if some and sel.any() else (0.0, 1.0)
+            sel &= base != 0.0
+            ends = np.concatenate([d_lo[sel], d_hi[sel]]) / np.tile(base[sel], 2)
+            r_lo, r_hi = (float(ends.min()), float(ends.max())) if some and sel.any() else (0.0, 1.0)
             pad_a, pad_r = max(1e-9, 1e-6 * (a_hi - a_lo)), max(1e-9, 1e-6 * (r_hi - r_lo))
             rng[c] = (a_lo, a_hi + pad_a, r_lo, r_hi + pad_r)
     for c, t in enumerate(types):
