@@ -91,9 +91,10 @@ __global__ void __launch_bounds__(768) k_adjoint(const KArgs a) {
             const bool delayed = (code & kAdjDelayed) != 0u;
             uint32_t c = delayed ? 1u : 0u;
             if (WIN_SMEM) {
-                if (ev.slot >= 0) {  // read and clear: the slot's next tenant starts from zero
-                    c += cnt[ev.slot * kTile + lane];
-                    cnt[ev.slot * kTile + lane] = 0u;
+                const int32_t slot = window_row<1>(ev.slot);
+                if (slot >= 0) {  // read and clear: the slot's next tenant starts from zero
+                    c += cnt[slot * kTile + lane];
+                    cnt[slot * kTile + lane] = 0u;
                 }
             } else if (active) {
                 c += a.cnt_rows[(int64_t)row_off(ev.user, (uint32_t)a.ld) + s];
@@ -109,7 +110,8 @@ __global__ void __launch_bounds__(768) k_adjoint(const KArgs a) {
             if (wins) {
                 const PredRec pr = load_pred(spred + (ev.pred_begin - meta.z + (int)k));
                 if (WIN_SMEM) {
-                    if (pr.src_slot >= 0) atomicAdd(&cnt[pr.src_slot * kTile + lane], c);
+                    const int32_t slot = window_row<1>(pr.src_slot);
+                    if (slot >= 0) atomicAdd(&cnt[slot * kTile + lane], c);
                 } else {
                     atomicAdd(&a.cnt_rows[(int64_t)row_off(pr.src_user, (uint32_t)a.ld) + s], c);
                 }
@@ -138,13 +140,13 @@ __global__ void __launch_bounds__(768) k_adjoint(const KArgs a) {
 // off chip, predecessors come from (and realized times go to) the global rows
 // a.scratch[E][ld], which hold every event's time: a level block's recomputation
 // needs no other checkpoint.
-template <bool WIN_SMEM, bool POSITIVE, int TS>
+template <bool WIN_SMEM, bool POSITIVE, int TS, int S = 1>
 __global__ void __launch_bounds__(768) k_adjoint_forward(const KArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
-    propagate_tile<false, WIN_SMEM, false, POSITIVE, true, TS>(a, (int64_t)blockIdx.x, WIN_SMEM ? nullptr : a.scratch,
-                                                               a.ld, false, smem,
-                                                               reinterpret_cast<uint64_t *>(smem + a.smem_bar_off),
-                                                               false);
+    double *spill = S > 1 && a.spill ? a.spill + (int64_t)blockIdx.x * a.window_spill * (kTile * S) : nullptr;
+    propagate_tile<false, WIN_SMEM, false, POSITIVE, true, TS, true, S>(
+        a, (int64_t)blockIdx.x, WIN_SMEM ? nullptr : a.scratch, a.ld, false, smem,
+        reinterpret_cast<uint64_t *>(smem + a.smem_bar_off), false, spill);
 }
 
 // grad_earliest[e] = grad_e[e] / n, grad_base[l] = grad_l[l] 2^-20 / n, and the
@@ -180,6 +182,16 @@ static void (*forward_kernel(const KArgs &a))(const KArgs) {
 // The forward half over stages [a.stage_begin, a.stage_end).
 cudaError_t launch_adjoint_forward(const KArgs &a, cudaStream_t st) {
     if (a.n <= 0) return cudaSuccess;
+    // (level blocks start from window checkpoints, which are those of 32-sample tiles)
+    if (a.win_smem && !a.win_in && !a.win_ckpt && use_wide(a)) {
+        const KArgs w = wide_args(a);
+        const dim3 grid((unsigned)((a.n + kWideTile - 1) / kWideTile));
+        const cudaError_t e = raise_smem_limit((const void *)k_adjoint_forward<true, true, kTablesSmem, 2>, (size_t)w.smem_total);
+        if (e != cudaSuccess) return e;
+        k_adjoint_forward<true, true, kTablesSmem, 2>
+            <<<grid, (unsigned)(pick_warps(w, grid.x) * 32), (size_t)w.smem_total, st>>>(w);
+        return cudaGetLastError();
+    }
     const dim3 grid((unsigned)((a.n + kTile - 1) / kTile)), block((unsigned)(pick_warps(a, (int64_t)grid.x) * 32));
     const size_t smem = (size_t)a.smem_total;
     void (*fwd)(const KArgs) = a.win_smem ? forward_kernel<true>(a) : forward_kernel<false>(a);

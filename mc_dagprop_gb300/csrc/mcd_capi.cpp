@@ -64,9 +64,6 @@ KArgs base_args(const mcd_dag *g) {
     a.aux = g->d_aux;
     a.dist = g->d_dist;
     a.vals = g->d_vals;
-    a.groups = g->d_groups;
-    a.draws = g->d_draws;
-    a.n_groups = (int32_t)g->h.groups.size();
     a.wk_off = g->d_wk;
     a.stage_meta = g->d_stage_meta;
     a.n_stages = g->h.n_stages;
@@ -84,8 +81,40 @@ KArgs base_args(const mcd_dag *g) {
     a.smem_tables_off = g->h.smem_tables_off;
     a.smem_bar_off = g->h.smem_bar_off;
     a.smem_total = g->h.smem_total;
+    a.wide_rows = g->h.wide_rows;
+    a.window_spill = g->h.window_spill;
+    a.wide_stage_off = g->h.wide_stage_off;
+    a.wide_tables_off = g->h.wide_tables_off;
+    a.wide_bar_off = g->h.wide_bar_off;
+    a.wide_total = g->h.wide_total;
+    a.ev_spill = g->d_ev_spill;
     a.err = g->d_err;
     return a;
+}
+
+// (call_once runs again after an exception, so a failed allocation may be retried;
+// the image's device is the current one here)
+void image_draws(const mcd_dag *g, KArgs &a) {
+    const DagImage &im = *g->img;
+    std::call_once(im.draws_once, [&] {
+        std::vector<DrawGroup> groups;
+        std::vector<DrawRec> draws;
+        draw_groups(im.h, groups, draws);
+        const size_t s_groups = align_up(groups.size() * sizeof(DrawGroup), 256), s_draws = draws.size() * sizeof(DrawRec);
+        char *p = nullptr;
+        cuda_check(cudaMalloc(&p, std::max<size_t>(s_groups + s_draws, 256)), "drawing groups allocation");
+        cudaError_t e = cudaSuccess;
+        if (!groups.empty()) e = cudaMemcpy(p, groups.data(), groups.size() * sizeof(DrawGroup), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess && s_draws) e = cudaMemcpy(p + s_groups, draws.data(), s_draws, cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) cudaFree(p);
+        cuda_check(e, "drawing groups upload");
+        im.d_groups = reinterpret_cast<DrawGroup *>(p);
+        im.d_draws = reinterpret_cast<DrawRec *>(p + s_groups);
+        im.n_groups = (int32_t)groups.size();
+    });
+    a.groups = im.d_groups;
+    a.draws = im.d_draws;
+    a.n_groups = im.n_groups;
 }
 
 void check_device_error(mcd_dag *g) {
@@ -115,6 +144,7 @@ DagImage::~DagImage() {
     cudaGetDevice(&prev);
     cudaSetDevice(device);
     cudaFree(dmem);
+    if (d_groups) cudaFree(d_groups);
     cudaSetDevice(prev);
 }
 
@@ -368,12 +398,11 @@ void upload_image(DagImage &im) {
                  s_aux = align_up(h.aux.size() * sizeof(LinkRec), 256),
                  s_tables = align_up(tables_bytes(h), 256),
                  s_vals = align_up(h.vals.size() * sizeof(double), 256),
-                 s_groups = align_up(h.groups.size() * sizeof(DrawGroup), 256),
-                 s_draws = align_up(h.draws.size() * sizeof(DrawRec), 256),
+                 s_spill = align_up(h.ev_spill.size() * sizeof(int32_t), 256),
                  s_wk = align_up(h.wk_off.size() * sizeof(int32_t), 256),
                  s_meta = align_up(h.stage_meta.size() * sizeof(int32_t), 256),
                  s_times = align_up(h.earliest.size() * sizeof(double), 256);
-    im.dbytes = s_ev + s_pred + s_aux + s_tables + s_vals + s_groups + s_draws + s_wk + s_meta + 2 * s_times;
+    im.dbytes = s_ev + s_pred + s_aux + s_tables + s_vals + s_spill + s_wk + s_meta + 2 * s_times;
     cuda_check(cudaMalloc(&im.dmem, std::max<size_t>(im.dbytes, 256)), "compiled DAG allocation");
     char *p = im.dmem;
     auto place = [&](auto *&dst, const auto &vec, size_t sz) {
@@ -391,8 +420,7 @@ void upload_image(DagImage &im) {
         place(im.d_dist, tb, s_tables);
     }
     place(im.d_vals, h.vals, s_vals);
-    place(im.d_groups, h.groups, s_groups);
-    place(im.d_draws, h.draws, s_draws);
+    place(im.d_ev_spill, h.ev_spill, s_spill);
     place(im.d_wk, h.wk_off, s_wk);
     place(im.d_stage_meta, h.stage_meta, s_meta);
     place(im.d_earliest, h.earliest, s_times);
@@ -518,8 +546,10 @@ int mcd_dag_create_ex(const mcd_dag_desc *desc, const mcd_generator *gen, const 
         if (!img) {
             auto fresh = std::make_shared<DagImage>();
             compile_dag(*desc, *gen, fresh->h, nw, win);
+            auto verified = beside(fresh->h.E, [&h = fresh->h] { verify_layout(h); });
             cuda_check(cudaGetDevice(&fresh->device), "cudaGetDevice");
             upload_image(*fresh);
+            verified.get();
             if (!key.empty()) fresh->key = std::move(key);
             img = fresh;
             if (!img->key.empty()) cache_insert(hash, img);
@@ -602,6 +632,7 @@ int mcd_dag_describe(const mcd_dag_desc *desc, const mcd_generator *gen, mcd_dag
         if (!desc || !gen || !info) throw McdError(MCD_ERR_INVALID, "null argument");
         HostDag h;
         compile_dag(*desc, *gen, h, 0);
+        verify_layout(h);
         fill_info(h, info);
         info->device = -1;
         info->device_bytes = -1;
@@ -773,28 +804,44 @@ int mcd_propagate_host(mcd_dag *g, const double *durations, int64_t n, double *r
     });
 }
 
+// How a statistics run of n samples uses the handle's workspace beside the
+// accumulators: samples per launch, and the rows that do not fit on chip --
+// realized rows when the window is off chip (512 MiB of them a launch), or the
+// off-chip window rows of wide tiles (256 MiB a launch).
+struct StatsChunk {
+    int64_t C;
+    size_t rows_bytes, spill_bytes;
+};
+static StatsChunk stats_chunk(const HostDag &h, int64_t n) {
+    StatsChunk c{n, 0, 0};
+    if (!h.win_smem) {
+        const size_t row = std::max<size_t>((size_t)h.E * 8, 1);
+        c.C = std::max<int64_t>(32, std::min<int64_t>(n, (int64_t)((512ull << 20) / row) / 32 * 32));
+        c.rows_bytes = align_up((size_t)h.E * (size_t)c.C * 8, 256);
+    } else if (h.wide_rows > 0 && h.window_spill > 0) {
+        const size_t tile = (size_t)h.window_spill * kWideTile * sizeof(double);
+        c.C = std::min<int64_t>(n, (int64_t)((256ull << 20) / tile) * kWideTile);
+        c.spill_bytes = align_up((size_t)((c.C + kWideTile - 1) / kWideTile) * tile, 256);
+    }
+    return c;
+}
+
 // Statistics of n samples into device outputs, asynchronously on st.  The
-// handle's workspace holds the per-event accumulators (and, when the window is
-// not on chip, scratch realized rows for one chunk of samples at a time).
+// handle's workspace holds the per-event accumulators (and what stats_chunk says).
 static void stats_device(mcd_dag *g, const int64_t *seeds, int64_t seed0, int64_t n, const mcd_stats *out,
                          cudaStream_t st) {
     const HostDag &h = g->h;
     const size_t E = (size_t)h.E;
     const StatsParams sp = stats_params(h, n);
-    int64_t C = n;
-    size_t scratch_bytes = 0;
-    if (!h.win_smem) {
-        C = std::max<int64_t>(32, std::min<int64_t>(n, (int64_t)((512ull << 20) / std::max<size_t>(E * 8, 1)) / 32 * 32));
-        scratch_bytes = align_up(E * (size_t)C * 8, 256);
-    }
+    const StatsChunk ch = stats_chunk(h, n);
+    const int64_t C = ch.C;
     const size_t acc_bytes = align_up(E * 8, 256), hist_bytes = align_up(E * kHistStride * 4, 256),
                  te_bytes = align_up(E * 8, 256);
-    ensure_ws(g, acc_bytes + hist_bytes + te_bytes + scratch_bytes);
+    ensure_ws(g, acc_bytes + hist_bytes + te_bytes + ch.rows_bytes + ch.spill_bytes);
     auto *acc = reinterpret_cast<unsigned long long *>(g->ws);
     auto *hist = reinterpret_cast<uint32_t *>(g->ws + acc_bytes);
     auto *te = reinterpret_cast<long long *>(g->ws + acc_bytes + hist_bytes);
-    double *scratch =
-        scratch_bytes ? reinterpret_cast<double *>(g->ws + acc_bytes + hist_bytes + te_bytes) : nullptr;
+    auto *rows = reinterpret_cast<double *>(g->ws + acc_bytes + hist_bytes + te_bytes);
     cuda_check(cudaMemsetAsync(g->ws, 0, acc_bytes + hist_bytes, st), "accumulator reset");
     if (sp.fixed) cuda_check(launch_event_ticks(g->d_earliest, h.E, sp.q, te, st), "earliest ticks");
     for (int64_t off = 0; off < n; off += C) {
@@ -804,7 +851,8 @@ static void stats_device(mcd_dag *g, const int64_t *seeds, int64_t seed0, int64_
         a.seed0 = seed0 + off;
         a.n = m;
         a.ld = C;
-        a.scratch = scratch;
+        a.scratch = ch.rows_bytes ? rows : nullptr;
+        a.spill = ch.spill_bytes ? rows : nullptr;
         a.stats_fixed = sp.fixed;
         a.tick_q = sp.q;
         a.bin_mul = sp.bin_mul;
@@ -854,8 +902,8 @@ int mcd_stats_host(mcd_dag *g, const int64_t *seeds, int64_t seed0, int64_t n, c
         cudaStream_t st = g->stream[0];
         const size_t E = (size_t)g->h.E;
         // device copies of the seeds and the outputs live after every region
-        // stats_device carves (accumulators, histograms, earliest ticks, and the
-        // chunk scratch when the window is off chip), so none of them aliases
+        // stats_device carves (accumulators, histograms, earliest ticks, off-chip rows),
+        // so none of them aliases
         const size_t acc_bytes = align_up(E * 8, 256), hist_bytes = align_up(E * kHistStride * 4, 256),
                      te_bytes = align_up(E * 8, 256);
         const size_t seeds_bytes = seeds ? align_up((size_t)n * 8, 256) : 0;
@@ -863,12 +911,8 @@ int mcd_stats_host(mcd_dag *g, const int64_t *seeds, int64_t seed0, int64_t n, c
         const size_t hist_out = out->hist ? hist_bytes : 0;
         // reserve: [accumulators | hist | ticks | scratch] ... [outputs (5 x E doubles) | hist copy | seeds]
         const size_t head = 5 * out_bytes + hist_out + seeds_bytes;
-        size_t scratch_bytes = 0;
-        if (!g->h.win_smem) {
-            const int64_t C = std::max<int64_t>(32, std::min<int64_t>(n, (int64_t)((512ull << 20) / std::max<size_t>(E * 8, 1)) / 32 * 32));
-            scratch_bytes = align_up(E * (size_t)C * 8, 256);
-        }
-        ensure_ws(g, acc_bytes + hist_bytes + te_bytes + scratch_bytes + head);
+        const StatsChunk ch = stats_chunk(g->h, n);
+        ensure_ws(g, acc_bytes + hist_bytes + te_bytes + ch.rows_bytes + ch.spill_bytes + head);
         // stats_device carves its regions from the start of the workspace, so the
         // staging area goes at the end
         char *tail = g->ws + g->ws_bytes - head;

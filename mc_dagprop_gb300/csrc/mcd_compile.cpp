@@ -110,7 +110,7 @@ static void check_table(const DistSpec &d) {
 // after the stage of the last read of the previous tenant; and every KD_REUSE
 // reference naming the block its work unit drew last.  A violation is a
 // compiler defect and fails the compile rather than a launch.
-static void verify_layout(const HostDag &H) {
+void verify_layout(const HostDag &H) {
     auto fail = [](const char *what) {
         throw McdError(MCD_ERR_RUNTIME, std::string("internal layout check failed: ") + what);
     };
@@ -167,36 +167,26 @@ static void verify_layout(const HostDag &H) {
         pred_next = pfirst + npred;
     }
     if (ev_next != E || pred_next != P || val_next != (int64_t)H.vals.size()) fail("stage coverage");
-    // drawing groups: every link once, a group's words within its block, tables within vals
-    {
-        std::vector<char> drawn((size_t)H.L, 0);
-        int64_t next = 0;
-        for (size_t k = 0; k < H.groups.size(); ++k) {
-            const DrawGroup &q = H.groups[k];
-            if (q.first != next || q.n < 1 || q.n > kGroupLinks || (q.block >= 0) != ((int64_t)k < H.n_draw_groups))
-                fail("drawing groups");
-            next += q.n;
-            for (int32_t j = q.first; j < q.first + q.n; ++j) {
-                const DrawRec &r = H.draws[(size_t)j];
-                if (r.link < 0 || r.link >= H.L || drawn[(size_t)r.link] || H.link_block[(size_t)r.link] != q.block)
-                    fail("drawing record");
-                drawn[(size_t)r.link] = 1;
-                const int kind = r.kd & KD_KIND_MASK;
-                if ((kind == K_FIXED) != (q.block < 0)) fail("drawing kind");
-                if (kind == K_FIXED) continue;
-                if (r.kd >> 8 >= (int32_t)H.dist.size()) fail("drawing distribution");
-                const DistParam &dp = H.dist[(size_t)(r.kd >> 8)];
-                const int words = kind == K_GAMMA ? dp.erlang : 1;
-                if (((r.kd >> KD_WORD_SHIFT) & 3) + words > 4) fail("drawing words");
-                if (r.vt >= 0 && (int64_t)r.vt + dp.tab_n > (int64_t)H.vals.size()) fail("drawing table");
-            }
-        }
-        if (next != (int64_t)H.draws.size() || next != H.L) fail("drawing coverage");
+    // wide tiles: the layout, and (below) every source's row held by it when read
+    struct Rows {  // window rows: who holds each, and the stage of its last read
+        std::vector<int32_t> tenant, last_read;
+        explicit Rows(int32_t n) : tenant((size_t)std::max(n, 1), -1), last_read((size_t)std::max(n, 1), -1) {}
+    };
+    Rows wide(H.wide_rows), spill(H.window_spill);
+    if (H.wide_rows > 0) {
+        if (!H.win_smem || !H.positive || !H.tables_in_smem) fail("wide tiles");
+        if ((int64_t)H.wide_stage_off < (int64_t)H.wide_rows * kWideTile * 8 || H.wide_stage_off % 16 ||
+            H.wide_tables_off < (int64_t)H.wide_stage_off + 2 * (int64_t)H.stage_bytes || H.wide_tables_off % 16 ||
+            H.wide_bar_off < H.wide_tables_off + tables || H.wide_bar_off % 8 ||
+            H.wide_total < H.wide_bar_off + kBarRegionBytes || H.wide_total > (int64_t)kSmemMax)
+            fail("wide layout");
+        if (H.window_spill > 0 && (int64_t)H.ev_spill.size() != E) fail("off-chip rows");
     }
     // sources and window slots, in execution order
     std::vector<int32_t> slot_of((size_t)E, -1), tenant((size_t)std::max(H.window_slots, 1), -1),
         last_read((size_t)std::max(H.window_slots, 1), -1);
-    for (int64_t i = 0; i < E; ++i) slot_of[(size_t)H.ev[(size_t)i].user] = H.ev[(size_t)i].slot;
+    auto narrow_row = [](int32_t word) { return (int32_t)(int16_t)word; };
+    for (int64_t i = 0; i < E; ++i) slot_of[(size_t)H.ev[(size_t)i].user] = narrow_row(H.ev[(size_t)i].slot);
     for (int64_t st = 0, i = 0; st < NS; ++st) {
         const int64_t end = H.wk_off[(size_t)((st + 1) * NW)];
         const int32_t *sm = &H.stage_meta[(size_t)st * kStageMetaInts];
@@ -253,20 +243,183 @@ static void verify_layout(const HostDag &H) {
                     if (p.src_slot != -1) fail("window slot without a window");
                     continue;
                 }
-                if (p.src_slot < 0 || p.src_slot >= H.window_slots || p.src_slot != slot_of[(size_t)p.src_user] ||
-                    tenant[(size_t)p.src_slot] != p.src_user)
+                const int32_t sr = narrow_row(p.src_slot);
+                if (sr < 0 || sr >= H.window_slots || sr != slot_of[(size_t)p.src_user] ||
+                    tenant[(size_t)sr] != p.src_user)
                     fail("window slot of a source");
-                last_read[(size_t)p.src_slot] = std::max(last_read[(size_t)p.src_slot], (int32_t)st);
+                last_read[(size_t)sr] = std::max(last_read[(size_t)sr], (int32_t)st);
+                if (H.wide_rows > 0) {
+                    const int32_t w = p.src_slot >> 16, k = w >= 0 ? w : ~w;
+                    Rows &rows = w >= 0 ? wide : spill;
+                    if (k >= (w >= 0 ? H.wide_rows : H.window_spill) || rows.tenant[(size_t)k] != p.src_user)
+                        fail("wide row of a source");
+                    rows.last_read[(size_t)k] = std::max(rows.last_read[(size_t)k], (int32_t)st);
+                }
             }
-            if (r.slot >= 0) {
-                if (!H.win_smem || r.slot >= H.window_slots || last_read[(size_t)r.slot] >= st)
+            const int32_t er = narrow_row(r.slot);
+            if (er >= 0) {
+                if (!H.win_smem || er >= H.window_slots || last_read[(size_t)er] >= st)
                     fail("window slot reuse");
-                tenant[(size_t)r.slot] = r.user;
-            } else if (r.slot != -1) {
+                tenant[(size_t)er] = r.user;
+            } else if (er != -1) {
                 fail("window slot");
+            }
+            if (H.wide_rows > 0) {
+                const int32_t k[2] = {r.slot >> 16, H.window_spill > 0 ? H.ev_spill[(size_t)i] : -1};
+                Rows *rows[2] = {&wide, &spill};
+                const int32_t most[2] = {H.wide_rows, H.window_spill};
+                for (int j = 0; j < 2; ++j) {
+                    if (k[j] < -1 || k[j] >= most[j]) fail("wide row");
+                    if (k[j] < 0) continue;
+                    if (rows[j]->last_read[(size_t)k[j]] >= st) fail("wide row reuse");
+                    rows[j]->tenant[(size_t)k[j]] = r.user;
+                }
             }
         }
     }
+}
+
+// Least share of the window that must fit on chip for wide tiles.  At 0.5 (the
+// 200,000-event DAG) three quarters of the reads find their row there.
+constexpr double kMinWideShare = 0.4;
+
+// Deals the `fit` on-chip window rows of wide tiles out (compile_dag, step 11): ev_row
+// by caller index (-1: off chip from the start), src_row by predecessor entry in
+// compiled order (negative: ~ off-chip row), and the off-chip rows themselves.
+static bool plan_wide(const mcd_dag_desc &d, const std::vector<int64_t> &tstart, const std::vector<int64_t> &tlen,
+                      const std::vector<int32_t> &level, const std::vector<int32_t> &lvl_off,
+                      const std::vector<int32_t> &order, int32_t n_levels, int32_t fit, std::vector<int32_t> &ev_row,
+                      std::vector<int32_t> &src_row, HostDag &H) {
+    const size_t E = order.size();
+    constexpr int32_t kOff = -1;
+    struct Ev {                   // one cache line an access
+        int64_t next = 0, end = 0;  // reads not yet reached: levels rd[next, end), ascending
+        int32_t row = kOff;       // on-chip row now
+        int32_t busy = -1;        // last level that read or wrote the row
+        int32_t last_off = -1;    // last level with an off-chip read
+    };
+    std::vector<Ev> ev(E);
+    std::vector<int32_t> src;  // source of each entry in compiled order
+    for (int32_t e : order)
+        for (int64_t k = 0; k < tlen[e]; ++k) {
+            src.push_back(d.pred_src[tstart[e] + k]);
+            ++ev[(size_t)src.back()].end;
+        }
+    const size_t P = src.size();
+    int64_t sum = 0;
+    for (Ev &x : ev) {
+        const int64_t n = x.end;
+        x.next = x.end = sum;
+        sum += n;
+    }
+    std::vector<int32_t> rd(P);
+    {
+        size_t p = 0;
+        for (int32_t e : order)
+            for (int64_t k = 0; k < tlen[e]; ++k) rd[(size_t)ev[(size_t)src[p++]].end++] = level[e];
+    }
+    std::vector<int32_t> free_rows((size_t)fit), freed, touched, fresh;
+    for (int32_t k = 0; k < fit; ++k) free_rows[(size_t)k] = fit - 1 - k;
+    // events with a row, by the level of their next read (stale entries are dropped
+    // when met); far: no bucket above it holds any
+    std::vector<std::vector<int32_t>> at_level((size_t)n_levels + 1);
+    int32_t far = 0;
+    auto enter = [&](int32_t s) {
+        const int32_t l = rd[(size_t)ev[(size_t)s].next];
+        at_level[(size_t)l].push_back(s);
+        far = std::max(far, l);
+    };
+    ev_row.assign(E, kOff);
+    src_row.assign(P, kOff);
+    size_t at = 0;
+    for (int32_t l = 0; l < n_levels; ++l) {
+        freed.clear();
+        touched.clear();
+        fresh.clear();
+        for (int32_t i = lvl_off[l]; i < lvl_off[l + 1]; ++i) {  // the level's reads
+            const int32_t e = order[(size_t)i];
+            for (int64_t k = 0; k < tlen[e]; ++k, ++at) {
+                Ev &x = ev[(size_t)src[at]];
+                src_row[at] = x.row;
+                if (x.row < 0) x.last_off = l;
+                if (x.busy == l) continue;
+                x.busy = l;
+                touched.push_back(src[at]);
+            }
+            if (ev[(size_t)e].next < ev[(size_t)e].end) fresh.push_back(e);
+        }
+        for (int32_t s : touched) {
+            Ev &x = ev[(size_t)s];
+            while (x.next < x.end && rd[(size_t)x.next] <= l) ++x.next;
+            if (x.row < 0) continue;
+            if (x.next < x.end) {
+                enter(s);
+            } else {  // read for the last time: its row is free from the next level on
+                freed.push_back(x.row);
+                x.row = kOff;
+            }
+        }
+        // the level's events, those read soonest first
+        std::stable_sort(fresh.begin(), fresh.end(), [&](int32_t x, int32_t y) {
+            return rd[(size_t)ev[(size_t)x].next] < rd[(size_t)ev[(size_t)y].next];
+        });
+        int32_t scan = far;
+        size_t depth = 0;  // entries of bucket `scan` looked at
+        for (int32_t e : fresh) {
+            const int32_t first = rd[(size_t)ev[(size_t)e].next];
+            while (free_rows.empty() && scan > first) {  // the row read farthest ahead gives way
+                auto &bucket = at_level[(size_t)scan];
+                if (depth == bucket.size()) {
+                    if (scan == far && bucket.empty()) --far;
+                    --scan;
+                    depth = 0;
+                    continue;
+                }
+                const size_t k = bucket.size() - 1 - depth;
+                Ev &x = ev[(size_t)bucket[k]];
+                const bool stale = x.row < 0 || x.next == x.end || rd[(size_t)x.next] != scan;
+                if (!stale && x.busy == l) {  // read or written in this very level
+                    ++depth;
+                    continue;
+                }
+                bucket[k] = bucket.back();
+                bucket.pop_back();
+                if (stale) continue;
+                free_rows.push_back(x.row);
+                x.row = kOff;
+            }
+            ev[(size_t)e].busy = l;
+            if (free_rows.empty()) continue;
+            ev[(size_t)e].row = ev_row[(size_t)e] = free_rows.back();
+            free_rows.pop_back();
+        }
+        for (int32_t e : fresh)
+            if (ev[(size_t)e].row >= 0) enter(e);
+        at_level[(size_t)l].clear();
+        free_rows.insert(free_rows.end(), freed.begin(), freed.end());
+    }
+    // off-chip rows: from an event's level to its last off-chip read
+    std::vector<int32_t> spill(E, kOff), spare;
+    std::vector<std::vector<int32_t>> release((size_t)n_levels + 1);
+    int32_t n_spill = 0;
+    for (int32_t l = 0; l < n_levels; ++l) {
+        spare.insert(spare.end(), release[(size_t)l].begin(), release[(size_t)l].end());
+        for (int32_t i = lvl_off[l]; i < lvl_off[l + 1]; ++i) {
+            const size_t e = (size_t)order[(size_t)i];
+            if (ev[e].last_off < 0) continue;
+            if (spare.empty()) spare.push_back(n_spill++);
+            spill[e] = spare.back();
+            spare.pop_back();
+            release[(size_t)ev[e].last_off + 1].push_back(spill[e]);
+        }
+    }
+    if (n_spill > 0x7FFF || fit > 0x7FFF) return false;  // half words
+    for (size_t p = 0; p < P; ++p)
+        if (src_row[p] < 0) src_row[p] = ~spill[(size_t)src[p]];
+    H.ev_spill.resize(E);
+    for (size_t i = 0; i < E; ++i) H.ev_spill[i] = spill[(size_t)order[i]];
+    H.window_spill = n_spill;
+    return true;
 }
 
 void compile_dag(const mcd_dag_desc &d, const mcd_generator &g, HostDag &H, int32_t n_warps, int32_t window) {
@@ -290,7 +443,7 @@ void compile_dag(const mcd_dag_desc &d, const mcd_generator &g, HostDag &H, int3
     H.dist.clear();
     H.alias.clear();
     H.picks.clear();
-    std::unordered_map<int32_t, std::vector<double>> dist_values;  // empirical dists: values by bin
+    std::vector<std::vector<double>> dist_values;  // by distribution: an empirical one's values by bin
     for (const auto &kv : type_spec) {
         const DistSpec &s = g.dists[kv.second];
         TypeForm f{K_FIXED, -1, 0, 0.0, false};
@@ -373,7 +526,8 @@ void compile_dag(const mcd_dag_desc &d, const mcd_generator &g, HostDag &H, int3
                 build_alias(s.values, s.weights, H.alias, H.picks);
                 f.kind = p.kind;
                 f.dist = (int32_t)H.dist.size();
-                dist_values[f.dist] = s.values;
+                dist_values.resize((size_t)f.dist + 1);
+                dist_values[(size_t)f.dist] = s.values;
                 H.dist.push_back(p);
                 break;
             }
@@ -761,15 +915,45 @@ void compile_dag(const mcd_dag_desc &d, const mcd_generator &g, HostDag &H, int3
         if (off > kSmemMax) throw McdError(MCD_ERR_INVALID, "compiled DAG does not fit the shared-memory budget");
     }
 
+    // ---- 11) wide tiles: 64-sample window rows, as many as the same staging buffers
+    // leave room for.  When every slot's row fits, wide tiles use the slots above.
+    // Otherwise the rows on chip are dealt out level by level, an event whose next
+    // read lies farthest ahead giving way (Belady's rule); reads that find their row
+    // gone go to its off-chip row.
+    // The plan is made beside the records; their slot words take its rows at the end.
+    std::vector<int32_t> wide_ev(slot), wide_src;  // by caller index; by predecessor entry in compiled order
+    H.wide_rows = H.window_spill = 0;
+    H.ev_spill.clear();
+    const size_t wide_row = (size_t)kWideTile * sizeof(double);
+    const int32_t wide_fit = (int32_t)((kSmemMax - fixed_bytes - 2 * (size_t)H.stage_bytes) / wide_row);
+    const bool wide_tried = H.win_smem && H.tables_in_smem && n_warps != kBatchClassWarps && E > 0;
+    const bool wide_all = wide_tried && H.window_slots <= wide_fit;
+    std::future<bool> wide_plan;
+    if (wide_tried && !wide_all && wide_fit >= kMinWideShare * (double)H.window_slots)
+        wide_plan = beside(E, [&] {
+            return plan_wide(d, tstart, tlen, level, lvl_off, order, n_levels, wide_fit, wide_ev, wide_src, H);
+        });
+
     // ---- 9) records in compiled order
     H.ev.resize((size_t)E);
     H.pred.clear();
     H.pred.reserve((size_t)(d.n_targets > 0 ? d.pred_offsets[d.n_targets] : 0));
-    std::vector<char> referenced((size_t)L, 0), written((size_t)L, 0);
+    // what the records read and write of a link, side by side (its events' records are
+    // made in level order, far from link order)
+    struct Link {
+        double v;
+        int32_t kd, block, vt;
+        float dv;
+        int16_t bins;      // of its duration table, 0 without one
+        int8_t word, words;  // first word in its block, -1: owns it; words it takes of a shared block
+        bool referenced;
+    };
+    std::vector<Link> links((size_t)L);
+    for (int32_t l = 0; l < L; ++l)
+        links[(size_t)l] = Link{H.link_v[(size_t)l], H.link_kd[(size_t)l], -1, -1, H.link_dv[(size_t)l],
+                                (int16_t)table_bins(l), -1, (int8_t)link_words(l), false};
     // Philox blocks (see KD_REUSE): links drawing from a shared block group per
     // work unit, up to four words a block; the rest own one
-    H.link_block.assign((size_t)L, -1);
-    H.link_word.assign((size_t)L, -1);
     H.earliest.assign(d.earliest, d.earliest + E);
     H.ub.resize((size_t)E);
     H.max_delay = d.max_delay;
@@ -783,6 +967,9 @@ void compile_dag(const mcd_dag_desc &d, const mcd_generator &g, HostDag &H, int3
         H.max_span = std::max(H.max_span, H.ub[e] - d.earliest[e]);
     }
     H.vals.clear();
+    H.vals.reserve(H.n_stages > 0 ? (size_t)(H.stage_meta[(size_t)(H.n_stages - 1) * kStageMetaInts + 4] +
+                                             H.stage_meta[(size_t)(H.n_stages - 1) * kStageMetaInts + 5])
+                                  : 0);
     int32_t st_cur = -1;
     int64_t st_end = 0, vbase = 0;
     auto close_stage = [&]() {  // pad the stage's value region to its recorded (even) size
@@ -791,7 +978,6 @@ void compile_dag(const mcd_dag_desc &d, const mcd_generator &g, HostDag &H, int3
         if ((int64_t)H.vals.size() - vbase > m[5]) throw McdError(MCD_ERR_RUNTIME, "value region overflow");
         while ((int64_t)H.vals.size() < vbase + m[5]) H.vals.push_back(0.0);
     };
-    std::vector<int32_t> link_vt((size_t)L, -1);  // a link's (first) duration table in vals
     int32_t group = -1, group_n = 0;  // the work unit's open Philox block of one-word links
     int32_t last_block = -1;          // block its last non-gamma random reference drew (in registers)
     for (int32_t i = 0; i < E; ++i) {
@@ -815,7 +1001,7 @@ void compile_dag(const mcd_dag_desc &d, const mcd_generator &g, HostDag &H, int3
         }
         EvRec r{};
         r.user = e;
-        r.slot = H.win_smem ? slot[e] : -1;
+        r.slot = H.win_smem ? slot_word(slot[e], slot[e]) : -1;
         r.pred_begin = (int32_t)H.pred.size();
         const double earliest = d.earliest[e];
         const double ub = earliest + d.max_delay;  // _core.cpp:334
@@ -827,7 +1013,7 @@ void compile_dag(const mcd_dag_desc &d, const mcd_generator &g, HostDag &H, int3
             const int32_t src = d.pred_src[tstart[e] + k];
             const int32_t l = d.pred_act[tstart[e] + k];
             PredRec p{};
-            p.src_slot = H.win_smem ? slot[src] : -1;
+            p.src_slot = H.win_smem ? slot_word(slot[src], slot[src]) : -1;
             p.src_user = src;
             if (l >= L) {
                 // Past the last link the reference reads beyond its duration
@@ -839,54 +1025,52 @@ void compile_dag(const mcd_dag_desc &d, const mcd_generator &g, HostDag &H, int3
                 p.v = 0.0;
                 p.dvo = float_bits(0.0f);
             } else {
+                Link &k_ = links[(size_t)l];
+                const int kind = k_.kd & KD_KIND_MASK;
                 p.link = l;
-                p.kd = H.link_kd[l];
-                p.v = H.link_v[l];
-                p.dvo = float_bits(H.link_dv[l]);
+                p.kd = k_.kd;
+                p.v = k_.v;
+                p.dvo = float_bits(k_.dv);
                 p.block = -1;
-                if ((H.link_kd[l] & KD_KIND_MASK) != K_FIXED) {
-                    const int32_t nw = link_words(l);
-                    if (H.link_block[l] < 0) {  // first reference: the link's block and first word
+                if (kind != K_FIXED) {
+                    const int32_t nw = k_.words;
+                    if (k_.block < 0) {  // first reference: the link's block and first word
                         if (nw > 0) {
                             if (group < 0 || group_n + nw > 4) {
                                 group = l;
                                 group_n = 0;
                             }
-                            H.link_block[l] = group;
-                            H.link_word[l] = (int8_t)group_n;
+                            k_.block = group;
+                            k_.word = (int8_t)group_n;
                             group_n += nw;
                         } else {
-                            H.link_block[l] = l;
+                            k_.block = l;
                         }
                     }
-                    p.block = H.link_block[l];
-                    const bool mt_gamma = (H.link_kd[l] & KD_KIND_MASK) == K_GAMMA && nw == 0;
+                    p.block = k_.block;
+                    const bool mt_gamma = kind == K_GAMMA && nw == 0;
                     if (!mt_gamma) {  // draws into the shared registers
-                        if (nw > 0) p.kd |= (int32_t)H.link_word[l] << KD_WORD_SHIFT;
+                        if (nw > 0) p.kd |= (int32_t)k_.word << KD_WORD_SHIFT;
                         else p.kd |= KD_TWO_WORD;
                         if (p.block == last_block) p.kd |= KD_REUSE;
                         last_block = p.block;
                     }
+                    p.dvo = -1;
                 }
-                if ((H.link_kd[l] & KD_KIND_MASK) != K_FIXED) p.dvo = -1;
-                if (const int32_t nb = table_bins(l)) {  // the link's duration table, bin by bin
-                    const int32_t di = H.link_kd[l] >> 8;
-                    const bool rel = (H.link_kd[l] & KD_KIND_MASK) == K_EMP_REL;
-                    const double base = H.link_v[l];
+                if (const int32_t nb = k_.bins) {  // the link's duration table, bin by bin
+                    const bool rel = kind == K_EMP_REL;
+                    const double base = k_.v;
                     const int32_t *sm = &H.stage_meta[(size_t)st_cur * kStageMetaInts];
                     const int64_t local = (int64_t)H.vals.size() - vbase;
                     if (sm[1] >= 0) p.dvo = (int32_t)(sm[7] + local * (int64_t)sizeof(double));  // staged: byte offset
                     else p.dvo = kVtGlobal | (int32_t)(vbase + local);                           // index in vals
-                    if (link_vt[l] < 0) link_vt[l] = (int32_t)(vbase + local);
-                    const std::vector<double> &vv = dist_values[di];
+                    if (k_.vt < 0) k_.vt = (int32_t)(vbase + local);
+                    const double *vv = dist_values[(size_t)(k_.kd >> 8)].data();
                     for (int32_t k = 0; k < nb; ++k)
-                        H.vals.push_back(rel ? base + vv[(size_t)k] * base : base + vv[(size_t)k]);  // _core.cpp:140, 328
+                        H.vals.push_back(rel ? base + vv[k] * base : base + vv[k]);  // _core.cpp:140, 328
                 }
-                if (!written[l]) {  // the first reference stores the link's duration row
-                    p.kd |= KD_WRITE;
-                    written[l] = 1;
-                }
-                referenced[l] = 1;
+                if (!k_.referenced) p.kd |= KD_WRITE;  // the first reference stores the link's duration row
+                k_.referenced = true;
             }
             H.pred.push_back(p);
         }
@@ -894,6 +1078,30 @@ void compile_dag(const mcd_dag_desc &d, const mcd_generator &g, HostDag &H, int3
         H.ev[i] = r;
     }
     close_stage();
+    if (wide_all) H.wide_rows = std::max(H.window_slots, 1);
+    if (wide_plan.valid() && wide_plan.get()) {
+        H.wide_rows = wide_fit;
+        for (int32_t i = 0; i < E; ++i) H.ev[(size_t)i].slot = slot_word(H.ev[(size_t)i].slot, wide_ev[(size_t)order[(size_t)i]]);
+        for (size_t k = 0; k < H.pred.size(); ++k) H.pred[k].src_slot = slot_word(H.pred[k].src_slot, wide_src[k]);
+    }
+    if (H.wide_rows > 0) {
+        size_t off = ((size_t)H.wide_rows * wide_row + 127) / 128 * 128;
+        H.wide_stage_off = (int32_t)off;
+        off = (off + 2 * (size_t)H.stage_bytes + 127) / 128 * 128;
+        H.wide_tables_off = (int32_t)off;
+        off = (off + table_bytes + 15) / 16 * 16;
+        H.wide_bar_off = (int32_t)off;
+        H.wide_total = (int32_t)(off + kBarRegionBytes);
+        if ((size_t)H.wide_total > kSmemMax) H.wide_rows = 0;
+    }
+    H.link_block.resize((size_t)L);
+    H.link_word.resize((size_t)L);
+    H.link_vt.resize((size_t)L);
+    for (int32_t l = 0; l < L; ++l) {
+        H.link_block[(size_t)l] = links[(size_t)l].block;
+        H.link_word[(size_t)l] = links[(size_t)l].word;
+        H.link_vt[(size_t)l] = links[(size_t)l].vt;
+    }
     // ---- 12) positive mode: every earliest, bound and duration is a non-negative
     // finite double, so t = src + dur never is NaN or negative and the raw bit
     // patterns order like the values
@@ -905,12 +1113,13 @@ void compile_dag(const mcd_dag_desc &d, const mcd_generator &g, HostDag &H, int3
         for (const AliasEntry &ae : H.alias) pos = pos && nonneg(ae.v_self) && nonneg(ae.v_alias) && ae.v_self < 1e300;
         for (double x : H.vals) pos = pos && nonneg(x);
         H.positive = pos;
+        if (!pos) H.wide_rows = 0;
     }
     H.aux.clear();
     H.n_orphan = 0;
     for (int32_t l = 0; l < L; ++l) {
-        if (!referenced[l]) ++H.n_orphan;
-        if (written[l]) continue;
+        if (links[(size_t)l].referenced) continue;
+        ++H.n_orphan;
         // an unreferenced random link owns its block (word 0)
         int32_t kd = H.link_kd[l];
         if ((kd & KD_KIND_MASK) != K_FIXED) {
@@ -919,47 +1128,6 @@ void compile_dag(const mcd_dag_desc &d, const mcd_generator &g, HostDag &H, int3
             else if ((kd & KD_KIND_MASK) != K_GAMMA) kd |= KD_TWO_WORD;
         }
         H.aux.push_back(LinkRec{l, kd, H.link_v[l]});
-    }
-    // ---- 13) the links by Philox block, for the kernel that draws durations alone:
-    // the same (block, word) of every link as the work units' draws
-    {
-        H.groups.clear();
-        H.draws.clear();
-        std::vector<int32_t> members((size_t)L, 0), at((size_t)L, -1);  // per block: links, its group
-        for (int32_t l = 0; l < L; ++l)
-            if (H.link_block[l] >= 0) ++members[(size_t)H.link_block[l]];
-        auto rec = [&](int32_t l) {
-            DrawRec r{};
-            r.link = l;
-            r.kd = H.link_kd[l];
-            if (H.link_word[l] >= 0) r.kd |= (int32_t)H.link_word[l] << KD_WORD_SHIFT;
-            else if ((r.kd & KD_KIND_MASK) != K_FIXED && (r.kd & KD_KIND_MASK) != K_GAMMA) r.kd |= KD_TWO_WORD;
-            r.v = H.link_v[l];
-            r.vt = link_vt[l];
-            return r;
-        };
-        int32_t n_rec = 0;
-        for (int32_t l = 0; l < L; ++l) {
-            const int32_t b = H.link_block[l];
-            if (b < 0 || at[(size_t)b] >= 0) continue;
-            at[(size_t)b] = (int32_t)H.groups.size();
-            H.groups.push_back(DrawGroup{b, n_rec, 0, 0});
-            n_rec += members[(size_t)b];
-        }
-        H.draws.resize((size_t)n_rec);
-        for (int32_t l = 0; l < L; ++l)
-            if (H.link_block[l] >= 0) {
-                DrawGroup &q = H.groups[(size_t)at[(size_t)H.link_block[l]]];
-                H.draws[(size_t)(q.first + q.n++)] = rec(l);
-            }
-        H.n_draw_groups = (int32_t)H.groups.size();
-        for (int32_t l = 0; l < L; ++l) {
-            if (H.link_block[l] >= 0) continue;
-            if ((int32_t)H.groups.size() == H.n_draw_groups || H.groups.back().n == kGroupLinks)
-                H.groups.push_back(DrawGroup{-1, (int32_t)H.draws.size(), 0, 0});
-            ++H.groups.back().n;
-            H.draws.push_back(rec(l));
-        }
     }
     // what the work units save: Philox blocks a sample's propagation draws
     H.n_pairs = 0;
@@ -973,7 +1141,73 @@ void compile_dag(const mcd_dag_desc &d, const mcd_generator &g, HostDag &H, int3
     H.block_draws = 0;
     for (const PredRec &p : H.pred)
         if ((p.kd & KD_KIND_MASK) != K_FIXED && !(p.kd & KD_REUSE)) ++H.block_draws;
-    verify_layout(H);
+}
+
+// The links by Philox block, for a kernel that draws durations without propagating:
+// the same (block, word) of every link as the work units' draws.  Drawing groups
+// first, then the fixed links in groups of their own.
+void draw_groups(const HostDag &H, std::vector<DrawGroup> &groups, std::vector<DrawRec> &draws) {
+    const int32_t L = H.L;
+    groups.clear();
+    std::vector<int32_t> at((size_t)L, -1);  // per block: its group
+    auto member = [&](int32_t l) -> DrawGroup * {
+        const int32_t b = H.link_block[(size_t)l];
+        if (b < 0) return nullptr;
+        if (at[(size_t)b] < 0) {
+            at[(size_t)b] = (int32_t)groups.size();
+            groups.push_back(DrawGroup{b, 0, 0, 0});
+        }
+        return &groups[(size_t)at[(size_t)b]];
+    };
+    for (int32_t l = 0; l < L; ++l)
+        if (DrawGroup *q = member(l)) ++q->n;
+    int32_t n_rec = 0;
+    for (DrawGroup &q : groups) {
+        q.first = n_rec;
+        n_rec += q.n;
+        q.n = 0;
+    }
+    const size_t drawing = groups.size();
+    draws.assign((size_t)L, DrawRec{});
+    for (int32_t l = 0; l < L; ++l) {
+        DrawRec r{};
+        r.link = l;
+        r.kd = H.link_kd[(size_t)l];
+        r.v = H.link_v[(size_t)l];
+        r.vt = H.link_vt[(size_t)l];
+        const int kind = r.kd & KD_KIND_MASK;
+        if (kind != K_FIXED && H.link_word[(size_t)l] >= 0) r.kd |= (int32_t)H.link_word[(size_t)l] << KD_WORD_SHIFT;
+        else if (kind != K_FIXED && kind != K_GAMMA) r.kd |= KD_TWO_WORD;
+        DrawGroup *q = member(l);
+        if (!q) {
+            if (groups.size() == drawing || groups.back().n == kGroupLinks) groups.push_back(DrawGroup{-1, n_rec, 0, 0});
+            q = &groups.back();
+            ++n_rec;
+        }
+        draws[(size_t)(q->first + q->n++)] = r;
+    }
+    // what the kernel's accesses rely on: every link once, at most four to a group,
+    // words within the block, tables within vals
+    auto fail = [](const char *what) {
+        throw McdError(MCD_ERR_RUNTIME, std::string("internal layout check failed: ") + what);
+    };
+    int64_t next = 0;
+    for (size_t k = 0; k < groups.size(); ++k) {
+        const DrawGroup &q = groups[k];
+        if (q.first != next || q.n < 1 || q.n > kGroupLinks || (q.block >= 0) != (k < drawing)) fail("drawing groups");
+        next += q.n;
+        for (int32_t j = q.first; j < q.first + q.n; ++j) {
+            const DrawRec &r = draws[(size_t)j];
+            const int kind = r.kd & KD_KIND_MASK;
+            if ((kind == K_FIXED) != (q.block < 0) || H.link_block[(size_t)r.link] != q.block) fail("drawing record");
+            if (kind == K_FIXED) continue;
+            if (r.kd >> 8 >= (int32_t)H.dist.size()) fail("drawing distribution");
+            const DistParam &dp = H.dist[(size_t)(r.kd >> 8)];
+            if (((r.kd >> KD_WORD_SHIFT) & 3) + (kind == K_GAMMA ? dp.erlang : 1) > 4) fail("drawing words");
+            if (r.vt >= 0 && (int64_t)r.vt + dp.tab_n > (int64_t)H.vals.size()) fail("drawing table");
+        }
+    }
+    if (next != L) fail("drawing coverage");
 }
 
 size_t tables_bytes(const HostDag &h) {

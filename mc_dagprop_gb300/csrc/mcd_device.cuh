@@ -1,7 +1,7 @@
 // mcd_device.cuh -- device code of the Monte Carlo DAG-propagation path (sm_103a).
 //
-// k_propagate: one CTA owns a tile of 32 samples (one per lane) and walks the
-// whole compiled DAG stage by stage (a stage is a level, or a slice of a wide
+// k_propagate: one CTA owns a tile of 32 samples (one per lane), or a wide tile of
+// 64 (two per lane; use_wide), and walks the whole compiled DAG stage by stage (a stage is a level, or a slice of a wide
 // level); the warps of the CTA split each stage's events and meet at a barrier
 // between stages.  The records of the next stage are copied into shared memory
 // by the TMA bulk-copy engine (cp.async.bulk + mbarrier, double-buffered) while
@@ -27,6 +27,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "mcd_internal.hpp"
 
@@ -39,6 +40,11 @@ cudaError_t raise_smem_limit(const void *fn, size_t smem);
 
 // Warps per CTA of a single-DAG launch over `tiles` tiles.
 int pick_warps(const KArgs &a, int64_t tiles);
+
+// Wide tiles (two samples a lane) of a sampled launch: whether they run it, and the
+// arguments with their layout in place.
+bool use_wide(const KArgs &a);
+KArgs wide_args(const KArgs &a);
 
 // ---------------------------------------------------------------- Philox4x32-10
 // Counter mode under one fixed key: the 128-bit counter is (seed low, seed high,
@@ -228,34 +234,51 @@ __device__ __forceinline__ double draw_empirical(const DistParam &p, const Alias
     return relative ? __dadd_rn(base, __dmul_rn(val, base)) : __dadd_rn(base, val);
 }
 
-// A sampled link's duration.  TSMEM: the tables block is in shared memory;
+// A sampled link's durations of a lane's S samples.  TSMEM: the tables block is in shared memory;
 // STAGED: the link's duration table (if any) is in the current stage's staging
 // buffer.  Both are compile-time here so that every table read is a
 // shared-memory load (or a global one) rather than a generic load.
-template <bool STAGED, bool TSMEM>
-__device__ __forceinline__ double sampled_duration(const KArgs &a, int32_t kd, double v, int32_t dvo, uint32_t block,
-                                                   uint32_t link, uint64_t seed, U4 &grp, const unsigned char *smem,
-                                                   int buf, float &dfac) {
+template <bool STAGED, bool TSMEM, int S>
+__device__ __forceinline__ void sampled_duration(const KArgs &a, int32_t kd, double v, int32_t dvo, uint32_t block,
+                                                 uint32_t link, const uint64_t (&seed)[S], U4 (&grp)[S],
+                                                 const unsigned char *smem, int buf, double (&dur)[S], float (&dfac)[S]) {
     const DistParam *dists = TSMEM ? reinterpret_cast<const DistParam *>(smem + a.smem_tables_off) : a.dist;
     const DistParam &p = dists[kd >> 8];
     int32_t *err = a.err;
     const AliasEntry *alias = reinterpret_cast<const AliasEntry *>(dists + a.n_dist);
     const AliasPick *picks = reinterpret_cast<const AliasPick *>(alias + a.n_alias);
     const int kind = kd & KD_KIND_MASK;
-    if (kind == K_GAMMA && !p.erlang) return draw_gamma(p, v, block, seed, err, &dfac);
-    if (!(kd & KD_REUSE)) grp = draw_words(seed, block, 0u, 0u);
+    if (kind == K_GAMMA && !p.erlang) {
+#pragma unroll
+        for (int j = 0; j < S; ++j) dur[j] = draw_gamma(p, v, block, seed[j], err, &dfac[j]);
+        return;
+    }
+    if (!(kd & KD_REUSE)) {
+#pragma unroll
+        for (int j = 0; j < S; ++j) grp[j] = draw_words(seed[j], block, 0u, 0u);
+    }
     const int wsel = (kd >> KD_WORD_SHIFT) & 3;
-    if (kind == K_GAMMA) return draw_erlang(p, v, link, seed, grp, wsel, err, &dfac);
-    const uint32_t r = word_of(grp, wsel);
-    if (kind == K_EXP) return draw_exponential(p, v, r, dfac);
+    if (kind == K_GAMMA) {
+#pragma unroll
+        for (int j = 0; j < S; ++j) dur[j] = draw_erlang(p, v, link, seed[j], grp[j], wsel, err, &dfac[j]);
+        return;
+    }
+    if (kind == K_EXP) {
+#pragma unroll
+        for (int j = 0; j < S; ++j) dur[j] = draw_exponential(p, v, word_of(grp[j], wsel), dfac[j]);
+        return;
+    }
     const double *vt = nullptr;
     if (dvo >= 0)
         vt = STAGED ? reinterpret_cast<const double *>(smem + a.smem_stage_off + buf * a.stage_bytes + dvo)
                     : a.vals + (dvo ^ kVtGlobal);
-    return draw_empirical(p, alias, picks, vt, v, kind == K_EMP_REL, r, grp.y, (kd & KD_TWO_WORD) != 0, dfac);
+#pragma unroll
+    for (int j = 0; j < S; ++j)
+        dur[j] = draw_empirical(p, alias, picks, vt, v, kind == K_EMP_REL, word_of(grp[j], wsel), grp[j].y,
+                                (kd & KD_TWO_WORD) != 0, dfac[j]);
 }
 
-// The link's duration for one sample, and (dfac) its derivative with respect to
+// The link's duration for each of a lane's samples, and (dfac) its derivative with respect to
 // the base duration: 1 + X for the multiplicative kinds, 1 for absolute tables,
 // the host-computed value for fixed links.  block: the link's Philox block;
 // grp: the words of the block the event's previous exponential or empirical
@@ -269,17 +292,22 @@ __device__ __forceinline__ double sampled_duration(const KArgs &a, int32_t kd, d
 // kernel: one copy of the samplers, no branch per edge), or kTablesEither
 // (KArgs::tables_in_smem decides per launch or per DAG).
 enum : int { kTablesGlobal = 0, kTablesSmem = 1, kTablesEither = 2 };
-template <bool STAGED, int TS>
-__device__ __forceinline__ double link_duration(const KArgs &a, int32_t kd, double v, int32_t dvo, uint32_t block,
-                                                uint32_t link, uint64_t seed, U4 &grp, const unsigned char *smem,
-                                                int buf, float &dfac) {
+template <bool STAGED, int TS, int S>
+__device__ __forceinline__ void link_duration(const KArgs &a, int32_t kd, double v, int32_t dvo, uint32_t block,
+                                              uint32_t link, const uint64_t (&seed)[S], U4 (&grp)[S],
+                                              const unsigned char *smem, int buf, double (&dur)[S], float (&dfac)[S]) {
     if ((kd & KD_KIND_MASK) == K_FIXED) {
-        dfac = __int_as_float(dvo);
-        return v;
+#pragma unroll
+        for (int j = 0; j < S; ++j) {
+            dfac[j] = __int_as_float(dvo);
+            dur[j] = v;
+        }
+        return;
     }
     if (TS == kTablesSmem || (TS == kTablesEither && a.tables_in_smem))
-        return sampled_duration<STAGED, true>(a, kd, v, dvo, block, link, seed, grp, smem, buf, dfac);
-    return sampled_duration<STAGED, false>(a, kd, v, dvo, block, link, seed, grp, smem, buf, dfac);
+        sampled_duration<STAGED, true, S>(a, kd, v, dvo, block, link, seed, grp, smem, buf, dur, dfac);
+    else
+        sampled_duration<STAGED, false, S>(a, kd, v, dvo, block, link, seed, grp, smem, buf, dur, dfac);
 }
 
 // ---------------------------------------------------------------- records
@@ -400,45 +428,60 @@ __device__ __forceinline__ long long warp_sum_ticks(long long d) {
     return (long long)((unsigned long long)s0 + ((unsigned long long)s1 << 27));
 }
 
-// One event's realized values of the tile into the per-event accumulators:
-// the tile's sum of (realized - earliest) with one 64-bit atomic, and the
-// histogram with one atomic per lane (LANE_HIST and KArgs::hist_lane) or per
+// One event's realized values of the tile (S samples a lane) into the per-event
+// accumulators: the tile's sum of (realized - earliest) with one 64-bit atomic, and
+// the histogram with one atomic per sample (LANE_HIST and KArgs::hist_lane) or per
 // distinct bin of the warp.  te: the event's earliest in ticks (KArgs::te),
 // loaded when the event started.
-template <bool POSITIVE, bool LANE_HIST>
-__device__ __forceinline__ void accumulate_stats(const KArgs &a, const EvRec &ev, long long lbits, long long te,
-                                                 bool active, unsigned active_mask) {
-    int bin;
+template <bool POSITIVE, bool LANE_HIST, int S>
+__device__ __forceinline__ void accumulate_stats(const KArgs &a, const EvRec &ev, const long long (&lbits)[S],
+                                                 long long te, const bool (&active)[S],
+                                                 const unsigned (&active_mask)[S]) {
+    int bin[S];
     if (a.stats_fixed) {
-        // realized >= earliest and ticks are monotone: d >= 0
-        const long long d = active ? tick_count<POSITIVE>(lbits, a.tick_q) - te : 0ll;
-        bin = (int)__umul64hi((unsigned long long)d, a.bin_mul);
-        bin = bin > kHistBins - 1 ? kHistBins - 1 : bin;
-        const long long s = warp_sum_ticks(d);
+        long long sum = 0;  // of S <= 2 counts below 2^53 each
+#pragma unroll
+        for (int j = 0; j < S; ++j) {
+            // realized >= earliest and ticks are monotone: d >= 0
+            const long long d = active[j] ? tick_count<POSITIVE>(lbits[j], a.tick_q) - te : 0ll;
+            bin[j] = (int)__umul64hi((unsigned long long)d, a.bin_mul);
+            bin[j] = bin[j] > kHistBins - 1 ? kHistBins - 1 : bin[j];
+            sum += d;
+        }
+        const long long s = warp_sum_ticks(sum);
         if ((threadIdx.x & 31) == 0 && s != 0) atomicAdd(&a.acc[ev.user], (unsigned long long)s);
     } else {
-        const double dd = active ? __longlong_as_double(lbits) - __longlong_as_double(ev.init_bits) : 0.0;
-        const double x = dd * a.hist_inv_w;
-        bin = x >= (double)(kHistBins - 1) ? kHistBins - 1 : (x > 0.0 ? (int)x : 0);
-        if (active && dd != 0.0) atomicAdd(reinterpret_cast<double *>(&a.acc[ev.user]), dd);
+#pragma unroll
+        for (int j = 0; j < S; ++j) {
+            const double dd = active[j] ? __longlong_as_double(lbits[j]) - __longlong_as_double(ev.init_bits) : 0.0;
+            const double x = dd * a.hist_inv_w;
+            bin[j] = x >= (double)(kHistBins - 1) ? kHistBins - 1 : (x > 0.0 ? (int)x : 0);
+            if (active[j] && dd != 0.0) atomicAdd(reinterpret_cast<double *>(&a.acc[ev.user]), dd);
+        }
     }
-    if (lbits == ev.init_bits) bin = kBinLo;
-    else if (lbits == ev.ub_bits) bin = kBinHi;
-    if (LANE_HIST && a.hist_lane) {
-        if (active) atomicAdd(&a.hist[(int64_t)ev.user * kHistStride + bin], 1u);
-    } else if (active) {
-        const unsigned same = __match_any_sync(active_mask, bin);
-        if ((threadIdx.x & 31) == __ffs(same) - 1)
-            atomicAdd(&a.hist[(int64_t)ev.user * kHistStride + bin], (unsigned)__popc(same));
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+        if (lbits[j] == ev.init_bits) bin[j] = kBinLo;
+        else if (lbits[j] == ev.ub_bits) bin[j] = kBinHi;
+        if (LANE_HIST && a.hist_lane) {
+            if (active[j]) atomicAdd(&a.hist[(int64_t)ev.user * kHistStride + bin[j]], 1u);
+        } else if (active[j]) {
+            const unsigned same = __match_any_sync(active_mask[j], bin[j]);
+            if ((threadIdx.x & 31) == __ffs(same) - 1)
+                atomicAdd(&a.hist[(int64_t)ev.user * kHistStride + bin[j]], (unsigned)__popc(same));
+        }
     }
 }
 
 // The tile's sum of (realized - earliest) ticks into a.acc (objective of the
 // adjoint; the same integer accumulation as the statistics mean).
-template <bool POSITIVE>
-__device__ __forceinline__ void accumulate_sum(const KArgs &a, const EvRec &ev, long long lbits, long long te,
-                                               bool active) {
-    const long long s = warp_sum_ticks(active ? tick_count<POSITIVE>(lbits, a.tick_q) - te : 0ll);
+template <bool POSITIVE, int S>
+__device__ __forceinline__ void accumulate_sum(const KArgs &a, const EvRec &ev, const long long (&lbits)[S],
+                                               long long te, const bool (&active)[S]) {
+    long long sum = 0;
+#pragma unroll
+    for (int j = 0; j < S; ++j) sum += active[j] ? tick_count<POSITIVE>(lbits[j], a.tick_q) - te : 0ll;
+    const long long s = warp_sum_ticks(sum);
     if ((threadIdx.x & 31) == 0 && s != 0) atomicAdd(&a.acc[ev.user], (unsigned long long)s);
 }
 
@@ -452,19 +495,32 @@ __device__ __forceinline__ uint64_t row_off(int32_t row, uint32_t ld) { return (
 // host keeps leading dimensions below 2^29).
 template <typename T>
 __device__ __forceinline__ T *at_row(T *col, int32_t row, uint32_t ld_bytes) {
-    return reinterpret_cast<T *>(reinterpret_cast<uintptr_t>(col) + (uint64_t)(uint32_t)row * ld_bytes);
+    using Byte = std::conditional_t<std::is_const<T>::value, const char, char>;
+    return reinterpret_cast<T *>(reinterpret_cast<Byte *>(col) + (uint64_t)(uint32_t)row * ld_bytes);
 }
 
-// A tile's per-lane state: its sample, seed, and output columns.
+// The window row of a slot word (PredRec::src_slot, EvRec::slot): the low half for
+// tiles of 32 samples, the high half, signed, for wide tiles (negative: no row on
+// chip; of a source, ~ its off-chip row).
+template <int S>
+__device__ __forceinline__ int32_t window_row(int32_t slots) {
+    return S == 1 ? (int32_t)(int16_t)slots : slots >> 16;
+}
+
+// A tile's per-lane state: its S samples (s + 32 j), seeds, and output columns.
+// Columns are those of sample s; sample j's values lie 32 j elements further.
+template <int S>
 struct TileCtx {
     int lane;
-    int64_t s;                 // the lane's sample
-    bool active;               // s < n
-    unsigned active_mask;
-    uint64_t seed;
+    int64_t s;                 // the lane's first sample
+    bool active[S];            // s + 32 j < n
+    unsigned active_mask[S];
+    uint64_t seed[S];
     double *rcol;              // this lane's column of the global realized rows (window off chip, or
                                // output), or null
     uint32_t rows_ld8;         // their row pitch in bytes
+    double *scol;              // this lane's column of the off-chip window rows (wide tiles), or null: the
+                               // realized rows serve
     double *dcol;              // durations output column of this lane (null: none, or inactive)
     int32_t *ccol;             // cause_event output column of this lane (null: none, or inactive)
     uint32_t ld8, ld4;         // row pitches of the outputs in bytes (doubles, int32)
@@ -491,12 +547,34 @@ __device__ __forceinline__ int take_next(uint32_t ctr) {
 // global memory.  pred0: the stage's first predecessor record (the records'
 // pred_begin/pred_end are global indices); ev0: its first event's compiled
 // index; buf: the staging buffer (0 or 1) that holds the stage.
-template <bool GIVEN, bool WIN_SMEM, bool STATS, bool POSITIVE, bool ADJ, bool STAGED, int TS, bool LANE_HIST>
+template <bool GIVEN, bool WIN_SMEM, bool STATS, bool POSITIVE, bool ADJ, bool STAGED, int TS, bool LANE_HIST, int S>
 __device__ __forceinline__ void stage_events(const KArgs &a, int buf, const EvRec *sev, const PredRec *spred, int pred0,
-                                             int ev0, int n_ev, int n_pair, uint32_t ctr, const TileCtx &t,
-                                             unsigned char *smem, U4 &grp) {
+                                             int ev0, int n_ev, int n_pair, uint32_t ctr, const TileCtx<S> &t,
+                                             unsigned char *smem, U4 (&grp)[S]) {
     double *win = reinterpret_cast<double *>(smem);
     const int lane = t.lane;
+    // The realized times of a predecessor: from the window row of its slot; a wide
+    // tile's predecessor without one (see window_row) from its off-chip window row
+    // or, where the realized times are an output, from that; window off chip: from
+    // the realized rows.
+    auto source = [&](int32_t slots, int32_t user, double (&v)[S]) {
+        if (WIN_SMEM) {
+            const int32_t slot = window_row<S>(slots);
+            if (S == 1 || slot >= 0) {
+#pragma unroll
+                for (int j = 0; j < S; ++j) v[j] = win[slot * (kTile * S) + lane + 32 * j];
+                return;
+            }
+            if (t.scol) {
+#pragma unroll
+                for (int j = 0; j < S; ++j) v[j] = __ldcg(t.scol + (~slot) * (kTile * S) + 32 * j);
+                return;
+            }
+        }
+        const double *row = at_row(t.rcol, user, t.rows_ld8);
+#pragma unroll
+        for (int j = 0; j < S; ++j) v[j] = t.active[j] ? row[32 * j] : 0.0;
+    };
     // The warp's next event: the second of the current pair, or the first event of
     // the next unit, which lane 0 takes before this event's work, hiding the
     // atomic's latency (a warp holds at most one extra unit: the cheapest, by
@@ -520,93 +598,134 @@ __device__ __forceinline__ void stage_events(const KArgs &a, int buf, const EvRe
         // latency hides behind them)
         const long long te =
             (STATS || (ADJ && (a.adj_flags & kAdjObjective))) && a.stats_fixed ? __ldg(a.te + ev.user) : 0ll;
+        const int32_t spill_row = S > 1 && t.scol ? __ldg(a.ev_spill + ev0 + i) : -1;  // off-chip window row
         // POSITIVE: keys are the bits themselves (init_key == init_bits, ub_key == ub_bits),
         // so one 64-bit value carries both
-        long long lk = POSITIVE ? ev.init_bits : ev.init_key, lbits = ev.init_bits;
+        long long lk[S], lbits[S];
         const long long ub_key = POSITIVE ? ev.ub_bits : ev.ub_key;
-        int32_t cause = -1;
-        uint32_t win_code = kAdjNone;  // ADJ: winner position | clamp flag
-        float win_dfac = 0.0f;
+        int32_t cause[S];
+        uint32_t win_code[S];  // ADJ: winner position | clamp flag
+        float win_dfac[S];
+#pragma unroll
+        for (int j = 0; j < S; ++j) {
+            lk[j] = POSITIVE ? ev.init_bits : ev.init_key;
+            lbits[j] = ev.init_bits;
+            cause[j] = -1;
+            win_code[j] = kAdjNone;
+            win_dfac[j] = 0.0f;
+        }
         const int pb = ev.pred_begin - pred0, pe = ev.pred_end - pred0;
+        // One entry of one sample (_core.cpp:341-347): the one FP64 add of the edge, the
+        // clamp t = std::min(t, ub), and if (t >= latest) { latest = t; cause = src; }.
+        auto relax = [&](int j, double src, double dur, int32_t user, int at, float dfac) {
+            const double tt = src + dur;
+            long long tb = __double_as_longlong(tt);
+            long long tk = order_key<POSITIVE>(tb);
+            const bool clamp = ub_key < tk;
+            if (clamp) {
+                tk = ub_key;
+                tb = ev.ub_bits;
+            }
+            if (tk >= lk[j]) {
+                lk[j] = tk;
+                lbits[j] = POSITIVE ? tk : tb;
+                cause[j] = user;
+                if (ADJ) {
+                    win_code[j] = (uint32_t)at | (clamp ? kAdjClamped : 0u);
+                    win_dfac[j] = dfac;
+                }
+            }
+        };
         // Given durations come from global memory, each an uncached DRAM read: the
         // reads of up to four entries are issued together, then the entries are
         // relaxed in order (one memory latency per four entries, not per entry).
         for (int p0 = pb; GIVEN && p0 < pe; p0 += 4) {
-            double dg[4];
+            double dg[4][S];
+            int4 rec[4];  // PredRec: src_slot, src_user, link, kd
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                dg[k] = 0.0;
+#pragma unroll
+                for (int j = 0; j < S; ++j) dg[k][j] = 0.0;
                 if (p0 + k < pe) {
-                    const int32_t link = reinterpret_cast<const int4 *>(spred + p0 + k)->z;  // PredRec::link
-                    if (t.active && link >= 0) dg[k] = __ldg(at_row(t.dincol, link, t.ld_in8));
+                    rec[k] = reinterpret_cast<const int4 *>(spred + p0 + k)[0];
+                    if (rec[k].z >= 0) {
+                        const double *row = at_row(t.dincol, rec[k].z, t.ld_in8);
+#pragma unroll
+                        for (int j = 0; j < S; ++j)
+                            if (t.active[j]) dg[k][j] = __ldg(row + 32 * j);
+                    }
                 }
             }
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 if (p0 + k >= pe) continue;
-                const PredRec pr = load_pred(spred + p0 + k);
-                const double src = WIN_SMEM ? win[pr.src_slot * kTile + lane]
-                                            : (t.active ? *at_row(t.rcol, pr.src_user, t.rows_ld8) : 0.0);
-                const double tt = src + dg[k];  // the one FP64 add of the edge (_core.cpp:341)
-                long long tb = __double_as_longlong(tt);
-                long long tk = order_key<POSITIVE>(tb);
-                const bool clamp = ub_key < tk;
-                if (clamp) {  // t = std::min(t, ub)
-                    tk = ub_key;
-                    tb = ev.ub_bits;
-                }
-                if (tk >= lk) {  // if (t >= latest) { latest = t; cause = src; }
-                    lk = tk;
-                    lbits = POSITIVE ? tk : tb;
-                    cause = pr.src_user;
-                    if (ADJ) win_code = (uint32_t)(p0 + k - pb) | (clamp ? kAdjClamped : 0u);
-                }
+                double src[S];
+                source(rec[k].x, rec[k].y, src);
+#pragma unroll
+                for (int j = 0; j < S; ++j) relax(j, src[j], dg[k][j], rec[k].y, p0 + k - pb, 0.0f);
             }
         }
         for (int p = pb; !GIVEN && p < pe; ++p) {
             const PredRec pr = load_pred(spred + p);
-            float dfac = 0.0f;
-            const double dur = link_duration<STAGED, TS>(a, pr.kd, pr.v, pr.dvo, (uint32_t)pr.block,
-                                                         (uint32_t)pr.link, t.seed, grp, smem, buf, dfac);
-            if (!STATS && !ADJ && (pr.kd & KD_WRITE) && t.dcol) *at_row(t.dcol, pr.link, t.ld8) = dur;
-            // with the window on chip every source has a slot (the compiler checks it)
-            const double src = WIN_SMEM ? win[pr.src_slot * kTile + lane]
-                                        : (t.active ? *at_row(t.rcol, pr.src_user, t.rows_ld8) : 0.0);
-            const double tt = src + dur;  // the one FP64 add of the edge (_core.cpp:341)
-            long long tb = __double_as_longlong(tt);
-            long long tk = order_key<POSITIVE>(tb);
-            const bool clamp = ub_key < tk;
-            if (clamp) {  // t = std::min(t, ub)
-                tk = ub_key;
-                tb = ev.ub_bits;
+            double src[S], dur[S];
+            float dfac[S];
+            if (S > 1) source(pr.src_slot, pr.src_user, src);  // (may come from L2: ahead of the draws)
+            link_duration<STAGED, TS, S>(a, pr.kd, pr.v, pr.dvo, (uint32_t)pr.block, (uint32_t)pr.link, t.seed, grp, smem,
+                                         buf, dur, dfac);
+            if (!STATS && !ADJ && (pr.kd & KD_WRITE) && t.dcol) {
+                double *row = at_row(t.dcol, pr.link, t.ld8);
+#pragma unroll
+                for (int j = 0; j < S; ++j)
+                    if (j == 0 || t.active[j]) row[32 * j] = dur[j];
             }
-            if (tk >= lk) {  // if (t >= latest) { latest = t; cause = src; }
-                lk = tk;
-                lbits = POSITIVE ? tk : tb;
-                cause = pr.src_user;
-                if (ADJ) {
-                    win_code = (uint32_t)(p - pb) | (clamp ? kAdjClamped : 0u);
-                    win_dfac = dfac;
-                }
-            }
+            if (S == 1) source(pr.src_slot, pr.src_user, src);
+#pragma unroll
+            for (int j = 0; j < S; ++j) relax(j, src[j], dur[j], pr.src_user, p - pb, dfac[j]);
         }
         // realized = std::min(latest, ub): latest only exceeds ub when earliest does, which
         // non-negative max_delay rules out in POSITIVE mode
-        if (!POSITIVE && ub_key < lk) lbits = ev.ub_bits;
-        const double real = __longlong_as_double(lbits);
-        if (WIN_SMEM && ev.slot >= 0) win[ev.slot * kTile + lane] = real;
-        if (STATS) accumulate_stats<POSITIVE, LANE_HIST>(a, ev, lbits, te, t.active, t.active_mask);
-        if (ADJ) {
-            const bool delayed = lk > (POSITIVE ? ev.init_bits : ev.init_key);  // realized > earliest
-            if (a.adj_flags & kAdjObjective) accumulate_sum<POSITIVE>(a, ev, lbits, te, t.active);
-            if (t.active && a.adj_code) {  // rows by compiled index, from the block's first event
-                const int64_t o = (int64_t)row_off(ev0 + i - a.code_base, (uint32_t)a.ld) + t.s;
-                a.adj_code[o] = (uint16_t)(win_code | (delayed ? kAdjDelayed : 0u));
-                a.adj_dfac[o] = win_dfac;
+#pragma unroll
+        for (int j = 0; j < S; ++j)
+            if (!POSITIVE && ub_key < lk[j]) lbits[j] = ev.ub_bits;
+        if (WIN_SMEM) {
+            const int32_t slot = window_row<S>(ev.slot);
+            if (slot >= 0) {
+#pragma unroll
+                for (int j = 0; j < S; ++j)
+                    win[slot * (kTile * S) + lane + 32 * j] = __longlong_as_double(lbits[j]);
+            }
+            if (S > 1 && spill_row >= 0) {
+#pragma unroll
+                for (int j = 0; j < S; ++j)
+                    __stcg(t.scol + spill_row * (kTile * S) + 32 * j, __longlong_as_double(lbits[j]));
             }
         }
-        if (t.active && t.rcol) *at_row(t.rcol, ev.user, t.rows_ld8) = real;
-        if (!STATS && !ADJ && t.ccol) *at_row(t.ccol, ev.user, t.ld4) = cause;
+        if (STATS) accumulate_stats<POSITIVE, LANE_HIST, S>(a, ev, lbits, te, t.active, t.active_mask);
+        if (ADJ) {
+            if (a.adj_flags & kAdjObjective) accumulate_sum<POSITIVE, S>(a, ev, lbits, te, t.active);
+            if (a.adj_code) {  // rows by compiled index, from the block's first event
+                const int64_t o = (int64_t)row_off(ev0 + i - a.code_base, (uint32_t)a.ld) + t.s;
+#pragma unroll
+                for (int j = 0; j < S; ++j) {
+                    if (!t.active[j]) continue;
+                    const bool delayed = lk[j] > (POSITIVE ? ev.init_bits : ev.init_key);  // realized > earliest
+                    a.adj_code[o + 32 * j] = (uint16_t)(win_code[j] | (delayed ? kAdjDelayed : 0u));
+                    a.adj_dfac[o + 32 * j] = win_dfac[j];
+                }
+            }
+        }
+        if (t.rcol && t.active[0]) {
+            double *row = at_row(t.rcol, ev.user, t.rows_ld8);
+#pragma unroll
+            for (int j = 0; j < S; ++j)
+                if (j == 0 || t.active[j]) row[32 * j] = __longlong_as_double(lbits[j]);
+        }
+        if (!STATS && !ADJ && t.ccol) {
+            int32_t *row = at_row(t.ccol, ev.user, t.ld4);
+#pragma unroll
+            for (int j = 0; j < S; ++j)
+                if (j == 0 || t.active[j]) row[32 * j] = cause[j];
+        }
         i_next = __shfl_sync(0xFFFFFFFFu, i_next, 0);
     }
 }
@@ -621,9 +740,12 @@ __device__ __forceinline__ void stage_events(const KArgs &a, int buf, const EvRe
 // per-event accumulators (mean, histogram); nothing per sample leaves the chip.
 // POSITIVE: all times non-negative and finite (host-checked): raw bits are keys.
 // reuse: the CTA ran an earlier tile with these barriers (persistent kernels).
+// S: samples a lane carries (1, or 2: a wide tile of 64 samples; see kWideTile).
+// spill: a wide tile's off-chip window rows (KArgs::window_spill of 64 doubles), or
+// null: the realized rows serve.
 // Returns false when a staged copy never landed (then every thread returns false).
 //
-// Shared memory: [window: window_slots x 32 doubles][stage buffer 0][stage
+// Shared memory: [window: window_slots x 32 S doubles][stage buffer 0][stage
 // buffer 1][distribution params][alias entries][alias picks][2 mbarriers, 2
 // stage counters]; a stage buffer holds [event records][predecessor
 // records][value region]; `bars` is that layout's barrier region
@@ -639,29 +761,34 @@ __device__ __forceinline__ void stage_events(const KArgs &a, int buf, const EvRe
 // a.blk_start stages begins -- the checkpoints a level-block recomputation
 // starts from.
 template <bool GIVEN, bool WIN_SMEM, bool STATS, bool POSITIVE, bool ADJ = false, int TS = kTablesEither,
-          bool LANE_HIST = true>
+          bool LANE_HIST = true, int S = 1>
 __device__ __forceinline__ bool propagate_tile(const KArgs &a, int64_t tile, double *rows, int64_t rows_ld,
                                                bool rows_tile_local, unsigned char *smem, uint64_t *bars,
-                                               bool reuse) {
+                                               bool reuse, double *spill = nullptr) {
     DistParam *s_dist = reinterpret_cast<DistParam *>(smem + a.smem_tables_off);
 
-    TileCtx t;
+    TileCtx<S> t;
     t.lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int NW = blockDim.x >> 5;
-    t.s = tile * kTile + t.lane;
-    t.active = t.s < a.n;
-    t.active_mask = __ballot_sync(0xFFFFFFFFu, t.active);
-    t.seed = 0;
-    if (!GIVEN && t.active) t.seed = a.seeds ? (uint64_t)a.seeds[t.s] : (uint64_t)(a.seed0 + t.s);
+    t.s = tile * (kTile * S) + t.lane;
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+        const int64_t s = t.s + 32 * j;
+        t.active[j] = s < a.n;
+        t.active_mask[j] = __ballot_sync(0xFFFFFFFFu, t.active[j]);
+        t.seed[j] = 0;
+        if (!GIVEN && t.active[j]) t.seed[j] = a.seeds ? (uint64_t)a.seeds[s] : (uint64_t)(a.seed0 + s);
+    }
     t.rcol = rows ? rows + (rows_tile_local ? (int64_t)t.lane : t.s) : nullptr;
+    t.scol = spill ? spill + t.lane : nullptr;
     t.rows_ld8 = (uint32_t)rows_ld * 8u;
     t.ld8 = (uint32_t)a.ld * 8u;
     t.ld4 = (uint32_t)a.ld * 4u;
     t.dincol = GIVEN ? a.dur_in + t.s : nullptr;
     t.ld_in8 = (uint32_t)a.ld_in * 8u;
-    t.dcol = (!STATS && !ADJ && !GIVEN && a.durations && t.active) ? a.durations + t.s : nullptr;
-    t.ccol = (!STATS && !ADJ && a.cause && t.active) ? a.cause + t.s : nullptr;
+    t.dcol = (!STATS && !ADJ && !GIVEN && a.durations && t.active[0]) ? a.durations + t.s : nullptr;
+    t.ccol = (!STATS && !ADJ && a.cause && t.active[0]) ? a.cause + t.s : nullptr;
 
     // distribution tables into shared memory; fresh barriers for this tile
     if (a.tables_in_smem) {  // the tables block, 8 bytes at a time (its size is a multiple of 8)
@@ -672,7 +799,7 @@ __device__ __forceinline__ bool propagate_tile(const KArgs &a, int64_t tile, dou
     // stages run: all, or (adjoint) one block of them
     const int s_begin = ADJ ? a.stage_begin : 0;
     const int s_end = ADJ ? a.stage_end : a.n_stages;
-    const int win_n = a.window_slots * kTile;  // doubles of one tile's window
+    const int win_n = a.window_slots * kTile * S;  // doubles of one tile's window
     if (ADJ && WIN_SMEM && a.win_in) {  // a block recomputed from its checkpoint
         const double *src = a.win_in + (int64_t)tile * win_n;
         double *win = reinterpret_cast<double *>(smem);
@@ -680,7 +807,7 @@ __device__ __forceinline__ bool propagate_tile(const KArgs &a, int64_t tile, dou
     }
     int next_blk = 0;  // the next checkpoint to save (ADJ with a.win_ckpt)
     int *stage_ctr = reinterpret_cast<int *>(bars + 2);
-    U4 grp{};  // the words of the Philox block the current event last drew (see KD_REUSE)
+    U4 grp[S] = {};  // the words of the Philox block the current event last drew (see KD_REUSE)
     if (threadIdx.x == 0) {
         if (reuse) {
             asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(&bars[0])) : "memory");
@@ -743,11 +870,11 @@ __device__ __forceinline__ bool propagate_tile(const KArgs &a, int64_t tile, dou
         const uint32_t ctr = smem_u32(&stage_ctr[j & 1]);
         if (meta.y >= 0) {  // records in the staging buffer (shared memory)
             const unsigned char *buf = smem + a.smem_stage_off + b * a.stage_bytes;
-            stage_events<GIVEN, WIN_SMEM, STATS, POSITIVE, ADJ, true, TS, LANE_HIST>(
+            stage_events<GIVEN, WIN_SMEM, STATS, POSITIVE, ADJ, true, TS, LANE_HIST, S>(
                 a, b, reinterpret_cast<const EvRec *>(buf), reinterpret_cast<const PredRec *>(buf + mv.z), meta.z,
                 meta.x, meta.y, n_pair, ctr, t, smem, grp);
         } else {  // a stage whose records exceed the buffer is read from global memory
-            stage_events<GIVEN, WIN_SMEM, STATS, POSITIVE, ADJ, false, TS, LANE_HIST>(
+            stage_events<GIVEN, WIN_SMEM, STATS, POSITIVE, ADJ, false, TS, LANE_HIST, S>(
                 a, b, a.ev + meta.x, a.pred + meta.z, meta.z, meta.x, -meta.y, n_pair, ctr, t, smem, grp);
         }
         __syncthreads();
@@ -758,26 +885,32 @@ __device__ __forceinline__ bool propagate_tile(const KArgs &a, int64_t tile, dou
     if (!STATS && !ADJ && !GIVEN && a.durations) {
         for (int i = warp; i < a.n_aux; i += NW) {
             const LinkRec lr = a.aux[i];
-            float dfac;
-            U4 own;  // an unreferenced link owns its block
-            const double dur =
-                link_duration<false, TS>(a, lr.kd, lr.v, -1, (uint32_t)lr.link, (uint32_t)lr.link, t.seed, own, smem, 0, dfac);
-            if (t.dcol) *at_row(t.dcol, lr.link, t.ld8) = dur;
+            float dfac[S];
+            double dur[S];
+            U4 own[S];  // an unreferenced link owns its block
+            link_duration<false, TS, S>(a, lr.kd, lr.v, -1, (uint32_t)lr.link, (uint32_t)lr.link, t.seed, own, smem, 0, dur,
+                                        dfac);
+            if (t.dcol) {
+                double *row = at_row(t.dcol, lr.link, t.ld8);
+#pragma unroll
+                for (int j = 0; j < S; ++j)
+                    if (j == 0 || t.active[j]) row[32 * j] = dur[j];
+            }
         }
     }
     return true;
 }
 
-// One CTA per tile of 32 samples.  TS: the tables block's place (kTablesGlobal or
+// One CTA per tile of 32 S samples.  TS: the tables block's place (kTablesGlobal or
 // kTablesSmem; the host launches the instantiation that matches the DAG).
-template <bool GIVEN, bool WIN_SMEM, bool STATS, bool POSITIVE, int TS>
+template <bool GIVEN, bool WIN_SMEM, bool STATS, bool POSITIVE, int TS, int S = 1>
 __global__ void __launch_bounds__(768, 1) k_propagate(const KArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     double *rows = a.realized ? a.realized : a.scratch;  // global realized rows
     if (STATS && WIN_SMEM) rows = nullptr;
-    propagate_tile<GIVEN, WIN_SMEM, STATS, POSITIVE, false, TS>(a, (int64_t)blockIdx.x, rows, a.ld, false, smem,
-                                                                reinterpret_cast<uint64_t *>(smem + a.smem_bar_off),
-                                                                false);
+    double *spill = S > 1 && a.spill ? a.spill + (int64_t)blockIdx.x * a.window_spill * (kTile * S) : nullptr;
+    propagate_tile<GIVEN, WIN_SMEM, STATS, POSITIVE, false, TS, true, S>(
+        a, (int64_t)blockIdx.x, rows, a.ld, false, smem, reinterpret_cast<uint64_t *>(smem + a.smem_bar_off), false, spill);
 }
 
 }  // namespace mcd

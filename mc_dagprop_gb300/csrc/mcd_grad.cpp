@@ -150,8 +150,13 @@ extern "C" int mcd_gradient_host(mcd_dag *g, int64_t seed0, int64_t n, double *o
                      s_cck = (h.win_smem && blocks) ? align_up(tiles * win_n * 4, 256) : 0,
                      s_rows = h.win_smem ? 0 : align_up(E * (size_t)C * 8, 256),
                      s_crow = h.win_smem ? 0 : align_up(E * (size_t)C * 4, 256),
-                     s_blk = align_up(n_blk * 4 + 4, 256);
-        ensure_ws(g, s_code + s_dfac + s_acc + s_ge + s_gl + s_out + s_te + s_wck + s_cck + s_rows + s_crow + s_blk);
+                     s_blk = align_up(n_blk * 4 + 4, 256),
+                     // off-chip window rows of the forward's wide tiles (level blocks run narrow ones)
+                     s_spill = (h.wide_rows > 0 && !blocks) ? align_up((size_t)((C + kWideTile - 1) / kWideTile) *
+                                                                           h.window_spill * kWideTile * 8, 256)
+                                                            : 0;
+        ensure_ws(g, s_code + s_dfac + s_acc + s_ge + s_gl + s_out + s_te + s_wck + s_cck + s_rows + s_crow + s_blk +
+                         s_spill);
         char *p = g->ws;
         auto take = [&p](size_t bytes) {
             char *q = p;
@@ -172,6 +177,7 @@ extern "C" int mcd_gradient_host(mcd_dag *g, int64_t seed0, int64_t n, double *o
         auto *rows = reinterpret_cast<double *>(take(s_rows));
         auto *crow = reinterpret_cast<uint32_t *>(take(s_crow));
         auto *d_blk = reinterpret_cast<int32_t *>(take(s_blk));
+        auto *spill = s_spill ? reinterpret_cast<double *>(take(s_spill)) : nullptr;
         if (blocks)  // the first stage of every block after the first
             cuda_check(cudaMemcpyAsync(d_blk, plan.blk.data() + 1, (n_blk - 1) * 4, cudaMemcpyHostToDevice, st),
                        "block table upload");
@@ -196,6 +202,7 @@ extern "C" int mcd_gradient_host(mcd_dag *g, int64_t seed0, int64_t n, double *o
             }
             if (!blocks) {
                 KArgs f = a;
+                f.spill = spill;
                 f.stage_begin = 0;
                 f.stage_end = h.n_stages;
                 f.adj_code = code;

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <memory>
+#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -25,12 +26,17 @@ struct DagImage {
     LinkRec *d_aux = nullptr;
     DistParam *d_dist = nullptr;  // tables block: distributions, alias entries, alias picks
     double *d_vals = nullptr;
-    DrawGroup *d_groups = nullptr;
-    DrawRec *d_draws = nullptr;
+    int32_t *d_ev_spill = nullptr;
     int32_t *d_wk = nullptr;
     int32_t *d_stage_meta = nullptr;
     double *d_earliest = nullptr;  // caller order, for the statistics finish
     double *d_ub = nullptr;
+    // the links by Philox block, made for the first kernel that draws without
+    // propagating (image_draws)
+    mutable std::once_flag draws_once;
+    mutable DrawGroup *d_groups = nullptr;  // one allocation, the records behind the groups
+    mutable DrawRec *d_draws = nullptr;
+    mutable int32_t n_groups = 0;
     std::vector<unsigned char> key;  // the creation inputs, serialized (empty: not cached)
     DagImage() = default;
     DagImage(const DagImage &) = delete;
@@ -54,8 +60,7 @@ struct mcd_dag {
     const mcd::LinkRec *d_aux = nullptr;
     const mcd::DistParam *d_dist = nullptr;
     const double *d_vals = nullptr;
-    const mcd::DrawGroup *d_groups = nullptr;
-    const mcd::DrawRec *d_draws = nullptr;
+    const int32_t *d_ev_spill = nullptr;
     const int32_t *d_wk = nullptr;
     const int32_t *d_stage_meta = nullptr;
     const double *d_earliest = nullptr;
@@ -67,7 +72,7 @@ struct mcd_dag {
     explicit mcd_dag(std::shared_ptr<const mcd::DagImage> image)
         : img(std::move(image)), h(img->h), device(img->device), dbytes(img->dbytes), d_ev(img->d_ev),
           d_pred(img->d_pred), d_aux(img->d_aux), d_dist(img->d_dist), d_vals(img->d_vals),
-          d_groups(img->d_groups), d_draws(img->d_draws), d_wk(img->d_wk), d_stage_meta(img->d_stage_meta),
+          d_ev_spill(img->d_ev_spill), d_wk(img->d_wk), d_stage_meta(img->d_stage_meta),
           d_earliest(img->d_earliest), d_ub(img->d_ub) {}
     mcd_dag(const mcd_dag &) = delete;
     mcd_dag &operator=(const mcd_dag &) = delete;
@@ -80,6 +85,7 @@ void set_last_error(const std::string &msg);
 void cuda_check(cudaError_t e, const char *what);
 void ensure_ws(mcd_dag *g, size_t bytes);
 KArgs base_args(const mcd_dag *g);
+void image_draws(const mcd_dag *g, KArgs &a);  // KArgs::groups, draws, n_groups
 void check_device_error(mcd_dag *g);
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }

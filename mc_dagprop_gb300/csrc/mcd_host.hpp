@@ -3,8 +3,11 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <future>
 #include <stdexcept>
 #include <string>
+#include <system_error>
+#include <utility>
 #include <vector>
 
 #include "../../include/mc_dagprop_gb300.h"
@@ -63,13 +66,15 @@ struct HostDag {
     int32_t max_units = 0;        // most work units of a stage (0: warps per CTA fixed by the caller)
     int32_t n_stages = 0, stage_bytes = 0;
     int32_t smem_stage_off = 0, smem_tables_off = 0, smem_bar_off = 0, smem_total = 0;
+    // wide tiles (KArgs): their layout, 0 rows when the DAG has none
+    int32_t wide_rows = 0, window_spill = 0;
+    int32_t wide_stage_off = 0, wide_tables_off = 0, wide_bar_off = 0, wide_total = 0;
+    std::vector<int32_t> ev_spill;  // off-chip window row by compiled index (empty: no off-chip rows)
     std::vector<int32_t> stage_meta;  // kStageMetaInts ints per stage (KArgs::stage_meta)
     std::vector<EvRec> ev;
     std::vector<PredRec> pred;
     std::vector<LinkRec> aux;  // links stored by the aux pass
-    std::vector<DrawGroup> groups;  // the links by Philox block: drawing groups, then fixed links
-    std::vector<DrawRec> draws;
-    int32_t n_draw_groups = 0;
+    std::vector<int32_t> link_vt;  // empirical links: their (first) duration table in vals (-1: none)
     int32_t n_orphan = 0;      // sampled links no precedence entry references
     int32_t n_pairs = 0;       // event pairs over all stages (KArgs::stage_meta)
     int64_t block_draws = 0;   // Philox blocks a sample draws on first attempts
@@ -102,6 +107,8 @@ struct StatsParams {
 };
 StatsParams stats_params(const HostDag &h, int64_t n);
 
+void draw_groups(const HostDag &h, std::vector<DrawGroup> &groups, std::vector<DrawRec> &draws);
+
 // The tables block as the kernels read it (KArgs::dist): DistParam[n_dist],
 // AliasEntry[n_alias], AliasPick[n_alias], back to back.
 size_t tables_bytes(const HostDag &h);
@@ -111,6 +118,23 @@ std::vector<unsigned char> tables_block(const HostDag &h);
 // window: MCD_WINDOW_AUTO (shared memory when it fits) or MCD_WINDOW_GLOBAL.
 void compile_dag(const mcd_dag_desc &d, const mcd_generator &g, HostDag &out, int32_t n_warps,
                  int32_t window = MCD_WINDOW_AUTO);
+
+// The invariants every kernel access relies on; no DAG is used without this check
+// (separate from the compile, so that it can run beside the upload).
+void verify_layout(const HostDag &h);
+
+// f() on another thread beside the caller's work, for DAGs where it takes longer than
+// starting one; the result, or f's exception, by the future's get().
+template <typename F>
+auto beside(int32_t n_events, F &&f) -> std::future<decltype(f())> {
+    if (n_events >= 4096) {
+        try {
+            return std::async(std::launch::async, f);
+        } catch (const std::system_error &) {  // no thread to be had
+        }
+    }
+    return std::async(std::launch::deferred, std::forward<F>(f));
+}
 
 // The content key of a compiled DAG: everything compile_dag reads, serialized
 // (the arrays, the generator, warps per CTA, device, the compiler's environment

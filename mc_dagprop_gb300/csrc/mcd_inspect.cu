@@ -313,11 +313,13 @@ int mcd_delay_histograms(mcd_dag *g, const int64_t *seeds, int64_t n, const int3
         ha.nb = n_bins;
         ha.counts = reinterpret_cast<unsigned long long *>(w + o_cnt);
         ha.moments = reinterpret_cast<double *>(w + o_mom);
-        const int64_t groups = (int64_t)hd.groups.size(), slots = (int64_t)std::max(per_sm, 1) * sms;
+        KArgs drawn = base_args(g);
+        image_draws(g, drawn);
+        const int64_t groups = drawn.n_groups, slots = (int64_t)std::max(per_sm, 1) * sms;
         for (int64_t off = 0; off < n && groups > 0; off += C) {
             const int64_t m = std::min(C, n - off);
             cuda_check(cudaMemcpyAsync(w + o_seed, seeds + off, (size_t)m * 8, cudaMemcpyHostToDevice, st), "seeds");
-            KArgs a = base_args(g);
+            KArgs a = drawn;
             a.seeds = reinterpret_cast<const int64_t *>(w + o_seed);
             a.n = m;
             // an item's fixed costs (binning table entries, reducing sums) want many

@@ -55,10 +55,18 @@ constexpr int32_t KD_TWO_WORD = 0x40;
 constexpr int32_t KD_WRITE = 0x80;
 constexpr int32_t kOneWordBins = 4096;  // one 32-bit word picks bin and alias (threshold lattice <= 2^-20)
 
+// A slot word holds an event's window row for tiles of 32 samples (low half, -1:
+// none) and for wide tiles (high half).  A wide tile's window rows are twice as
+// long, so some events' rows may not fit: a source's negative high half is then ~ its
+// off-chip row (HostDag::ev_spill), an event's is -1.
+MCD_HD constexpr int32_t slot_word(int32_t narrow, int32_t wide) {
+    return (int32_t)(((uint32_t)wide << 16) | ((uint32_t)narrow & 0xFFFFu));
+}
+
 // One event, in compiled (level) order.  48 bytes.
 struct alignas(16) EvRec {
     int32_t user;        // event index as the caller numbers it (output row)
-    int32_t slot;        // window slot holding this event's realized value, -1 if no consumer
+    int32_t slot;        // slot word (slot_word): window row holding this event's realized value, -1 if none
     int32_t pred_begin;  // range in the PredRec array
     int32_t pred_end;
     int64_t init_bits;   // earliest (bits): the running max starts here (_core.cpp:336)
@@ -71,7 +79,7 @@ struct alignas(16) EvRec {
 
 // One predecessor edge.  32 bytes.
 struct alignas(16) PredRec {
-    int32_t src_slot;  // window slot of the predecessor's realized value (-1: read its global row)
+    int32_t src_slot;  // slot word: window row of the predecessor's realized value (-1: read its global row)
     int32_t src_user;  // predecessor event index (cause_event value, global row)
     int32_t link;      // link index: durations row and Philox counter; -1 for an index
                        // past the last link, which has duration 0 (see the compiler)
@@ -199,7 +207,7 @@ struct KArgs {
                                 //  first pred, preds, first value, values, byte offsets of the predecessor
                                 //  records and of the value region inside a staging buffer, event pairs, 0, 0, 0}
     const double *vals;         // per-link duration tables, stage by stage (value regions)
-    const DrawGroup *groups;    // the links by Philox block (single-DAG handles only)
+    const DrawGroup *groups;    // the links by Philox block (image_draws)
     const DrawRec *draws;
     int32_t n_groups;
     int32_t n_stages;
@@ -214,6 +222,13 @@ struct KArgs {
     int32_t positive;         // every time non-negative and finite: raw bits order like doubles
     int32_t stage_bytes;      // one staging buffer
     int32_t smem_stage_off, smem_tables_off, smem_bar_off, smem_total;  // shared-memory layout (bytes)
+    // wide tiles (64 samples, two a lane): their layout, replacing the one above at a
+    // wide launch (wide_args); wide_rows 0: the DAG has none
+    int32_t wide_rows;        // window rows on chip
+    int32_t window_spill;     // window rows off chip
+    int32_t wide_stage_off, wide_tables_off, wide_bar_off, wide_total;
+    const int32_t *ev_spill;  // [E] off-chip row of each event by compiled index, -1: none
+    double *spill;            // [tiles][window_spill * 64] off-chip rows (null: realized, an output, serves)
     const int64_t *seeds;  // [n] per-sample seeds; null: sample s uses seed0 + s
     int64_t seed0;
     int64_t n;
@@ -287,6 +302,7 @@ struct FArgs {
 enum : int32_t { ERR_GAMMA_REJECTION = 1, ERR_STAGE_TIMEOUT = 2, ERR_LAYOUT = 4 };
 
 constexpr int kTile = 32;  // samples per tile: one per lane
+constexpr int kWideTile = 64;  // samples of a wide tile: two per lane
 // End of a CTA's shared memory: two mbarriers (8 bytes each), then the two
 // stage work counters (int32 each), padded to 32 bytes.
 constexpr int kBarRegionBytes = 32;

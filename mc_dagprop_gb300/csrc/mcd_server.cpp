@@ -468,6 +468,7 @@ void compile_loop(mcd_server *S) {
             if (mine) {
                 try {
                     compile_dag(d, r->gen, R->h, warps);
+                    verify_layout(R->h);
                     R->lay = img_layout_of(R->h);
                     R->bytes = R->lay.total;
                     if ((int64_t)(R->bytes + rq_layout_of(R->h.E).total) > S->opt.memory_budget)
