@@ -19,18 +19,49 @@
 
 namespace mcd {
 
+// Sum over the warp of 64-bit values (all lanes take part).  Values whose 32-lane sum
+// fits an int -- the common case, one redux -- are told apart by a vote.
+__device__ __forceinline__ long long warp_sum(long long x) {
+    const bool small = x >= -(1ll << 26) && x < (1ll << 26);
+    if (__all_sync(0xFFFFFFFFu, small)) return __reduce_add_sync(0xFFFFFFFFu, (int)x);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xFFFFFFFFu, x, o);
+    return x;
+}
+
+// The shared memory of k_adjoint: [counts: window_slots x 32 uint32 (window on chip)]
+// [stage buffer 0][stage buffer 1][2 mbarriers, 2 stage counters].  A stage buffer
+// holds event and predecessor records only (adj_stage_bytes).
+static KArgs backward_args(const KArgs &a) {
+    KArgs b = a;
+    size_t off = a.win_smem ? (size_t)a.window_slots * kTile * sizeof(uint32_t) : 0;
+    off = (off + 127) / 128 * 128;
+    b.smem_stage_off = (int32_t)off;
+    b.stage_bytes = a.adj_stage_bytes;
+    b.smem_bar_off = (int32_t)(off + 2 * (size_t)a.adj_stage_bytes);
+    b.smem_total = b.smem_bar_off + kBarRegionBytes;
+    return b;
+}
+
+constexpr int kBackwardWarps = 48;  // warps an SM holds at the kernel's registers (at most 42 a thread)
+
 // One CTA per tile of 32 samples; warps take each stage's events one at a time
 // from the stage's counter, stages from a.stage_end - 1 down to a.stage_begin
 // (the whole DAG, or one level block of a recomputation).  Counts of events still
 // to be visited: with the window on chip, the forward window's slots in shared
-// memory -- [counts: window_slots x 32 uint32][stage buffer 0][stage buffer
-// 1][tables][2 mbarriers], the forward layout, whose window rows are twice the
-// size the counts need -- started from and left in a.cnt_ckpt between blocks
-// (kAdjCntLoad / kAdjCntSave); otherwise one uint32 per event and sample in
-// a.cnt_rows (global, by caller index).  Records: row (compiled index -
-// a.code_base) of a.adj_code / a.adj_dfac.
+// memory, started from and left in a.cnt_ckpt between blocks (kAdjCntLoad /
+// kAdjCntSave); otherwise one uint32 per event and sample in a.cnt_rows (global, by
+// caller index).  Records: row (compiled index - a.code_base) of a.adj_code /
+// a.adj_dfac.
+// Bound by latency and instruction issue, not by the 6 bytes an event and sample it
+// reads: an event's records are read one event ahead, its predecessors are walked one
+// by one, uniformly (a vote finds the lanes each of them won), and its sums are one
+// redux each.  The counts and the records alone take 80 KB where the forward's layout
+// takes 166 (10,000 events, 100 a layer), so an SM holds two CTAs and 48 warps.
+// 10,000 events x 65,536 samples: 10.0 ms with the forward's layout, records read when
+// needed and lanes grouped by match, 3.2 ms now.
 template <bool WIN_SMEM>
-__global__ void __launch_bounds__(768) k_adjoint(const KArgs a) {
+__global__ void __launch_bounds__(768, 2) k_adjoint(const KArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     uint32_t *cnt = reinterpret_cast<uint32_t *>(smem);
     char *stage_buf0 = reinterpret_cast<char *>(smem + a.smem_stage_off);
@@ -54,9 +85,11 @@ __global__ void __launch_bounds__(768) k_adjoint(const KArgs a) {
     __syncthreads();
     const int NS = a.stage_end - a.stage_begin;
     if (threadIdx.x == 0) {
-        if (NS > 0) stage_issue(a, a.stage_end - 1, stage_buf0, &bars[0]);
-        if (NS > 1) stage_issue(a, a.stage_end - 2, stage_buf0 + a.stage_bytes, &bars[1]);
+        if (NS > 0) stage_issue<false>(a, a.stage_end - 1, stage_buf0, &bars[0]);
+        if (NS > 1) stage_issue<false>(a, a.stage_end - 2, stage_buf0 + a.stage_bytes, &bars[1]);
     }
+    const uint16_t *codes = a.adj_code + s;
+    const float *dfacs = a.adj_dfac + s;
     for (int j = 0; j < NS; ++j) {  // j-th stage from the end of the range
         const int l = a.stage_end - 1 - j;
         const int b = j & 1;
@@ -75,60 +108,79 @@ __global__ void __launch_bounds__(768) k_adjoint(const KArgs a) {
         const int n_ev = meta.y >= 0 ? meta.y : -meta.y;
         if (threadIdx.x == 0) stage_ctr[(j + 1) & 1] = 0;  // last used by stage j - 1, before the barrier
         const uint32_t ctr = smem_u32(&stage_ctr[j & 1]);
-        // events one at a time from the stage's counter, the next taken ahead
-        int i_next = 0;
-        if (lane == 0) i_next = take_next(ctr);
-        i_next = __shfl_sync(0xFFFFFFFFu, i_next, 0);
+        // events one at a time from the stage's counter, the next taken ahead and its
+        // records with it
+        auto take = [&]() {
+            int i = 0;
+            if (lane == 0) i = take_next(ctr);
+            return __shfl_sync(0xFFFFFFFFu, i, 0);
+        };
+        const int row0 = meta.x - a.code_base;
+        auto read = [&](int i, uint32_t &code, float &dfac) {
+            code = kAdjNone;
+            dfac = 0.0f;
+            if (i < n_ev && active) {
+                const uint64_t o = row_off(row0 + i, (uint32_t)a.ld);
+                code = __ldcs(codes + o);
+                dfac = __ldcs(dfacs + o);
+            }
+        };
+        int i_next = take();
+        uint32_t code_next;
+        float dfac_next;
+        read(i_next, code_next, dfac_next);
         while (i_next < n_ev) {
             const int i = i_next;
-            if (lane == 0) i_next = take_next(ctr);
-            const EvRec ev = load_ev(sev + i);
-            const int64_t o = (int64_t)row_off(meta.x + i - a.code_base, (uint32_t)a.ld) + s;
-            const uint32_t code = active ? (uint32_t)a.adj_code[o] : kAdjNone;
-            const float dfac = active ? a.adj_dfac[o] : 0.0f;
+            const uint32_t code = code_next;
+            const float dfac = dfac_next;
+            i_next = take();
+            read(i_next, code_next, dfac_next);
+            const int4 ev = reinterpret_cast<const int4 *>(sev + i)[0];  // user, slot, pred_begin, pred_end
             const uint32_t k = code & kAdjNone;
             const bool clamped = (code & kAdjClamped) != 0u;
             const bool delayed = (code & kAdjDelayed) != 0u;
             uint32_t c = delayed ? 1u : 0u;
             if (WIN_SMEM) {
-                const int32_t slot = window_row<1>(ev.slot);
+                const int32_t slot = window_row<1>(ev.y);
                 if (slot >= 0) {  // read and clear: the slot's next tenant starts from zero
                     c += cnt[slot * kTile + lane];
                     cnt[slot * kTile + lane] = 0u;
                 }
             } else if (active) {
-                c += a.cnt_rows[(int64_t)row_off(ev.user, (uint32_t)a.ld) + s];
+                c += a.cnt_rows[(int64_t)row_off(ev.x, (uint32_t)a.ld) + s];
             }
             if (!active) c = 0u;
-            // this lane's share of d J / d earliest, >= -1: summed over the warp as ge + 1
-            const long long ge = ((k == kAdjNone || clamped) ? (long long)c : 0ll) - (delayed ? 1ll : 0ll);
-            const long long ge_sum = warp_sum_ticks(ge + 1) - 32;
-            if (lane == 0 && ge_sum != 0)
-                atomicAdd(reinterpret_cast<unsigned long long *>(&a.grad_e[ev.user]), (unsigned long long)ge_sum);
             const bool wins = k != kAdjNone && !clamped && c != 0u;
-            const unsigned wmask = __ballot_sync(0xFFFFFFFFu, wins);
-            if (wins) {
-                const PredRec pr = load_pred(spred + (ev.pred_begin - meta.z + (int)k));
-                if (WIN_SMEM) {
-                    const int32_t slot = window_row<1>(pr.src_slot);
-                    if (slot >= 0) atomicAdd(&cnt[slot * kTile + lane], c);
-                } else {
-                    atomicAdd(&a.cnt_rows[(int64_t)row_off(pr.src_user, (uint32_t)a.ld) + s], c);
+            // d J / d earliest: the counts no predecessor takes over, less one per delayed sample
+            const long long ge = warp_sum(k == kAdjNone || clamped ? (long long)c : 0ll) -
+                                 __popc(__ballot_sync(0xFFFFFFFFu, delayed));
+            if (lane == 0 && ge != 0)
+                atomicAdd(reinterpret_cast<unsigned long long *>(&a.grad_e[ev.x]), (unsigned long long)ge);
+            if (!__any_sync(0xFFFFFFFFu, wins)) continue;
+            // this sample's share of d J / d base of the winning link
+            const long long gl = wins && dfac != 0.0f ? __float2ll_rn((float)c * dfac * (float)(1 << kAdjDfacShift)) : 0ll;
+            const int4 *pred = reinterpret_cast<const int4 *>(spred + (ev.z - meta.z));
+            const int np = ev.w - ev.z;
+            for (int q = 0; q < np; ++q) {
+                const bool won = wins && k == (uint32_t)q;
+                if (!__any_sync(0xFFFFFFFFu, won)) continue;
+                const int4 pr = pred[2 * q];  // src_slot, src_user, link, kd
+                if (won) {
+                    if (WIN_SMEM) {
+                        const int32_t slot = window_row<1>(pr.x);
+                        if (slot >= 0) atomicAdd(&cnt[slot * kTile + lane], c);
+                    } else {
+                        atomicAdd(&a.cnt_rows[(int64_t)row_off(pr.y, (uint32_t)a.ld) + s], c);
+                    }
                 }
-                // lanes whose winner is the same predecessor add their link terms in one atomic
-                const long long gl = (pr.link >= 0 && dfac != 0.0f)
-                                         ? __float2ll_rn((float)c * dfac * (float)(1 << kAdjDfacShift))
-                                         : 0ll;
-                const unsigned grp = __match_any_sync(wmask, k);
-                long long sum = 0;
-                for (unsigned mm = grp; mm; mm &= mm - 1) sum += __shfl_sync(grp, gl, __ffs(mm) - 1);
-                if (lane == __ffs(grp) - 1 && pr.link >= 0 && sum != 0)
-                    atomicAdd(reinterpret_cast<unsigned long long *>(&a.grad_l[pr.link]), (unsigned long long)sum);
+                if (pr.z < 0) continue;
+                const long long sum = warp_sum(won ? gl : 0ll);
+                if (lane == 0 && sum != 0)
+                    atomicAdd(reinterpret_cast<unsigned long long *>(&a.grad_l[pr.z]), (unsigned long long)sum);
             }
-            i_next = __shfl_sync(0xFFFFFFFFu, i_next, 0);
         }
         __syncthreads();
-        if (threadIdx.x == 0 && j + 2 < NS) stage_issue(a, l - 2, stage_buf0 + b * a.stage_bytes, &bars[b]);
+        if (threadIdx.x == 0 && j + 2 < NS) stage_issue<false>(a, l - 2, stage_buf0 + b * a.stage_bytes, &bars[b]);
     }
     if (WIN_SMEM && (a.adj_flags & kAdjCntSave)) {  // counts of earlier events, for the next block down
         uint32_t *out = a.cnt_ckpt + (int64_t)blockIdx.x * cnt_n;
@@ -204,12 +256,14 @@ cudaError_t launch_adjoint_forward(const KArgs &a, cudaStream_t st) {
 // The backward half over stages [a.stage_begin, a.stage_end), last stage first.
 cudaError_t launch_adjoint_backward(const KArgs &a, cudaStream_t st) {
     if (a.n <= 0) return cudaSuccess;
-    const dim3 grid((unsigned)((a.n + kTile - 1) / kTile)), block((unsigned)(pick_warps(a, (int64_t)grid.x) * 32));
-    const size_t smem = (size_t)a.smem_total;
+    const KArgs w = backward_args(a);
+    const dim3 grid((unsigned)((a.n + kTile - 1) / kTile));
+    const dim3 block((unsigned)(pick_warps(w, (int64_t)grid.x, kBackwardWarps) * 32));
+    const size_t smem = (size_t)w.smem_total;
     void (*bwd)(const KArgs) = a.win_smem ? k_adjoint<true> : k_adjoint<false>;
     cudaError_t e = raise_smem_limit((const void *)bwd, smem);
     if (e != cudaSuccess) return e;
-    bwd<<<grid, block, smem, st>>>(a);
+    bwd<<<grid, block, smem, st>>>(w);
     return cudaGetLastError();
 }
 

@@ -38,8 +38,9 @@ namespace mcd {
 // keep the limit they were recorded with.
 cudaError_t raise_smem_limit(const void *fn, size_t smem);
 
-// Warps per CTA of a single-DAG launch over `tiles` tiles.
-int pick_warps(const KArgs &a, int64_t tiles);
+// Warps per CTA of a single-DAG launch over `tiles` tiles (sm_warps: what an SM holds
+// at the kernel's registers).
+int pick_warps(const KArgs &a, int64_t tiles, int sm_warps = 24);
 
 // Wide tiles (two samples a lane) of a sampled launch: whether they run it, and the
 // arguments with their layout in place.
@@ -378,7 +379,8 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
 // region into a buffer.  A stage too large for the buffer (n_ev stored negated)
 // copies nothing; its barrier phase still completes, so the buffers' phases
 // stay in step.  A value region holds an even number of doubles (16-byte sizes
-// and offsets).
+// and offsets); kernels that draw nothing leave it out.
+template <bool VALUES = true>
 __device__ __forceinline__ void stage_issue(const KArgs &a, int stage, char *buf, uint64_t *bar) {
     const int4 *meta = reinterpret_cast<const int4 *>(a.stage_meta + kStageMetaInts * stage);
     const int4 m = __ldg(meta);       // ev_first, n_ev, pred_first, n_pred
@@ -386,7 +388,7 @@ __device__ __forceinline__ void stage_issue(const KArgs &a, int stage, char *buf
     const bool staged = m.y >= 0;
     const uint32_t ev_bytes = staged ? (uint32_t)m.y * (uint32_t)sizeof(EvRec) : 0u;
     const uint32_t pr_bytes = staged ? (uint32_t)m.w * (uint32_t)sizeof(PredRec) : 0u;
-    const uint32_t va_bytes = staged ? (uint32_t)mv.y * (uint32_t)sizeof(double) : 0u;
+    const uint32_t va_bytes = VALUES && staged ? (uint32_t)mv.y * (uint32_t)sizeof(double) : 0u;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     mbar_expect_tx(bar, ev_bytes + pr_bytes + va_bytes);
     if (ev_bytes) bulk_g2s(buf, a.ev + m.x, ev_bytes, bar);
@@ -791,7 +793,7 @@ __device__ __forceinline__ bool propagate_tile(const KArgs &a, int64_t tile, dou
     t.ccol = (!STATS && !ADJ && a.cause && t.active[0]) ? a.cause + t.s : nullptr;
 
     // distribution tables into shared memory; fresh barriers for this tile
-    if (a.tables_in_smem) {  // the tables block, 8 bytes at a time (its size is a multiple of 8)
+    if (!GIVEN && a.tables_in_smem) {  // the tables block, 8 bytes at a time (its size is a multiple of 8)
         const int n8 = (a.n_dist * (int)sizeof(DistParam) + a.n_alias * (int)(sizeof(AliasEntry) + sizeof(AliasPick))) / 8;
         for (int i = threadIdx.x; i < n8; i += blockDim.x)
             reinterpret_cast<uint2 *>(s_dist)[i] = reinterpret_cast<const uint2 *>(a.dist)[i];
@@ -826,8 +828,8 @@ __device__ __forceinline__ bool propagate_tile(const KArgs &a, int64_t tile, dou
     __syncthreads();
     char *stage_buf0 = reinterpret_cast<char *>(smem + a.smem_stage_off);
     if (threadIdx.x == 0) {
-        if (s_begin < s_end) stage_issue(a, s_begin, stage_buf0, &bars[0]);
-        if (s_begin + 1 < s_end) stage_issue(a, s_begin + 1, stage_buf0 + a.stage_bytes, &bars[1]);
+        if (s_begin < s_end) stage_issue<!GIVEN>(a, s_begin, stage_buf0, &bars[0]);
+        if (s_begin + 1 < s_end) stage_issue<!GIVEN>(a, s_begin + 1, stage_buf0 + a.stage_bytes, &bars[1]);
     }
 
     // a stage's metadata is loaded one stage ahead: its latency then hides behind
@@ -879,7 +881,7 @@ __device__ __forceinline__ bool propagate_tile(const KArgs &a, int64_t tile, dou
         }
         __syncthreads();
         if (threadIdx.x == 0 && l + 2 < s_end)
-            stage_issue(a, l + 2, stage_buf0 + b * a.stage_bytes, &bars[b]);
+            stage_issue<!GIVEN>(a, l + 2, stage_buf0 + b * a.stage_bytes, &bars[b]);
     }
     // Aux pass: duration rows of links no precedence entry references.
     if (!STATS && !ADJ && !GIVEN && a.durations) {

@@ -182,8 +182,14 @@ extern "C" int mcd_gradient_host(mcd_dag *g, int64_t seed0, int64_t n, double *o
             cuda_check(cudaMemcpyAsync(d_blk, plan.blk.data() + 1, (n_blk - 1) * 4, cudaMemcpyHostToDevice, st),
                        "block table upload");
         cuda_check(launch_event_ticks(g->d_earliest, h.E, sp.q, te, st), "earliest ticks");
+        int64_t rec_bytes = 0;  // the backward's staging buffers hold no value regions
+        for (int32_t k = 0; k < h.n_stages; ++k) {
+            const int32_t *m = &h.stage_meta[(size_t)k * kStageMetaInts];
+            if (m[1] >= 0) rec_bytes = std::max(rec_bytes, m[6] + (int64_t)m[3] * (int64_t)sizeof(PredRec));
+        }
         for (int64_t off = 0; off < n; off += C) {
             KArgs a = base_args(g);
+            a.adj_stage_bytes = (int32_t)align_up((size_t)rec_bytes, 128);
             a.seeds = nullptr;
             a.seed0 = seed0 + off;
             a.n = std::min(C, n - off);

@@ -258,6 +258,7 @@ struct KArgs {
     long long *grad_l;            // [L] sum over samples of cnt * dfac * 2^20 per link
     // adjoint by level blocks: the kernels run stages [stage_begin, stage_end)
     int32_t stage_begin, stage_end;
+    int32_t adj_stage_bytes;      // one staging buffer of event and predecessor records alone (backward)
     int32_t code_base;            // compiled index of the event whose records are row 0 of adj_code
     int32_t adj_flags;            // kAdjObjective | kAdjCntLoad | kAdjCntSave
     const int32_t *blk_start;     // [n_blk] first stage of each block after the first (checkpoint pass)

@@ -199,11 +199,12 @@ static int deal_warps(int sm_warps, int64_t tiles, int smem) {
 // Measured against the compiler's choice: one sample of 1,000 events 250 -> 172 us
 // (4 -> 14 warps), 20,017 events x 3,001 samples 2.95 -> 1.75 ms (7 -> 24), the
 // statistics of 10,000 events x 65,536 samples 11.1 -> 10.2 ms (19 -> 24).
-int pick_warps(const KArgs &a, int64_t tiles) {
+int pick_warps(const KArgs &a, int64_t tiles, int sm_warps) {
     if (a.max_units <= 0) return a.n_warps;
-    const int nw = deal_warps(24, tiles, a.smem_total);
+    const int nw = deal_warps(sm_warps, tiles, a.smem_total);
     if (nw <= 0) return a.n_warps;
-    const int most = nw < a.max_units ? nw : a.max_units;
+    const int cap = a.max_units < 24 ? a.max_units : 24;  // (CTAs have at most 24 warps)
+    const int most = nw < cap ? nw : cap;
     return 4 * most > 5 * a.n_warps ? most : a.n_warps;
 }
 
