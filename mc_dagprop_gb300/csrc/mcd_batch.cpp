@@ -1,11 +1,12 @@
 // mcd_batch.cpp -- many DAGs, each with its own samples, in one persistent launch.
 //
-// The work is a queue of (DAG, 32-sample tile) items, most expensive DAG first
+// The work is a queue of (DAG, tile of 32 samples, or 64 where the DAG has wide
+// tiles) items, most expensive DAG first
 // (longest-processing-time order), consumed by a persistent grid of CTAs that
 // fills every SM whatever the DAGs' sizes -- a plain per-DAG launch of a DAG
 // with 1,000 samples keeps 32 CTAs busy and leaves the rest of the GPU idle.
 // DAGs are grouped by kernel variant (window on chip or not, tables in shared
-// memory or not, positive times or not); each group is one launch with its own
+// memory or not, positive times or not, wide tiles or not); each group is one launch with its own
 // queue.  Each run is one CUDA
 // graph: reset the accumulators and the queue heads, the persistent statistics
 // launches, the batched finish.  The graph is recorded on the first run and
@@ -21,10 +22,10 @@
 #include "mcd_handle.hpp"
 
 namespace mcd {
-cudaError_t launch_batch_stats(const BatchArgs &b, bool win_smem, bool positive, bool tsmem, int n_warps, size_t smem,
-                               int grid,
-                               cudaStream_t st);
-cudaError_t batch_blocks_per_sm(bool win_smem, bool positive, bool tsmem, int n_warps, size_t smem, int *out);
+cudaError_t launch_batch_stats(const BatchArgs &b, bool win_smem, bool positive, bool tsmem, bool wide, int n_warps,
+                               size_t smem, int grid, cudaStream_t st);
+cudaError_t batch_blocks_per_sm(bool win_smem, bool positive, bool tsmem, bool wide, int n_warps, size_t smem, int *out);
+KArgs wide_args(const KArgs &a);
 cudaError_t launch_batch_finish(const FArgs *fs, int32_t n_dags, int32_t max_events, cudaStream_t st);
 }  // namespace mcd
 
@@ -33,10 +34,11 @@ using namespace mcd;
 namespace {
 // One persistent launch: the DAGs of one kernel variant.
 struct Launch {
-    bool win_smem = true, positive = true, tsmem = true;
+    bool win_smem = true, positive = true, tsmem = true, wide = false;
     std::vector<int32_t> dags;
     size_t smem = 0;
-    int grid = 1;
+    int grid = 1, n_warps = 1;
+    int64_t scratch = 0;  // doubles of off-chip rows a CTA
     BatchArgs args{};
 };
 }  // namespace
@@ -87,22 +89,31 @@ int mcd_batch_create(mcd_dag *const *dags, int32_t n_dags, const int64_t *seed0,
         cuda_check(cudaStreamCreateWithFlags(&B->stream, cudaStreamNonBlocking), "stream create");
         // layout of the batch's device memory; launches by kernel variant
         B->ev_off.resize((size_t)n_dags + 1, 0);
+        std::vector<int32_t> launch_of((size_t)n_dags);
         for (int32_t i = 0; i < n_dags; ++i) {
             const HostDag &h = B->dags[i]->h;
             B->max_E = std::max(B->max_E, h.E);
             B->ev_off[i + 1] = B->ev_off[i] + h.E;
+            // (more than one narrow tile of samples fills a wide one)
+            const bool wide = h.wide_rows > 0 && B->n[i] > kTile;
             Launch *L = nullptr;
             for (Launch &x : B->launches)
-                if (x.win_smem == h.win_smem && x.positive == h.positive && x.tsmem == h.tables_in_smem) L = &x;
+                if (x.win_smem == h.win_smem && x.positive == h.positive && x.tsmem == h.tables_in_smem && x.wide == wide)
+                    L = &x;
             if (!L) {
                 B->launches.emplace_back();
                 L = &B->launches.back();
                 L->win_smem = h.win_smem;
                 L->positive = h.positive;
                 L->tsmem = h.tables_in_smem;
+                L->wide = wide;
             }
             L->dags.push_back(i);
-            L->smem = std::max(L->smem, (size_t)h.smem_total);
+            launch_of[(size_t)i] = (int32_t)(L - B->launches.data());
+            L->smem = std::max(L->smem, (size_t)(wide ? h.wide_total : h.smem_total));
+            if (wide) L->scratch = std::max(L->scratch, (int64_t)h.window_spill * kWideTile);
+            else if (!h.win_smem) L->scratch = std::max(L->scratch, (int64_t)h.E * kTile);
+            B->n_items += (B->n[i] + kTile - 1) / kTile;
         }
         B->total_E = B->ev_off[n_dags];
         int sms = 0;
@@ -111,30 +122,34 @@ int mcd_batch_create(mcd_dag *const *dags, int32_t n_dags, const int64_t *seed0,
         auto cost = [&](int32_t i) { return (double)B->dags[i]->h.pred.size() + 2.0 * B->dags[i]->h.E; };
         std::vector<int32_t> items;
         std::vector<size_t> item_off;  // first item of each launch
-        int32_t max_E_global = 0;
-        int grid_global = 0;
+        int64_t scratch_all = 0;  // doubles; launches run one after another
         B->grid = 0;
         for (Launch &L : B->launches) {
+            // a wide CTA takes twice the shared memory, so fewer fit an SM: its 24 warps
+            // are dealt out over those
+            L.n_warps = B->n_warps;
+            if (L.wide) {
+                const int fit = (int)std::max<size_t>(1, (227 * 1024) / (L.smem + 1024));
+                L.n_warps = std::max(B->n_warps, kMaxBatchWarps / std::min(fit, (int)kMaxBatchWarps));
+            }
             int per_sm = 0;
-            cuda_check(batch_blocks_per_sm(L.win_smem, L.positive, L.tsmem, B->n_warps, L.smem, &per_sm),
+            cuda_check(batch_blocks_per_sm(L.win_smem, L.positive, L.tsmem, L.wide, L.n_warps, L.smem, &per_sm),
                        "occupancy query");
             L.grid = std::max(1, per_sm) * std::max(1, sms);
             B->grid += L.grid;
             std::stable_sort(L.dags.begin(), L.dags.end(), [&](int32_t x, int32_t y) { return cost(x) > cost(y); });
             item_off.push_back(items.size() / 2);
             for (int32_t i : L.dags) {
-                if (!L.win_smem) max_E_global = std::max(max_E_global, B->dags[i]->h.E);
-                const int64_t tiles = (B->n[i] + kTile - 1) / kTile;
+                const int64_t tile = L.wide ? kWideTile : kTile, tiles = (B->n[i] + tile - 1) / tile;
                 for (int64_t t = 0; t < tiles; ++t) {
                     items.push_back(i);
                     items.push_back((int32_t)t);
                 }
             }
             L.args.n_items = (int32_t)(items.size() / 2 - item_off.back());
-            if (!L.win_smem) grid_global = std::max(grid_global, L.grid);  // launches run one after another
+            scratch_all = std::max(scratch_all, L.scratch * L.grid);
         }
-        B->n_items = (int64_t)items.size() / 2;
-        if (B->n_items > (int64_t)INT32_MAX) throw McdError(MCD_ERR_INVALID, "too many work items");
+        if ((int64_t)items.size() / 2 > (int64_t)INT32_MAX) throw McdError(MCD_ERR_INVALID, "too many work items");
         const size_t E = (size_t)B->total_E;
         // one queue head per launch, 64 bytes apart (up to eight kernel variants)
         const size_t s_acc = align_up(E * 8, 256), s_hist = align_up(E * kHistStride * 4, 256),
@@ -143,7 +158,7 @@ int mcd_batch_create(mcd_dag *const *dags, int32_t n_dags, const int64_t *seed0,
                      s_args = align_up((size_t)n_dags * sizeof(KArgs), 256),
                      s_fargs = align_up((size_t)n_dags * sizeof(FArgs), 256),
                      s_items = align_up(items.size() * 4, 256),
-                     s_scr = align_up((size_t)grid_global * max_E_global * kTile * 8, 256);
+                     s_scr = align_up((size_t)scratch_all * 8, 256);
         B->zero_bytes = s_acc + s_hist + s_ctr;
         cuda_check(cudaMalloc(&B->dmem, B->zero_bytes + s_out + s_te + s_args + s_fargs + s_items + s_scr),
                    "batch allocation");
@@ -183,6 +198,11 @@ int mcd_batch_create(mcd_dag *const *dags, int32_t n_dags, const int64_t *seed0,
             a.te = d_te + B->ev_off[i];
             a.hist = B->hist + (size_t)B->ev_off[i] * kHistStride;
             ka[i] = a;
+            const Launch &L = B->launches[(size_t)launch_of[(size_t)i]];
+            if (L.wide) {
+                ka[i] = wide_args(a);
+                ka[i].n_warps = L.n_warps;
+            }
             for (int32_t e = 0; e < g->h.E; ++e) {
                 long long b;
                 std::memcpy(&b, &g->h.earliest[(size_t)e], 8);
@@ -213,8 +233,8 @@ int mcd_batch_create(mcd_dag *const *dags, int32_t n_dags, const int64_t *seed0,
             L.args.dags = d_args;
             L.args.items = d_items + 2 * item_off[k];
             L.args.counter = counter + 16 * k;  // one queue head per launch, 64 bytes apart
-            L.args.scratch = L.win_smem ? nullptr : scratch;
-            L.args.scratch_stride = L.win_smem ? 0 : (int64_t)max_E_global * kTile;
+            L.args.scratch = L.scratch ? scratch : nullptr;
+            L.args.scratch_stride = L.scratch;
             L.args.smem_bytes = (int32_t)L.smem;
         }
         *out = B;
@@ -247,7 +267,7 @@ int mcd_batch_run(mcd_batch *B) {
             cudaError_t e = cudaMemsetAsync(B->dmem, 0, B->zero_bytes, B->stream);
             for (const Launch &L : B->launches)
                 if (e == cudaSuccess)
-                    e = launch_batch_stats(L.args, L.win_smem, L.positive, L.tsmem, B->n_warps, L.smem, L.grid,
+                    e = launch_batch_stats(L.args, L.win_smem, L.positive, L.tsmem, L.wide, L.n_warps, L.smem, L.grid,
                                            B->stream);
             if (e == cudaSuccess)
                 e = launch_batch_finish(B->d_fargs, (int32_t)B->dags.size(), B->max_E, B->stream);
@@ -277,7 +297,7 @@ int mcd_batch_occupancy(int32_t n_warps, int64_t smem_bytes, int32_t *blocks_per
             smem_bytes > (int64_t)kSmemMax)
             throw McdError(MCD_ERR_INVALID, "bad arguments");
         int per_sm = 0;
-        cuda_check(batch_blocks_per_sm(true, true, true, n_warps, (size_t)smem_bytes, &per_sm), "occupancy query");
+        cuda_check(batch_blocks_per_sm(true, true, true, false, n_warps, (size_t)smem_bytes, &per_sm), "occupancy query");
         *blocks_per_sm = per_sm;
     });
 }

@@ -15,7 +15,8 @@ namespace mcd {
 // Each DAG has its own shared-memory layout; the barrier pair and the stage
 // counters live outside all of them, in static shared memory, so they never
 // move between items.
-template <bool WIN_SMEM, bool POSITIVE, bool TSMEM>
+// S: samples a lane (2: wide tiles, whose off-chip window rows are the CTA's scratch).
+template <bool WIN_SMEM, bool POSITIVE, bool TSMEM, int S = 1>
 __global__ void __launch_bounds__(768, 1) k_batch_stats(const BatchArgs b) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ KArgs s_args;
@@ -38,18 +39,20 @@ __global__ void __launch_bounds__(768, 1) k_batch_stats(const BatchArgs b) {
             __syncthreads();
             continue;
         }
-        double *rows = WIN_SMEM ? nullptr : b.scratch + (int64_t)blockIdx.x * b.scratch_stride;
+        double *mine = b.scratch + (int64_t)blockIdx.x * b.scratch_stride;
+        double *rows = WIN_SMEM ? nullptr : mine;
         // (many DAGs' histogram counters at once: a warp's equal bins added once)
         const bool ok = propagate_tile<false, WIN_SMEM, true, POSITIVE, false, TSMEM ? kTablesSmem : kTablesGlobal,
-                                       false>(
-            a, it.y, rows, WIN_SMEM ? 0 : kTile, true, smem, s_bars, reuse);
+                                       false, S>(
+            a, it.y, rows, WIN_SMEM ? 0 : kTile, true, smem, s_bars, reuse, S > 1 && a.window_spill ? mine : nullptr);
         reuse = true;
         if (!ok) return;
         __syncthreads();  // s_args / s_item are rewritten by the next item
     }
 }
 
-static void (*batch_kernel(bool win_smem, bool positive, bool tsmem))(const BatchArgs) {
+static void (*batch_kernel(bool win_smem, bool positive, bool tsmem, bool wide))(const BatchArgs) {
+    if (wide) return k_batch_stats<true, true, true, 2>;
     if (tsmem) {
         if (win_smem) return positive ? k_batch_stats<true, true, true> : k_batch_stats<true, false, true>;
         return positive ? k_batch_stats<false, true, true> : k_batch_stats<false, false, true>;
@@ -83,9 +86,9 @@ cudaError_t launch_prop_sample(const KArgs &a, bool win_smem, bool stats, bool p
 }
 
 // Persistent batch launch: one CTA per SM slot, `blocks_per_sm` of them per SM.
-cudaError_t launch_batch_stats(const BatchArgs &b, bool win_smem, bool positive, bool tsmem, int n_warps, size_t smem,
-                               int grid, cudaStream_t st) {
-    void (*fn)(const BatchArgs) = batch_kernel(win_smem, positive, tsmem);
+cudaError_t launch_batch_stats(const BatchArgs &b, bool win_smem, bool positive, bool tsmem, bool wide, int n_warps,
+                               size_t smem, int grid, cudaStream_t st) {
+    void (*fn)(const BatchArgs) = batch_kernel(win_smem, positive, tsmem, wide);
     const cudaError_t e = raise_smem_limit((const void *)fn, smem);
     if (e != cudaSuccess) return e;
     fn<<<grid, n_warps * 32, smem, st>>>(b);
@@ -93,8 +96,8 @@ cudaError_t launch_batch_stats(const BatchArgs &b, bool win_smem, bool positive,
 }
 
 // CTAs of the batch kernel that fit on one SM at this block size and shared memory.
-cudaError_t batch_blocks_per_sm(bool win_smem, bool positive, bool tsmem, int n_warps, size_t smem, int *out) {
-    void (*fn)(const BatchArgs) = batch_kernel(win_smem, positive, tsmem);
+cudaError_t batch_blocks_per_sm(bool win_smem, bool positive, bool tsmem, bool wide, int n_warps, size_t smem, int *out) {
+    void (*fn)(const BatchArgs) = batch_kernel(win_smem, positive, tsmem, wide);
     const cudaError_t e = raise_smem_limit((const void *)fn, smem);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, fn, n_warps * 32, smem);

@@ -44,10 +44,9 @@
 #include "mcd_handle.hpp"
 
 namespace mcd {
-cudaError_t launch_batch_stats(const BatchArgs &b, bool win_smem, bool positive, bool tsmem, int n_warps, size_t smem,
-                               int grid,
-                               cudaStream_t st);
-cudaError_t batch_blocks_per_sm(bool win_smem, bool positive, bool tsmem, int n_warps, size_t smem, int *out);
+cudaError_t launch_batch_stats(const BatchArgs &b, bool win_smem, bool positive, bool tsmem, bool wide, int n_warps,
+                               size_t smem, int grid, cudaStream_t st);
+cudaError_t batch_blocks_per_sm(bool win_smem, bool positive, bool tsmem, bool wide, int n_warps, size_t smem, int *out);
 cudaError_t launch_batch_finish(const FArgs *fs, int32_t n_dags, int32_t max_events, cudaStream_t st);
 }  // namespace mcd
 
@@ -474,7 +473,7 @@ void compile_loop(mcd_server *S) {
                     if ((int64_t)(R->bytes + rq_layout_of(R->h.E).total) > S->opt.memory_budget)
                         throw McdError(MCD_ERR_INVALID, "request needs more device memory than the server's budget");
                     int per_sm = 0;
-                    cuda_check(batch_blocks_per_sm(R->h.win_smem, R->h.positive, R->h.tables_in_smem,
+                    cuda_check(batch_blocks_per_sm(R->h.win_smem, R->h.positive, R->h.tables_in_smem, false,
                                                    R->h.n_warps, (size_t)R->h.smem_total, &per_sm),
                                "occupancy query");
                     R->per_sm = std::max(1, per_sm);
@@ -690,7 +689,7 @@ void launch_batch(mcd_server *S, Slot &slot, std::vector<Request *> &batch) {
         }
         ba.scratch = slot.scratch;
     }
-    cuda_check(launch_batch_stats(ba, h0.win_smem, h0.positive, h0.tables_in_smem, nw, smem, grid, st),
+    cuda_check(launch_batch_stats(ba, h0.win_smem, h0.positive, h0.tables_in_smem, false, nw, smem, grid, st),
                "batch launch");
     cuda_check(launch_batch_finish(reinterpret_cast<const FArgs *>(slot.meta_dev + s_ka), (int32_t)nb, max_E, st),
                "batch finish");

@@ -66,3 +66,18 @@ def test_large_windows_keep_rows_off_chip(cuda):
     rest = [i["smem_bytes"] - i["window_slots"] * 256 for i in info]
     assert info[0]["window_in_smem"] and info[0]["window_slots"] * row + rest[0] <= 226 * 1024
     assert info[1]["window_in_smem"] and info[1]["window_slots"] * row + rest[1] > 226 * 1024
+
+
+def test_batches_run_wide_tiles_with_the_same_statistics(cuda):
+    """A batch's items are wide where the DAG has them; alone, these sample counts run narrow."""
+    from mc_dagprop_gb300 import _core
+
+    ns = [1, 32, 33, 64, 95, 3000]
+    props = [batching.compile_dag(*kitchen_sink(seed=30 + i, n_layers=5, width=w), 8)
+             for i, w in enumerate([60, 130, 130, 60, 130, 130])]
+    batch = _core.Batch(props, list(range(len(ns))), ns)
+    for _ in range(2):
+        batch.run()
+    for i, (p, n) in enumerate(zip(props, ns)):
+        a, b = batch.stats(i, True), p.run_stats(n=n, seed0=i, hist=True)
+        assert all(np.array_equal(a[k], b[k]) for k in ("mean", "p50", "p90", "p99", "p_on_time", "hist")), i
