@@ -38,9 +38,9 @@ namespace mcd {
 // keep the limit they were recorded with.
 cudaError_t raise_smem_limit(const void *fn, size_t smem);
 
-// Warps per CTA of a single-DAG launch over `tiles` tiles (sm_warps: what an SM holds
-// at the kernel's registers).
-int pick_warps(const KArgs &a, int64_t tiles, int sm_warps = 24);
+// Warps per CTA of a single-DAG launch over `tiles` tiles (sm_warps, cta_warps: what an
+// SM and a CTA hold at the kernel's registers).
+int pick_warps(const KArgs &a, int64_t tiles, int sm_warps = 24, int cta_warps = 24);
 
 // Wide tiles (two samples a lane) of a sampled launch: whether they run it, and the
 // arguments with their layout in place.
@@ -95,7 +95,7 @@ __device__ __forceinline__ float u01_open0(uint32_t r) {
 // the host), for which the bit pattern itself is the key.
 template <bool POSITIVE>
 __device__ __forceinline__ long long order_key(long long b) {
-    if (POSITIVE) return b;
+    if (POSITIVE || (uint32_t)(b >> 32) < 0x7FF00000u) return b;  // (non-negative and finite)
     const long long mag = b & 0x7FFFFFFFFFFFFFFFll;
     const long long k = b < 0 ? -mag : mag;
     return mag > 0x7FF0000000000000ll ? (long long)0x8000000000000000ull : k;
@@ -540,6 +540,148 @@ __device__ __forceinline__ int take_next(uint32_t ctr) {
     return v;
 }
 
+// The realized times of a predecessor: from the window row of its slot; a wide
+// tile's predecessor without one (see window_row) from its off-chip window row
+// or, where the realized times are an output, from that; window off chip: from
+// the realized rows.
+template <bool WIN_SMEM, int S>
+__device__ __forceinline__ void source(const TileCtx<S> &t, const double *win, int32_t slots, int32_t user,
+                                       double (&v)[S]) {
+    if (WIN_SMEM) {
+        const int32_t slot = window_row<S>(slots);
+        if (S == 1 || slot >= 0) {
+#pragma unroll
+            for (int j = 0; j < S; ++j) v[j] = win[slot * (kTile * S) + t.lane + 32 * j];
+            return;
+        }
+        if (t.scol) {
+#pragma unroll
+            for (int j = 0; j < S; ++j) v[j] = __ldcg(t.scol + (~slot) * (kTile * S) + 32 * j);
+            return;
+        }
+    }
+    const double *row = at_row(t.rcol, user, t.rows_ld8);
+#pragma unroll
+    for (int j = 0; j < S; ++j) v[j] = t.active[j] ? row[32 * j] : 0.0;
+}
+
+// One entry of one sample (_core.cpp:341-347): the one FP64 add of the edge, the
+// clamp t = std::min(t, ub), and if (t >= latest) { latest = t; cause = src; } --
+// true when the entry takes the maximum over.
+template <bool POSITIVE>
+__device__ __forceinline__ bool relax(double src, double dur, long long ub_key, long long ub_bits, long long &lk,
+                                      long long &lbits, bool &clamp) {
+    const double tt = src + dur;
+    long long tb = __double_as_longlong(tt);
+    long long tk = order_key<POSITIVE>(tb);
+    clamp = ub_key < tk;
+    if (clamp) {
+        tk = ub_key;
+        tb = ub_bits;
+    }
+    if (tk < lk) return false;
+    lk = tk;
+    lbits = POSITIVE ? tk : tb;
+    return true;
+}
+
+// One stage's events under given durations, one at a time from the stage's counter
+// (no draws, so no pairs).  The durations are uncached DRAM reads: an event's first
+// kGivenAhead entries are read while the event before it runs, later ones when
+// reached.  Without the sampler the kernel fits 64 registers, so 32 warps an SM.
+// 200,000 events x 4,864 samples: reads four at a time when reached, 24 warps 13.2 ms
+// (2.3 TB/s); one event ahead, 32 warps 9.6 (3.2 TB/s).  20,017 events x 3,001
+// samples 3.5 -> 1.45 ms.  Prefetching the next stage's rows into L2 gained 2 %.
+constexpr int kGivenAhead = 4;
+template <bool WIN_SMEM, int S>
+__device__ __forceinline__ void stage_given(const KArgs &a, const EvRec *sev, const PredRec *spred, int pred0, int n_ev,
+                                            uint32_t ctr, const TileCtx<S> &t, unsigned char *smem) {
+    double *win = reinterpret_cast<double *>(smem);
+    auto take = [&]() {
+        int i = 0;
+        if (t.lane == 0) i = take_next(ctr);
+        return __shfl_sync(0xFFFFFFFFu, i, 0);
+    };
+    auto duration = [&](int32_t link, double (&d)[S]) {
+#pragma unroll
+        for (int j = 0; j < S; ++j) d[j] = 0.0;
+        if (link < 0) return;
+        const double *row = at_row(t.dincol, link, t.ld_in8);
+#pragma unroll
+        for (int j = 0; j < S; ++j)
+            if (t.active[j]) d[j] = __ldcs(row + 32 * j);
+    };
+    auto read = [&](int i, double (&d)[kGivenAhead][S]) {
+        if (i >= n_ev) return;
+        const int4 e = reinterpret_cast<const int4 *>(sev + i)[0];  // user, slot, pred_begin, pred_end
+#pragma unroll
+        for (int k = 0; k < kGivenAhead; ++k)
+            if (e.z + k < e.w) duration(reinterpret_cast<const int4 *>(spred + (e.z - pred0 + k))->z, d[k]);
+    };
+    int i_next = take();
+    double d[kGivenAhead][S], d_next[kGivenAhead][S];
+    read(i_next, d_next);
+    while (i_next < n_ev) {
+        const int i = i_next;
+#pragma unroll
+        for (int k = 0; k < kGivenAhead; ++k)
+#pragma unroll
+            for (int j = 0; j < S; ++j) d[k][j] = d_next[k][j];
+        i_next = take();
+        read(i_next, d_next);
+        const EvRec ev = load_ev(sev + i);
+        long long lk[S], lbits[S];
+        int32_t cause[S];
+#pragma unroll
+        for (int j = 0; j < S; ++j) {
+            lk[j] = ev.init_key;
+            lbits[j] = ev.init_bits;
+            cause[j] = -1;
+        }
+        const int pb = ev.pred_begin - pred0, np = ev.pred_end - ev.pred_begin;
+        auto entry = [&](int4 rec, const double (&dur)[S]) {
+            double src[S];
+            source<WIN_SMEM, S>(t, win, rec.x, rec.y, src);
+#pragma unroll
+            for (int j = 0; j < S; ++j) {
+                bool clamp;
+                if (relax<false>(src[j], dur[j], ev.ub_key, ev.ub_bits, lk[j], lbits[j], clamp)) cause[j] = rec.y;
+            }
+        };
+#pragma unroll
+        for (int k = 0; k < kGivenAhead; ++k)
+            if (k < np) entry(reinterpret_cast<const int4 *>(spred + pb + k)[0], d[k]);
+        for (int k = kGivenAhead; k < np; ++k) {
+            const int4 rec = reinterpret_cast<const int4 *>(spred + pb + k)[0];
+            double dur[S];
+            duration(rec.z, dur);
+            entry(rec, dur);
+        }
+#pragma unroll
+        for (int j = 0; j < S; ++j)
+            if (ev.ub_key < lk[j]) lbits[j] = ev.ub_bits;  // realized = std::min(latest, ub)
+        if (WIN_SMEM) {
+            const int32_t slot = window_row<S>(ev.slot);
+            if (slot >= 0) {
+#pragma unroll
+                for (int j = 0; j < S; ++j) win[slot * (kTile * S) + t.lane + 32 * j] = __longlong_as_double(lbits[j]);
+            }
+        }
+        if (t.rcol && t.active[0]) {
+            double *row = at_row(t.rcol, ev.user, t.rows_ld8);
+#pragma unroll
+            for (int j = 0; j < S; ++j)
+                if (j == 0 || t.active[j]) row[32 * j] = __longlong_as_double(lbits[j]);
+        }
+        if (t.ccol) {
+            int32_t *row = at_row(t.ccol, ev.user, t.ld4);
+#pragma unroll
+            for (int j = 0; j < S; ++j)
+                if (j == 0 || t.active[j]) row[32 * j] = cause[j];
+        }
+    }
+}
+
 // One stage's work units, taken one at a time from the stage's counter: unit
 // u < n_pair is the pair of events 2u and 2u + 1, run back to back so that the
 // second continues the first's Philox block (grp); unit u >= n_pair is event
@@ -549,34 +691,12 @@ __device__ __forceinline__ int take_next(uint32_t ctr) {
 // global memory.  pred0: the stage's first predecessor record (the records'
 // pred_begin/pred_end are global indices); ev0: its first event's compiled
 // index; buf: the staging buffer (0 or 1) that holds the stage.
-template <bool GIVEN, bool WIN_SMEM, bool STATS, bool POSITIVE, bool ADJ, bool STAGED, int TS, bool LANE_HIST, int S>
+template <bool WIN_SMEM, bool STATS, bool POSITIVE, bool ADJ, bool STAGED, int TS, bool LANE_HIST, int S>
 __device__ __forceinline__ void stage_events(const KArgs &a, int buf, const EvRec *sev, const PredRec *spred, int pred0,
                                              int ev0, int n_ev, int n_pair, uint32_t ctr, const TileCtx<S> &t,
                                              unsigned char *smem, U4 (&grp)[S]) {
     double *win = reinterpret_cast<double *>(smem);
     const int lane = t.lane;
-    // The realized times of a predecessor: from the window row of its slot; a wide
-    // tile's predecessor without one (see window_row) from its off-chip window row
-    // or, where the realized times are an output, from that; window off chip: from
-    // the realized rows.
-    auto source = [&](int32_t slots, int32_t user, double (&v)[S]) {
-        if (WIN_SMEM) {
-            const int32_t slot = window_row<S>(slots);
-            if (S == 1 || slot >= 0) {
-#pragma unroll
-                for (int j = 0; j < S; ++j) v[j] = win[slot * (kTile * S) + lane + 32 * j];
-                return;
-            }
-            if (t.scol) {
-#pragma unroll
-                for (int j = 0; j < S; ++j) v[j] = __ldcg(t.scol + (~slot) * (kTile * S) + 32 * j);
-                return;
-            }
-        }
-        const double *row = at_row(t.rcol, user, t.rows_ld8);
-#pragma unroll
-        for (int j = 0; j < S; ++j) v[j] = t.active[j] ? row[32 * j] : 0.0;
-    };
     // The warp's next event: the second of the current pair, or the first event of
     // the next unit, which lane 0 takes before this event's work, hiding the
     // atomic's latency (a warp holds at most one extra unit: the cheapest, by
@@ -617,61 +737,11 @@ __device__ __forceinline__ void stage_events(const KArgs &a, int buf, const EvRe
             win_dfac[j] = 0.0f;
         }
         const int pb = ev.pred_begin - pred0, pe = ev.pred_end - pred0;
-        // One entry of one sample (_core.cpp:341-347): the one FP64 add of the edge, the
-        // clamp t = std::min(t, ub), and if (t >= latest) { latest = t; cause = src; }.
-        auto relax = [&](int j, double src, double dur, int32_t user, int at, float dfac) {
-            const double tt = src + dur;
-            long long tb = __double_as_longlong(tt);
-            long long tk = order_key<POSITIVE>(tb);
-            const bool clamp = ub_key < tk;
-            if (clamp) {
-                tk = ub_key;
-                tb = ev.ub_bits;
-            }
-            if (tk >= lk[j]) {
-                lk[j] = tk;
-                lbits[j] = POSITIVE ? tk : tb;
-                cause[j] = user;
-                if (ADJ) {
-                    win_code[j] = (uint32_t)at | (clamp ? kAdjClamped : 0u);
-                    win_dfac[j] = dfac;
-                }
-            }
-        };
-        // Given durations come from global memory, each an uncached DRAM read: the
-        // reads of up to four entries are issued together, then the entries are
-        // relaxed in order (one memory latency per four entries, not per entry).
-        for (int p0 = pb; GIVEN && p0 < pe; p0 += 4) {
-            double dg[4][S];
-            int4 rec[4];  // PredRec: src_slot, src_user, link, kd
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-#pragma unroll
-                for (int j = 0; j < S; ++j) dg[k][j] = 0.0;
-                if (p0 + k < pe) {
-                    rec[k] = reinterpret_cast<const int4 *>(spred + p0 + k)[0];
-                    if (rec[k].z >= 0) {
-                        const double *row = at_row(t.dincol, rec[k].z, t.ld_in8);
-#pragma unroll
-                        for (int j = 0; j < S; ++j)
-                            if (t.active[j]) dg[k][j] = __ldg(row + 32 * j);
-                    }
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                if (p0 + k >= pe) continue;
-                double src[S];
-                source(rec[k].x, rec[k].y, src);
-#pragma unroll
-                for (int j = 0; j < S; ++j) relax(j, src[j], dg[k][j], rec[k].y, p0 + k - pb, 0.0f);
-            }
-        }
-        for (int p = pb; !GIVEN && p < pe; ++p) {
+        for (int p = pb; p < pe; ++p) {
             const PredRec pr = load_pred(spred + p);
             double src[S], dur[S];
             float dfac[S];
-            if (S > 1) source(pr.src_slot, pr.src_user, src);  // (may come from L2: ahead of the draws)
+            if (S > 1) source<WIN_SMEM, S>(t, win, pr.src_slot, pr.src_user, src);  // (may come from L2: ahead of the draws)
             link_duration<STAGED, TS, S>(a, pr.kd, pr.v, pr.dvo, (uint32_t)pr.block, (uint32_t)pr.link, t.seed, grp, smem,
                                          buf, dur, dfac);
             if (!STATS && !ADJ && (pr.kd & KD_WRITE) && t.dcol) {
@@ -680,9 +750,18 @@ __device__ __forceinline__ void stage_events(const KArgs &a, int buf, const EvRe
                 for (int j = 0; j < S; ++j)
                     if (j == 0 || t.active[j]) row[32 * j] = dur[j];
             }
-            if (S == 1) source(pr.src_slot, pr.src_user, src);
+            if (S == 1) source<WIN_SMEM, S>(t, win, pr.src_slot, pr.src_user, src);
 #pragma unroll
-            for (int j = 0; j < S; ++j) relax(j, src[j], dur[j], pr.src_user, p - pb, dfac[j]);
+            for (int j = 0; j < S; ++j) {
+                bool clamp;
+                if (relax<POSITIVE>(src[j], dur[j], ub_key, ev.ub_bits, lk[j], lbits[j], clamp)) {
+                    cause[j] = pr.src_user;
+                    if (ADJ) {
+                        win_code[j] = (uint32_t)(p - pb) | (clamp ? kAdjClamped : 0u);
+                        win_dfac[j] = dfac[j];
+                    }
+                }
+            }
         }
         // realized = std::min(latest, ub): latest only exceeds ub when earliest does, which
         // non-negative max_delay rules out in POSITIVE mode
@@ -872,11 +951,18 @@ __device__ __forceinline__ bool propagate_tile(const KArgs &a, int64_t tile, dou
         const uint32_t ctr = smem_u32(&stage_ctr[j & 1]);
         if (meta.y >= 0) {  // records in the staging buffer (shared memory)
             const unsigned char *buf = smem + a.smem_stage_off + b * a.stage_bytes;
-            stage_events<GIVEN, WIN_SMEM, STATS, POSITIVE, ADJ, true, TS, LANE_HIST, S>(
+            if constexpr (GIVEN)
+                stage_given<WIN_SMEM, S>(a, reinterpret_cast<const EvRec *>(buf), reinterpret_cast<const PredRec *>(buf + mv.z),
+                                         meta.z, meta.y, ctr, t, smem);
+            else
+                stage_events<WIN_SMEM, STATS, POSITIVE, ADJ, true, TS, LANE_HIST, S>(
                 a, b, reinterpret_cast<const EvRec *>(buf), reinterpret_cast<const PredRec *>(buf + mv.z), meta.z,
                 meta.x, meta.y, n_pair, ctr, t, smem, grp);
         } else {  // a stage whose records exceed the buffer is read from global memory
-            stage_events<GIVEN, WIN_SMEM, STATS, POSITIVE, ADJ, false, TS, LANE_HIST, S>(
+            if constexpr (GIVEN)
+                stage_given<WIN_SMEM, S>(a, a.ev + meta.x, a.pred + meta.z, meta.z, -meta.y, ctr, t, smem);
+            else
+                stage_events<WIN_SMEM, STATS, POSITIVE, ADJ, false, TS, LANE_HIST, S>(
                 a, b, a.ev + meta.x, a.pred + meta.z, meta.z, meta.x, -meta.y, n_pair, ctr, t, smem, grp);
         }
         __syncthreads();
@@ -905,14 +991,24 @@ __device__ __forceinline__ bool propagate_tile(const KArgs &a, int64_t tile, dou
 
 // One CTA per tile of 32 S samples.  TS: the tables block's place (kTablesGlobal or
 // kTablesSmem; the host launches the instantiation that matches the DAG).
-template <bool GIVEN, bool WIN_SMEM, bool STATS, bool POSITIVE, int TS, int S = 1>
+template <bool WIN_SMEM, bool STATS, bool POSITIVE, int TS, int S = 1>
 __global__ void __launch_bounds__(768, 1) k_propagate(const KArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     double *rows = a.realized ? a.realized : a.scratch;  // global realized rows
     if (STATS && WIN_SMEM) rows = nullptr;
     double *spill = S > 1 && a.spill ? a.spill + (int64_t)blockIdx.x * a.window_spill * (kTile * S) : nullptr;
-    propagate_tile<GIVEN, WIN_SMEM, STATS, POSITIVE, false, TS, true, S>(
+    propagate_tile<false, WIN_SMEM, STATS, POSITIVE, false, TS, true, S>(
         a, (int64_t)blockIdx.x, rows, a.ld, false, smem, reinterpret_cast<uint64_t *>(smem + a.smem_bar_off), false, spill);
+}
+
+// The same with given durations (a.dur_in), which may be anything.
+constexpr int kGivenWarps = 32;  // most warps of a CTA, and of an SM (64 registers a thread)
+template <bool WIN_SMEM, int S>
+__global__ void __launch_bounds__(kGivenWarps * 32, 1) k_propagate_given(const KArgs a) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    propagate_tile<true, WIN_SMEM, false, false, false, kTablesEither, true, S>(
+        a, (int64_t)blockIdx.x, a.realized ? a.realized : a.scratch, a.ld, false, smem,
+        reinterpret_cast<uint64_t *>(smem + a.smem_bar_off), false);
 }
 
 }  // namespace mcd

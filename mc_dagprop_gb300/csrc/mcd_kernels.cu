@@ -199,11 +199,11 @@ static int deal_warps(int sm_warps, int64_t tiles, int smem) {
 // Measured against the compiler's choice: one sample of 1,000 events 250 -> 172 us
 // (4 -> 14 warps), 20,017 events x 3,001 samples 2.95 -> 1.75 ms (7 -> 24), the
 // statistics of 10,000 events x 65,536 samples 11.1 -> 10.2 ms (19 -> 24).
-int pick_warps(const KArgs &a, int64_t tiles, int sm_warps) {
+int pick_warps(const KArgs &a, int64_t tiles, int sm_warps, int cta_warps) {
     if (a.max_units <= 0) return a.n_warps;
     const int nw = deal_warps(sm_warps, tiles, a.smem_total);
     if (nw <= 0) return a.n_warps;
-    const int cap = a.max_units < 24 ? a.max_units : 24;  // (CTAs have at most 24 warps)
+    const int cap = a.max_units < cta_warps ? a.max_units : cta_warps;
     const int most = nw < cap ? nw : cap;
     return 4 * most > 5 * a.n_warps ? most : a.n_warps;
 }
@@ -240,14 +240,14 @@ KArgs wide_args(const KArgs &a) {
 cudaError_t launch_prop_wide(const KArgs &w, bool stats, dim3 grid, dim3 block, size_t smem, cudaStream_t st);
 cudaError_t launch_prop_sample(const KArgs &a, bool win_smem, bool stats, bool positive, dim3 grid, dim3 block,
                                size_t smem, cudaStream_t st);
-cudaError_t launch_prop_given(const KArgs &a, bool win_smem, bool stats, dim3 grid, dim3 block, size_t smem,
-                              cudaStream_t st);
+cudaError_t launch_prop_given(const KArgs &a, bool win_smem, cudaStream_t st);
 
 // One launch of the propagation kernel over a.n samples: one CTA per tile of 32.
 // The shared-memory layout is fixed by the host compiler (KArgs::smem_*).
 cudaError_t launch_propagate(const KArgs &a, bool given, bool win_smem, bool stats, cudaStream_t st) {
     if (a.n <= 0) return cudaSuccess;
-    if (!given && win_smem && use_wide(a)) {
+    if (given) return launch_prop_given(a, win_smem, st);
+    if (win_smem && use_wide(a)) {
         const KArgs w = wide_args(a);
         const dim3 grid((unsigned)((a.n + kWideTile - 1) / kWideTile));
         return launch_prop_wide(w, stats, grid, dim3((unsigned)(pick_warps(w, grid.x) * 32)), (size_t)w.smem_total, st);
@@ -255,7 +255,6 @@ cudaError_t launch_propagate(const KArgs &a, bool given, bool win_smem, bool sta
     const dim3 grid((unsigned)((a.n + kTile - 1) / kTile));
     const dim3 block((unsigned)(pick_warps(a, grid.x) * 32));
     const size_t smem = (size_t)a.smem_total;
-    if (given) return launch_prop_given(a, win_smem, stats, grid, block, smem, st);
     return launch_prop_sample(a, win_smem, stats, a.positive != 0, grid, block, smem, st);
 }
 

@@ -1,18 +1,18 @@
-// mcd_prop_given.cu -- instantiations of k_propagate that read given durations.
+// mcd_prop_given.cu -- the propagation of given durations.
 #include "mcd_device.cuh"
 
 namespace mcd {
 
-cudaError_t launch_prop_given(const KArgs &a, bool win_smem, bool stats, dim3 grid, dim3 block, size_t smem,
-                              cudaStream_t st) {
-    void (*fn)(const KArgs);
-    // (given durations: no sampler, so the tables' place does not matter)
-    constexpr int E = kTablesEither;
-    if (stats) fn = win_smem ? k_propagate<true, true, true, false, E> : k_propagate<true, false, true, false, E>;
-    else fn = win_smem ? k_propagate<true, true, false, false, E> : k_propagate<true, false, false, false, E>;
-    const cudaError_t e = raise_smem_limit((const void *)fn, smem);
+cudaError_t launch_prop_given(const KArgs &a, bool win_smem, cudaStream_t st) {
+    const bool wide = win_smem && use_wide(a);
+    const KArgs w = wide ? wide_args(a) : a;
+    const int tile = wide ? kWideTile : kTile;
+    const dim3 grid((unsigned)((a.n + tile - 1) / tile));
+    void (*fn)(const KArgs) = wide ? k_propagate_given<true, 2>
+                                   : win_smem ? k_propagate_given<true, 1> : k_propagate_given<false, 1>;
+    const cudaError_t e = raise_smem_limit((const void *)fn, (size_t)w.smem_total);
     if (e != cudaSuccess) return e;
-    fn<<<grid, block, smem, st>>>(a);
+    fn<<<grid, (unsigned)(pick_warps(w, grid.x, kGivenWarps, kGivenWarps) * 32), (size_t)w.smem_total, st>>>(w);
     return cudaGetLastError();
 }
 

@@ -73,11 +73,11 @@ cudaError_t launch_prop_sample(const KArgs &a, bool win_smem, bool stats, bool p
     constexpr int S = kTablesSmem;
     void (*fn)(const KArgs);
     if (stats) {
-        if (positive) fn = win_smem ? k_propagate<false, true, true, true, S> : k_propagate<false, false, true, true, S>;
-        else fn = win_smem ? k_propagate<false, true, true, false, S> : k_propagate<false, false, true, false, S>;
+        if (positive) fn = win_smem ? k_propagate<true, true, true, S> : k_propagate<false, true, true, S>;
+        else fn = win_smem ? k_propagate<true, true, false, S> : k_propagate<false, true, false, S>;
     } else {
-        if (positive) fn = win_smem ? k_propagate<false, true, false, true, S> : k_propagate<false, false, false, true, S>;
-        else fn = win_smem ? k_propagate<false, true, false, false, S> : k_propagate<false, false, false, false, S>;
+        if (positive) fn = win_smem ? k_propagate<true, false, true, S> : k_propagate<false, false, true, S>;
+        else fn = win_smem ? k_propagate<true, false, false, S> : k_propagate<false, false, false, S>;
     }
     const cudaError_t e = raise_smem_limit((const void *)fn, smem);
     if (e != cudaSuccess) return e;

@@ -10,11 +10,11 @@ cudaError_t launch_prop_sample_gt(const KArgs &a, bool win_smem, bool stats, boo
     constexpr int G = kTablesGlobal;
     void (*fn)(const KArgs);
     if (stats) {
-        if (positive) fn = win_smem ? k_propagate<false, true, true, true, G> : k_propagate<false, false, true, true, G>;
-        else fn = win_smem ? k_propagate<false, true, true, false, G> : k_propagate<false, false, true, false, G>;
+        if (positive) fn = win_smem ? k_propagate<true, true, true, G> : k_propagate<false, true, true, G>;
+        else fn = win_smem ? k_propagate<true, true, false, G> : k_propagate<false, true, false, G>;
     } else {
-        if (positive) fn = win_smem ? k_propagate<false, true, false, true, G> : k_propagate<false, false, false, true, G>;
-        else fn = win_smem ? k_propagate<false, true, false, false, G> : k_propagate<false, false, false, false, G>;
+        if (positive) fn = win_smem ? k_propagate<true, false, true, G> : k_propagate<false, false, true, G>;
+        else fn = win_smem ? k_propagate<true, false, false, G> : k_propagate<false, false, false, G>;
     }
     const cudaError_t e = raise_smem_limit((const void *)fn, smem);
     if (e != cudaSuccess) return e;

@@ -7,8 +7,8 @@ namespace mcd {
 // For DAGs of non-negative finite times whose tables block sits in shared memory
 // (use_wide).
 cudaError_t launch_prop_wide(const KArgs &w, bool stats, dim3 grid, dim3 block, size_t smem, cudaStream_t st) {
-    void (*fn)(const KArgs) = stats ? k_propagate<false, true, true, true, kTablesSmem, 2>
-                                    : k_propagate<false, true, false, true, kTablesSmem, 2>;
+    void (*fn)(const KArgs) = stats ? k_propagate<true, true, true, kTablesSmem, 2>
+                                    : k_propagate<true, false, true, kTablesSmem, 2>;
     const cudaError_t e = raise_smem_limit((const void *)fn, smem);
     if (e != cudaSuccess) return e;
     fn<<<grid, block, smem, st>>>(w);
