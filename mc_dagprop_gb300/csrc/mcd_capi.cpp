@@ -69,6 +69,7 @@ KArgs base_args(const mcd_dag *g) {
     a.n_stages = g->h.n_stages;
     a.n_warps = g->h.n_warps;
     a.max_units = g->h.max_units;
+    a.avg_units = g->h.avg_units;
     a.n_aux = (int32_t)g->h.aux.size();
     a.window_slots = g->h.window_slots;
     a.n_dist = (int32_t)g->h.dist.size();

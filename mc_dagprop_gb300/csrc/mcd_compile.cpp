@@ -1131,13 +1131,14 @@ void compile_dag(const mcd_dag_desc &d, const mcd_generator &g, HostDag &H, int3
     }
     // what the work units save: Philox blocks a sample's propagation draws
     H.n_pairs = 0;
-    H.max_units = 0;
+    H.max_units = H.avg_units = 0;
     for (int32_t st = 0; st < H.n_stages; ++st) {
         const int32_t *m = &H.stage_meta[(size_t)st * kStageMetaInts];
         H.n_pairs += m[8];
         if (n_warps == 0 && !std::getenv("MCD_WARPS"))
             H.max_units = std::max(H.max_units, (m[1] >= 0 ? m[1] : -m[1]) - m[8]);
     }
+    if (H.max_units > 0) H.avg_units = std::max<int32_t>(1, (H.E - H.n_pairs) / H.n_stages);
     H.block_draws = 0;
     for (const PredRec &p : H.pred)
         if ((p.kd & KD_KIND_MASK) != K_FIXED && !(p.kd & KD_REUSE)) ++H.block_draws;

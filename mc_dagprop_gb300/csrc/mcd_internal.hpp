@@ -212,8 +212,8 @@ struct KArgs {
     int32_t n_groups;
     int32_t n_stages;
     int32_t n_warps;
-    int32_t max_units;        // most work units of a stage: the single-DAG launches choose their warps per
-                              // CTA by it and the tile count (pick_warps); 0: n_warps is the caller's choice
+    int32_t max_units;        // most and mean work units of a stage, by which the single-DAG launches choose
+    int32_t avg_units;        // their warps per CTA (pick_warps); 0: n_warps is the caller's choice
     int32_t n_aux;
     int32_t window_slots;
     int32_t n_dist, n_alias;

@@ -176,48 +176,59 @@ static int sm_count() {
     return sms;
 }
 
-// An SM's warps (sm_warps) dealt out over the CTAs of `smem` bytes it holds of a
-// launch of `tiles`: warps per CTA, 0 on error.
-static int deal_warps(int sm_warps, int64_t tiles, int smem) {
-    const int sms = sm_count();
-    if (!sms) return 0;
-    constexpr int kSmBytes = 227 * 1024;
-    const int64_t per_sm = (tiles + sms - 1) / sms;
-    const int64_t fit = kSmBytes / (smem + 1024);  // a CTA takes 1 KB of shared memory beside its own
-    const int64_t ctas = per_sm < fit ? per_sm : fit;
-    return (int)(sm_warps / (ctas < 1 ? 1 : ctas > sm_warps ? sm_warps : ctas));
+// CTAs of `smem` bytes that fit an SM's shared memory.
+static int64_t ctas_fit(int64_t smem) {
+    constexpr int64_t kSmBytes = 228 * 1024;
+    return kSmBytes / (smem + 1024);  // a CTA takes 1 KB beside its own
 }
 
 // Warps take a stage's units from a counter, so a CTA may have any number of them.
-// The compiler's choice (a sixth of the level width) suits a device full of
-// CTAs: an SM then holds 24 warps in several CTAs.  A launch with fewer tiles
-// than that leaves warp slots empty while each level waits for a few warps to
-// run its units one after another, so the SM's 24 warps are dealt out over the
-// CTAs it will hold: tiles per SM, or as many as fit its shared memory.  More
-// warps than a stage has units would only wait at the barriers, and a raise by
-// less than a quarter is left (23 -> 24 warps on the 200,000-event DAG: 1 % slower).
-// Measured against the compiler's choice: one sample of 1,000 events 250 -> 172 us
-// (4 -> 14 warps), 20,017 events x 3,001 samples 2.95 -> 1.75 ms (7 -> 24), the
-// statistics of 10,000 events x 65,536 samples 11.1 -> 10.2 ms (19 -> 24).
+// An SM's warps (sm_warps) are dealt out over the c CTAs it holds at a time, nw each,
+// a multiple of four (warps go to the four sub-partitions in turn; six or ten leave
+// two of them short).  c CTAs then take sm_warps / nw for their work and a tail at
+// each stage's barrier, half a unit's time or so: 0.55 sm_warps / U with U units a
+// stage (fitted to 30-130 events a level, 4 to 24 warps).  Several small CTAs hide
+// each other's barriers where many tiles queue for an SM; a launch of a tile or two an
+// SM wants every warp on them.
+// Measured against the compiler's choice, a sixth of the level width: one sample of
+// 1,000 events 250 -> 172 us (4 -> 16 warps), 20,017 events x 3,001 samples 2.95 ->
+// 1.75 ms (7 -> 24), 45 events a level x 30,000 samples, the statistics, 1.79 -> 1.58
+// (9 -> 8, three CTAs an SM where two fitted).
 int pick_warps(const KArgs &a, int64_t tiles, int sm_warps, int cta_warps) {
-    if (a.max_units <= 0) return a.n_warps;
-    const int nw = deal_warps(sm_warps, tiles, a.smem_total);
-    if (nw <= 0) return a.n_warps;
-    const int cap = a.max_units < cta_warps ? a.max_units : cta_warps;
-    const int most = nw < cap ? nw : cap;
-    return 4 * most > 5 * a.n_warps ? most : a.n_warps;
+    const int sms = sm_count();
+    if (a.max_units <= 0 || !sms) return a.n_warps;
+    const int64_t per_sm = (tiles + sms - 1) / sms;
+    const int64_t fit = ctas_fit(a.smem_total);
+    const int most = (a.max_units + 3) / 4 * 4 < cta_warps ? (a.max_units + 3) / 4 * 4 : cta_warps;
+    const double tail = 0.55 * sm_warps / (a.avg_units > 0 ? a.avg_units : 1);
+    int best = 4;
+    double best_cost = 0.0;
+    for (int c = 1; c <= 8 && (c == 1 || (c <= fit && c <= per_sm)); ++c) {
+        int nw = sm_warps / c / 4 * 4;
+        nw = nw > most ? most : nw;
+        if (nw < 4) break;
+        const double cost = (double)((per_sm + c - 1) / c) * ((double)sm_warps / nw + tail);
+        if (c == 1 || cost < best_cost) {
+            best = nw;
+            best_cost = cost;
+        }
+    }
+    return best;
 }
 
 // A wide tile reads each record, decodes its kind and forms its addresses once for
 // 64 samples instead of 32 (121 -> 105 warp instructions per 32 sample-edges) and
-// its two samples' chains fill each other's latencies, so it takes 1.77 times a narrow
-// tile's time for twice the samples.  It pays where the SM with the most tiles has
-// fewer of them in that measure: not below one narrow tile an SM, where the chain of
-// levels is all there is, and not at three narrow tiles against two wide ones.
+// its two samples' chains fill each other's latencies, so a CTA of 24 warps takes
+// 1.77 times as long for twice the samples.  It pays where a narrow CTA has its SM to
+// itself anyway: with two or three narrow CTAs an SM these hide each other's barriers
+// better than one wide one does (45 and 60 events a level: 1.06-1.2 times the time).
+// And it pays where the SM with the most tiles has fewer of them in that measure: not
+// below one narrow tile an SM, where the chain of levels is all there is, and not at
+// three narrow tiles against two wide ones.
 // Measured (narrow, wide): 200,000 events x 9,728 samples, outputs 24.0, 21.4 ms;
-// statistics of 10,000 events x 65,536 samples 10.2, 8.6 ms; its gradient 19.8, 18.1.
+// statistics of 10,000 events x 65,536 samples 10.2, 8.6 ms.
 bool use_wide(const KArgs &a) {
-    if (a.wide_rows <= 0 || !a.positive || !a.tables_in_smem) return false;
+    if (a.wide_rows <= 0 || !a.positive || !a.tables_in_smem || ctas_fit(a.smem_total) > 1) return false;
     if (a.window_spill > 0 && !a.spill && !a.realized) return false;  // no place for the off-chip rows
     const int sms = sm_count();
     if (!sms) return false;

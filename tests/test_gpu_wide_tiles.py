@@ -34,8 +34,9 @@ def _device_run(prop, seeds):
     return real.cpu().numpy(), dur.cpu().numpy(), cause.cpu().numpy()
 
 
-# (DAG, fits): width 60 over 3 layers keeps a wide window on chip, width 130 does not
-@pytest.mark.parametrize("width,preds", [(60, 4), (130, 4), (130, 12)])
+# width 80 over 3 layers keeps a wide window on chip, width 130 does not (width 60: two
+# narrow CTAs an SM, which stay narrow)
+@pytest.mark.parametrize("width,preds", [(60, 4), (80, 4), (130, 4), (130, 12)])
 @pytest.mark.parametrize("n", [2 * WAVE - 64, 2 * WAVE - 31, 2 * WAVE - 33, 2 * WAVE + 2 * WAVE - 127])
 def test_wide_tiles_give_the_bits_of_narrow_ones(cuda, width, preds, n):
     flat, gen = kitchen_sink(seed=21, n_layers=7, width=width, max_preds=preds)
@@ -58,12 +59,14 @@ def test_wide_tiles_give_the_bits_of_narrow_ones(cuda, width, preds, n):
 
 
 def test_large_windows_keep_rows_off_chip(cuda):
-    """The cases above cover both plans: 130-wide levels need more rows than fit."""
-    small, gen = kitchen_sink(seed=21, n_layers=7, width=60)
+    """The cases above cover both plans: 130-wide levels need more rows than fit, 80-wide
+    ones fit and leave no room for a second narrow CTA."""
+    small, gen = kitchen_sink(seed=21, n_layers=7, width=80)
     large, _ = kitchen_sink(seed=21, n_layers=7, width=130)
     row = 64 * 8
     info = [batching.compile_dag(f, gen).info() for f in (small, large)]
     rest = [i["smem_bytes"] - i["window_slots"] * 256 for i in info]
+    assert 2 * (info[0]["smem_bytes"] + 1024) > 228 * 1024
     assert info[0]["window_in_smem"] and info[0]["window_slots"] * row + rest[0] <= 226 * 1024
     assert info[1]["window_in_smem"] and info[1]["window_slots"] * row + rest[1] > 226 * 1024
 
@@ -74,7 +77,7 @@ def test_batches_run_wide_tiles_with_the_same_statistics(cuda):
 
     ns = [1, 32, 33, 64, 95, 3000]
     props = [batching.compile_dag(*kitchen_sink(seed=30 + i, n_layers=5, width=w), 8)
-             for i, w in enumerate([60, 130, 130, 60, 130, 130])]
+             for i, w in enumerate([60, 130, 130, 80, 130, 130])]
     batch = _core.Batch(props, list(range(len(ns))), ns)
     for _ in range(2):
         batch.run()
