@@ -20,6 +20,8 @@
 
 namespace mcd {
 cudaError_t launch_propagate(const KArgs &a, bool given, bool win_smem, bool stats, cudaStream_t st);
+bool few_layout(const KArgs &a, int64_t n, bool direct, FewArgs &f);
+cudaError_t launch_few(const KArgs &a, const FewArgs &f, cudaStream_t st);
 cudaError_t launch_stats_finish(const FArgs &f, cudaStream_t st);
 cudaError_t launch_event_ticks(const double *earliest, int32_t E, int32_t q, long long *te, cudaStream_t st);
 cudaError_t launch_wait_selftest(int32_t *err, uint32_t limit, cudaStream_t st);
@@ -70,6 +72,10 @@ KArgs base_args(const mcd_dag *g) {
     a.n_warps = g->h.n_warps;
     a.max_units = g->h.max_units;
     a.avg_units = g->h.avg_units;
+    a.stage_events = g->h.stage_events;
+    a.stage_entries = g->h.stage_entries;
+    a.n_events = g->h.E;
+    a.n_entries = (int32_t)g->h.pred.size();
     a.n_aux = (int32_t)g->h.aux.size();
     a.window_slots = g->h.window_slots;
     a.n_dist = (int32_t)g->h.dist.size();
@@ -452,6 +458,138 @@ void move_rows(const T *minor, int64_t C, T *dv, T *host, T *major, int64_t rows
     }
 }
 
+// Few samples through host buffers (mcd_few.cu); false where that path does not apply.
+// seeds, or dur_in: what the samples are.  Few rows (kFewInline, kFewDirect) are written
+// sample-major, straight into pinned memory (or to the device and copied), which saves
+// the seeds' copy and the transposes; others are transposed (move_rows): their scattered
+// 8-byte writes cost more over the host link (1,000 events x 1 68 against 80 us, x 20 80
+// and 85, x 32 93 and 89; 10,000 x 4 138 and 143, x 8 159 and 151).
+bool run_few(mcd_dag *g, const int64_t *seeds, const double *dur_in, int64_t n, double *realized, double *durations,
+             int32_t *cause) {
+    const int64_t E = g->h.E, L = g->h.L;
+    KArgs a = base_args(g);
+    FewArgs f{};
+    a.dur_in = dur_in;  // (which rule applies)
+    const bool direct = n <= kFewInline && n * E <= kFewDirect;
+    if (!few_layout(a, n, direct, f)) return false;
+    double *real_dv = device_view(realized), *dur_dv = device_view(durations);
+    const double *in_dv = device_view(dur_in);
+    int32_t *cause_dv = device_view(cause);
+    const bool staged = (realized && !real_dv) || (durations && !dur_dv) || (cause && !cause_dv) || (dur_in && !in_dv);
+    const size_t s_re = align_up((size_t)(n * E) * 8, 256), s_du = align_up((size_t)(n * L) * 8, 256),
+                 s_ca = align_up((size_t)(n * E) * 4, 256), s_seeds = align_up((size_t)n * 8, 256);
+    // (the workspace's bounds are those of the general path, which needs less: host_chunk)
+    const size_t rows = s_re + s_du + s_ca;
+    const size_t bytes = s_seeds + f.scratch + (staged ? rows : 0) + (direct ? 0 : rows);
+    if (bytes > ((size_t)1 << 30)) {
+        size_t free_b = 0, total_b = 0;
+        cuda_check(cudaMemGetInfo(&free_b, &total_b), "device memory query");
+        if (bytes > std::min((free_b + g->ws_bytes) / 4, (size_t)32 << 30)) return false;
+    }
+    ensure_ws(g, bytes);
+    char *p = g->ws;
+    auto take = [&](size_t bytes) {
+        char *q = p;
+        p += bytes;
+        return q;
+    };
+    int64_t *d_seeds = (int64_t *)take(s_seeds);
+    f.entry_dur = (double *)take(f.scratch);
+    double *re_major = nullptr, *du_major = nullptr, *re = nullptr, *du = nullptr;
+    int32_t *ca_major = nullptr, *ca = nullptr;
+    if (staged) {
+        re_major = (double *)take(s_re);
+        du_major = (double *)take(s_du);
+        ca_major = (int32_t *)take(s_ca);
+    }
+    if (!direct) {
+        re = (double *)take(s_re);
+        du = (double *)take(s_du);
+        ca = (int32_t *)take(s_ca);
+    }
+    f.realized = !realized ? nullptr : !direct ? re : real_dv ? real_dv : re_major;
+    f.durations = !durations ? nullptr : !direct ? du : dur_dv ? dur_dv : du_major;
+    f.cause = !cause ? nullptr : !direct ? ca : cause_dv ? cause_dv : ca_major;
+    f.out_row = direct ? 1 : n;
+    f.out_col = direct ? E : 1;
+    f.dur_row = direct || dur_in ? 1 : n;
+    f.dur_col = direct || dur_in ? L : 1;
+    cudaStream_t st = g->stream[0];
+    if (dur_in) {
+        f.dur_in = in_dv ? in_dv : du_major;
+        if (!in_dv && L > 0)
+            cuda_check(cudaMemcpyAsync(du_major, dur_in, (size_t)(n * L) * 8, cudaMemcpyHostToDevice, st), "durations upload");
+    } else if (n <= kFewInline) {
+        std::copy(seeds, seeds + n, f.seed);
+    } else {
+        cuda_check(cudaMemcpyAsync(d_seeds, seeds, (size_t)n * 8, cudaMemcpyHostToDevice, st), "seed upload");
+        f.seeds = d_seeds;
+    }
+    cuda_check(launch_few(a, f, st), "propagate launch");
+    if (direct) {
+        auto down = [&](void *host, const void *dv, const void *dev, size_t bytes, const char *what) {
+            if (host && !dv && bytes) cuda_check(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st), what);
+        };
+        down(realized, real_dv, re_major, (size_t)(n * E) * 8, "realized download");
+        down(durations, dur_dv, du_major, (size_t)(n * L) * 8, "durations download");
+        down(cause, cause_dv, ca_major, (size_t)(n * E) * 4, "cause download");
+    } else {
+        move_rows(re, n, real_dv, realized, re_major, E, 0, n, st, "realized download");
+        move_rows(du, n, dur_dv, durations, du_major, L, 0, n, st, "durations download");
+        move_rows(ca, n, cause_dv, cause, ca_major, E, 0, n, st, "cause download");
+    }
+    check_device_error(g);
+    return true;
+}
+
+// The same with device buffers (a: the launch's arguments, sample-minor rows).  The
+// scratch comes from the handle's pool in the stream's order, so that calls on several
+// streams and threads share nothing; a stream that is being captured, and one whose
+// scratch cannot be had, keeps the general launch.
+bool run_few_device(mcd_dag *g, const KArgs &a, cudaStream_t st) {
+    FewArgs f{};
+    if (!few_layout(a, a.n, false, f)) return false;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    {
+        std::lock_guard<std::mutex> lk(g->few_mu);
+        if (!g->few_pool) {
+            cudaMemPoolProps props{};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = g->device;
+            uint64_t keep = kFewScratch;
+            if (cudaMemPoolCreate(&g->few_pool, &props) != cudaSuccess) {
+                (void)cudaGetLastError();
+                g->few_pool = nullptr;
+                return false;
+            }
+            cuda_check(cudaMemPoolSetAttribute(g->few_pool, cudaMemPoolAttrReleaseThreshold, &keep), "scratch pool");
+        }
+    }
+    void *p = nullptr;
+    if (cudaMallocFromPoolAsync(&p, f.scratch, g->few_pool, st) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    f.entry_dur = (double *)p;
+    f.seeds = a.seeds;
+    f.realized = a.realized;
+    f.cause = a.cause;
+    f.durations = a.durations;
+    f.dur_in = a.dur_in;
+    f.out_row = a.ld;
+    f.dur_row = a.dur_in ? a.ld_in : a.ld;
+    f.out_col = f.dur_col = 1;
+    const cudaError_t e = launch_few(a, f, st);
+    cudaFreeAsync(p, st);
+    cuda_check(e, "propagate launch");
+    return true;
+}
+
 }  // namespace
 
 extern "C" {
@@ -582,6 +720,7 @@ void mcd_dag_destroy(mcd_dag *g) {
             cudaStreamDestroy(g->stream[k]);
         }
     if (g->ws) cudaFree(g->ws);
+    if (g->few_pool) cudaMemPoolDestroy(g->few_pool);  // (what is in use goes with its last cudaFreeAsync)
     if (g->d_err) cudaFree(g->d_err);
     cudaSetDevice(prev);
     delete g;  // the image goes with its last handle
@@ -687,6 +826,7 @@ int mcd_run_device(mcd_dag *g, const int64_t *seeds, int64_t n, double *realized
             ensure_ws(g, (size_t)g->h.E * (size_t)ld * 8);
             a.scratch = (double *)g->ws;
         }
+        if (run_few_device(g, a, st)) return;
         cuda_check(launch_propagate(a, false, g->h.win_smem, false, st), "propagate launch");
     });
 }
@@ -711,6 +851,7 @@ int mcd_propagate_device(mcd_dag *g, const double *dur, int64_t ld_in, int64_t n
             ensure_ws(g, (size_t)g->h.E * (size_t)ld * 8);
             a.scratch = (double *)g->ws;
         }
+        if (run_few_device(g, a, st)) return;
         cuda_check(launch_propagate(a, true, g->h.win_smem, false, st), "propagate launch");
     });
 }
@@ -723,6 +864,7 @@ int mcd_run_many_host(mcd_dag *g, const int64_t *seeds, int64_t n, double *reali
         if (n == 0) return;
         if (!seeds) throw McdError(MCD_ERR_INVALID, "null seeds");
         cuda_check(cudaSetDevice(g->device), "cudaSetDevice");
+        if (run_few(g, seeds, nullptr, n, realized, durations, cause)) return;
         const int64_t E = g->h.E, L = g->h.L;
         double *real_dv = device_view(realized), *dur_dv = device_view(durations);
         int32_t *cause_dv = device_view(cause);
@@ -764,6 +906,7 @@ int mcd_propagate_host(mcd_dag *g, const double *durations, int64_t n, double *r
         if (n == 0) return;
         if (!durations && g->h.L > 0) throw McdError(MCD_ERR_INVALID, "null durations");
         cuda_check(cudaSetDevice(g->device), "cudaSetDevice");
+        if (run_few(g, nullptr, durations, n, realized, nullptr, cause)) return;
         const int64_t E = g->h.E, L = g->h.L;
         const double *dur_dv = device_view(durations);
         double *real_dv = device_view(realized);

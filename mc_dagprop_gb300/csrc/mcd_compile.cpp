@@ -140,6 +140,7 @@ void verify_layout(const HostDag &H) {
         const int64_t first = m[0], nev = m[1] >= 0 ? m[1] : -(int64_t)m[1], pfirst = m[2], npred = m[3];
         const int64_t vfirst = m[4], nval = m[5];
         if (first != ev_next || nev <= 0 || first + nev > E || pfirst != pred_next) fail("stage ranges");
+        if (nev > H.stage_events || npred > H.stage_entries) fail("stage sizes");
         if (m[8] < 0 || 2 * (int64_t)m[8] > nev || m[9] || m[10] || m[11]) fail("event pairs");
         if (vfirst != val_next || nval < 0 || nval % 2 || vfirst + nval > (int64_t)H.vals.size())
             fail("value region");
@@ -1132,9 +1133,12 @@ void compile_dag(const mcd_dag_desc &d, const mcd_generator &g, HostDag &H, int3
     // what the work units save: Philox blocks a sample's propagation draws
     H.n_pairs = 0;
     H.max_units = H.avg_units = 0;
+    H.stage_events = H.stage_entries = 0;
     for (int32_t st = 0; st < H.n_stages; ++st) {
         const int32_t *m = &H.stage_meta[(size_t)st * kStageMetaInts];
         H.n_pairs += m[8];
+        H.stage_events = std::max(H.stage_events, m[1] >= 0 ? m[1] : -m[1]);
+        H.stage_entries = std::max(H.stage_entries, m[3]);
         if (n_warps == 0 && !std::getenv("MCD_WARPS"))
             H.max_units = std::max(H.max_units, (m[1] >= 0 ? m[1] : -m[1]) - m[8]);
     }

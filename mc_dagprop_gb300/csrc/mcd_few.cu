@@ -1,0 +1,290 @@
+// mcd_few.cu -- few samples: lanes over predecessors or events, a CTA a sample.
+//
+// A tile of 32 samples an SM leaves most of the chip idle when few samples are run, and
+// its levels are then a chain: an event's entries one after another, each a Philox block
+// and a sampler, some 5,000 clocks a stage.  Here the draws come first, on all SMs
+// (k_few_draw), into a scratch in the order in which the propagation reads them; then a
+// CTA of one to sixteen samples walks the stages (k_few).  What is left of a stage is a
+// barrier, one add and a maximum, and nothing else may lie on that path: records and
+// durations come through a ring of stage buffers that a warp of its own fills by bulk
+// copies several stages ahead.  It is bound by that chain, about 1,800 clocks a stage of
+// 100 events, and by the draws' instructions as the samples grow.
+// Measured, before and after: 1,000 events, one seed through host buffers 168 -> 68 us;
+// 200,000 events, one seed 13.1 -> 1.9 ms; on the device, 10,000 events x 152 samples
+// 642 -> 129 us, 20,017 x 608 1,757 -> 692, 200,000 x 608 12.8 -> 4.5 ms.
+#include "mcd_device.cuh"
+
+namespace mcd {
+
+constexpr int kFewDrawThreads = 128;
+
+// First element of a stage's durations in KArgs-wide numbering, samples aside: even, so
+// that a copy starts on a 16-byte boundary (stages' ranges stay apart: each stage moves
+// the numbering on by one).
+__device__ __forceinline__ int64_t few_first(int stage, int first_entry) {
+    return (int64_t)((uint32_t)(first_entry + stage + 1) & ~1u);
+}
+
+// Durations of the stage blockIdx.x.  A warp's lanes are the samples of a block of up to
+// 32 and, when n is smaller, several entries; a lane takes kFewDrawRun entries one after
+// another where n fills the lanes (one otherwise: latency), drawing a Philox block once
+// for the entries that share it.  The last CTAs draw the links no entry references.  The
+// draws are the sampled propagation's own (same records, blocks, words and arithmetic):
+// equal bits.
+constexpr int kFewDrawRun = 4;
+template <bool GIVEN>
+__global__ void __launch_bounds__(kFewDrawThreads) k_few_draw(const KArgs a, const FewArgs f) {
+    const int stage = blockIdx.x, n = f.n, ns = 1 << f.ns_log, lane = threadIdx.x & 31;
+    const DistParam *dists = a.dist;
+    const AliasEntry *alias = reinterpret_cast<const AliasEntry *>(dists + a.n_dist);
+    const AliasPick *picks = reinterpret_cast<const AliasPick *>(alias + a.n_alias);
+    const int lanes_log = n > 16 ? 5 : n > 8 ? 4 : n > 4 ? 3 : n > 2 ? 2 : n > 1 ? 1 : 0;  // of a lane's samples
+    const int run = n >= 32 ? kFewDrawRun : 1;
+    const int blocks = (n + 31) >> 5, per_warp = run << (5 - lanes_log);  // sample blocks; entries a warp takes
+    U4 words{};
+    uint32_t drawn = 0xFFFFFFFFu;  // the block `words` are of (no block has this number)
+    uint64_t seed = 0;
+    auto draw = [&](int kd, double v, const double *vt, uint32_t block, uint32_t link) {
+        const int kind = kd & KD_KIND_MASK;
+        if (kind == K_FIXED) return v;
+        const DistParam &p = dists[kd >> 8];
+        float dfac;
+        if (kind == K_GAMMA && !p.erlang) return draw_gamma(p, v, block, seed, a.err, &dfac);
+        if (block != drawn) words = draw_words(seed, block, 0u, 0u);
+        drawn = block;
+        const int w = (kd >> KD_WORD_SHIFT) & 3;
+        if (kind == K_GAMMA) return draw_erlang(p, v, link, seed, words, w, a.err, &dfac);
+        if (kind == K_EXP) return draw_exponential(p, v, word_of(words, w), dfac);
+        return draw_empirical(p, alias, picks, vt, v, kind == K_EMP_REL, word_of(words, w), words.y,
+                              (kd & KD_TWO_WORD) != 0, dfac);
+    };
+    const bool aux = stage >= a.n_stages;
+    const int4 meta = aux ? make_int4(0, 0, 0, a.n_aux) : __ldg(reinterpret_cast<const int4 *>(a.stage_meta + kStageMetaInts * stage));
+    const int4 mv = aux ? meta : __ldg(reinterpret_cast<const int4 *>(a.stage_meta + kStageMetaInts * stage) + 1);
+    double *out = aux ? nullptr : f.entry_dur + (few_first(stage, meta.z) << f.ns_log);
+    const int cta = blockIdx.y + (aux ? (stage - a.n_stages) * gridDim.y : 0);
+    const int ctas = aux ? (gridDim.x - a.n_stages) * gridDim.y : gridDim.y;
+    const int items = (meta.w + per_warp - 1) / per_warp * blocks;
+    for (int item = cta * (kFewDrawThreads / 32) + (threadIdx.x >> 5); item < items; item += ctas * (kFewDrawThreads / 32)) {
+        const int g = item / blocks;
+        const int s = ((item - g * blocks) << 5) + (lane & ((1 << lanes_log) - 1));
+        if (s >= n) continue;
+        seed = f.seeds ? (uint64_t)__ldg(f.seeds + s) : (uint64_t)f.seed[s & (kFewInline - 1)];
+        drawn = 0xFFFFFFFFu;
+        const int first = g * per_warp + (lane >> lanes_log) * run;
+        for (int i = first; i < first + run && i < meta.w; ++i) {
+            if (aux) {
+                const LinkRec lr = a.aux[i];  // (owns its block)
+                f.durations[(int64_t)lr.link * f.dur_row + s * f.dur_col] =
+                    draw(lr.kd, lr.v, nullptr, (uint32_t)lr.link, (uint32_t)lr.link);
+                continue;
+            }
+            const int4 *q = reinterpret_cast<const int4 *>(a.pred + meta.z + i);
+            const int4 r0 = __ldg(q);  // src_slot, src_user, link, kd
+            double dur = 0.0;
+            if (GIVEN) {
+                if (r0.z >= 0) dur = __ldg(f.dur_in + (int64_t)r0.z * f.dur_row + s * f.dur_col);
+            } else {
+                const int4 r1 = __ldg(q + 1);  // v, dvo, block
+                const double *vt = nullptr;
+                if (r1.z >= 0 && (r0.w & KD_KIND_MASK) != K_FIXED)
+                    vt = meta.y >= 0 ? a.vals + mv.x + (r1.z - mv.w) / (int)sizeof(double) : a.vals + (r1.z ^ kVtGlobal);
+                dur = draw(r0.w, __hiloint2double(r1.y, r1.x), vt, (uint32_t)r1.w, (uint32_t)r0.z);
+                if (f.durations && (r0.w & KD_WRITE)) f.durations[(int64_t)r0.z * f.dur_row + s * f.dur_col] = dur;
+            }
+            // (CTA s / ns of the propagation reads its samples alone)
+            out[(int64_t)(s >> f.ns_log) * f.cta_entries + ((int64_t)i << f.ns_log) + (s & (ns - 1))] = dur;
+        }
+    }
+}
+
+// One CTA for 2^ns_log samples, its last warp the producer: unit u of a stage is lane
+// u % G of sample (u / G) % 2^ns_log of event u / G / 2^ns_log.  An entry's place in its
+// list decides ties as in the sequential loop (_core.cpp:338-347: a later equal time
+// takes over), so the maximum over (key, place), taken where its key reaches the event's
+// own, is the loop's result.
+template <bool POSITIVE, int G>
+__global__ void __launch_bounds__(1024, 1) k_few(const KArgs a, const FewArgs f) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ uint64_t bars[kFewRing];
+    __shared__ int2 head[kFewRing];  // of the stage in a buffer: events, first entry
+    double *win = reinterpret_cast<double *>(smem);
+    unsigned char *ring = smem + f.ring_off;
+    const int lane = threadIdx.x & 31, R = f.ring, NS = a.n_stages, ns = 1 << f.ns_log;
+    const int workers = blockDim.x - 32;
+    const bool producer = (int)threadIdx.x == workers;
+    const double *entry_dur = f.entry_dur + (int64_t)blockIdx.x * f.cta_entries;
+    const int4 *meta = reinterpret_cast<const int4 *>(a.stage_meta);
+    constexpr int kVecs = kStageMetaInts / 4;
+    int4 m_next[2] = {};  // the producer's next two stages: first event, events, first entry, entries
+    auto fill = [&](int l, int4 m) {
+        const int b = l % R;
+        const int n_ev = m.y >= 0 ? m.y : -m.y;
+        head[b] = make_int2(n_ev, m.z);
+        const uint32_t ev_bytes = (uint32_t)n_ev * (uint32_t)sizeof(EvRec);
+        const uint32_t pr_bytes = (uint32_t)m.w * (uint32_t)sizeof(PredRec);
+        const uint32_t du_bytes = (((uint32_t)(m.w + 1) & ~1u) << f.ns_log) * (uint32_t)sizeof(double);
+        unsigned char *buf = ring + b * f.buf_bytes;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        mbar_expect_tx(&bars[b], ev_bytes + pr_bytes + du_bytes);
+        bulk_g2s(buf, a.ev + m.x, ev_bytes, &bars[b]);
+        if (m.w) bulk_g2s(buf + f.pred_off, a.pred + m.z, pr_bytes, &bars[b]);
+        if (m.w) bulk_g2s(buf + f.dur_off, entry_dur + (few_first(l, m.z) << f.ns_log), du_bytes, &bars[b]);
+    };
+    bool ok = true;
+    int issued = 0, waits = 0;  // the producer's: stages copied, and the one last waited for
+    if (producer) {
+        for (int k = 0; k < R; ++k) mbar_init(&bars[k], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        for (; issued < R && issued < NS; ++issued) fill(issued, __ldg(meta + kVecs * issued));
+        for (int k = 0; k < 2; ++k)
+            if (R + k < NS) m_next[k] = __ldg(meta + kVecs * (R + k));
+        if (NS > 0) ok = stage_wait(&bars[0], 0u, a.err);
+    }
+    if (!__syncthreads_or(!ok)) {
+        int b = 0;
+        uint32_t phase = 0;
+        for (int l = 0; l < NS; ++l) {
+            if ((int)threadIdx.x < workers) {
+                const int2 h = head[b];
+                const unsigned char *buf = ring + b * f.buf_bytes;
+                const EvRec *sev = reinterpret_cast<const EvRec *>(buf);
+                const PredRec *pred = reinterpret_cast<const PredRec *>(buf + f.pred_off);
+                const double *durs = reinterpret_cast<const double *>(buf + f.dur_off);
+                const unsigned group = G == 32 ? 0xFFFFFFFFu : ((1u << G) - 1u) << (lane & ~(G - 1));
+                for (int u = threadIdx.x; u < (h.x * G) << f.ns_log; u += workers) {
+                    const int j = (u / G) & (ns - 1);
+                    const EvRec ev = load_ev(sev + ((u / G) >> f.ns_log));
+                    const long long init_key = POSITIVE ? ev.init_bits : ev.init_key;
+                    const long long ub_key = POSITIVE ? ev.ub_bits : ev.ub_key;
+                    const int pb = ev.pred_begin - h.y, pe = ev.pred_end - h.y;
+                    long long key = (long long)0x8000000000000000ull, bits = 0;  // (below any event's own key)
+                    int place = -1, cause = -1;
+                    for (int p = pb + (u & (G - 1)); p < pe; p += G) {
+                        const int2 src = *reinterpret_cast<const int2 *>(pred + p);  // src_slot, src_user
+                        bool clamp;
+                        if (relax<POSITIVE>(win[(window_row<1>(src.x) << f.ns_log) + j], durs[(p << f.ns_log) + j], ub_key,
+                                            ev.ub_bits, key, bits, clamp)) {
+                            place = p;
+                            cause = src.y;
+                        }
+                    }
+                    long long best = key;
+                    int at = place;
+#pragma unroll
+                    for (int m = 1; m < G; m *= 2) {
+                        const long long k = __shfl_xor_sync(group, best, m);
+                        const int q = __shfl_xor_sync(group, at, m);
+                        if (k > best || (k == best && q > at)) {
+                            best = k;
+                            at = q;
+                        }
+                    }
+                    const bool taken = at >= 0 && best >= init_key;
+                    if (G == 1 || (taken ? place == at : (u & (G - 1)) == 0)) {
+                        if (!taken) {
+                            cause = -1;
+                            bits = ub_key < init_key ? ev.ub_bits : ev.init_bits;  // realized = std::min(latest, ub)
+                        }
+                        const double v = __longlong_as_double(bits);
+                        const int slot = window_row<1>(ev.slot);
+                        if (slot >= 0) win[(slot << f.ns_log) + j] = v;
+                        const int s = (blockIdx.x << f.ns_log) + j;
+                        if (s < f.n) {
+                            if (f.realized) f.realized[(int64_t)ev.user * f.out_row + s * f.out_col] = v;
+                            if (f.cause) f.cause[(int64_t)ev.user * f.out_row + s * f.out_col] = cause;
+                        }
+                    }
+                }
+            }
+            const int nb = b + 1 == R ? 0 : b + 1;
+            const uint32_t nphase = phase ^ (nb == 0 ? 1u : 0u);
+            if (producer && l + 1 < NS) {
+                waits = l + 1;
+                ok = stage_wait(&bars[nb], nphase, a.err);
+            }
+            if (__syncthreads_or(!ok)) break;
+            if (producer && l + R < NS) {
+                fill(l + R, m_next[0]);
+                issued = l + R + 1;
+                m_next[0] = m_next[1];
+                if (l + R + 2 < NS) m_next[1] = __ldg(meta + kVecs * (l + R + 2));
+            }
+            b = nb;
+            phase = nphase;
+        }
+    }
+    if (producer && !ok)  // a copy that never landed: drain the others in flight, then leave
+        for (int l = waits + 1; l < issued; ++l) stage_wait(&bars[l % R], (uint32_t)((l / R) & 1), a.err);
+}
+
+int sm_count();
+
+// The layout of a launch of n samples; false where this path does not apply: windows off
+// chip, warps per CTA that the caller fixed, stages that leave no ring, more scratch than
+// kFewScratch, and sizes where it measured no faster.  With `work` the stages plus a 64th
+// of the events: samples drawn, general and few,
+//   100 events in 2 stages (work 4)   8.3 and 12.7 us: the second launch is not repaid
+//   203 in 11 (14)    x 152 24.7, 21.2   x 608 24.7, 22.7   x 2,432 24.7, 27.8
+//   600 in 20 (29)    x 152 59, 29       x 608 59, 37       x 2,432 59, 58
+//   20,017 in 545 (860) x 1,216 1,758, 934   x 2,432 1,760, 1,470   x 3,001 1,758, 1,857
+// and durations given, whose general kernel has less to do a stage,
+//   203  x 152 20.6, 19.9   x 608 20.6, 23.1;  600  x 608 45, 38   x 1,216 45, 43
+//   20,017  x 1,216 1,427, 998   x 2,432 1,432, 1,475
+// direct: the rows go straight to the host, which saves more launches than this adds.
+bool few_layout(const KArgs &a, int64_t n, bool direct, FewArgs &f) {
+    const int sms = sm_count();
+    if (n < 1 || !a.win_smem || a.avg_units <= 0 || a.n_stages <= 0 || sms <= 0) return false;
+    const int64_t work = a.n_stages + a.n_events / 64;
+    if (!direct && work < (a.dur_in ? 24 : 8)) return false;
+    const int most = work < 32 ? 2 : a.dur_in ? 3 : 4;
+    f.ns_log = 0;
+    while (f.ns_log <= most && ((int64_t)sms << f.ns_log) < n) ++f.ns_log;
+    if (f.ns_log > most) return false;
+    f.n = (int32_t)n;
+    f.ctas = (int32_t)((n + (1 << f.ns_log) - 1) >> f.ns_log);
+    f.cta_entries = ((int64_t)a.n_entries + a.n_stages + 2) / 2 * 2 << f.ns_log;
+    f.scratch = (size_t)f.ctas * (size_t)f.cta_entries * sizeof(double);
+    if (f.scratch > kFewScratch) return false;
+    const size_t win = (((size_t)a.window_slots << f.ns_log) * sizeof(double) + 127) / 128 * 128;
+    const size_t ev = (size_t)a.stage_events * sizeof(EvRec), pred = (size_t)a.stage_entries * sizeof(PredRec);
+    const size_t dur = ((size_t)(a.stage_entries + 1) / 2 * 2 << f.ns_log) * sizeof(double);
+    const size_t buf = (ev + pred + dur + 127) / 128 * 128;
+    if (win + 2 * buf > kFewSmem) return false;
+    f.ring_off = (int32_t)win;
+    f.pred_off = (int32_t)ev;
+    f.dur_off = (int32_t)(ev + pred);
+    f.buf_bytes = (int32_t)buf;
+    f.ring = (int32_t)((kFewSmem - win) / buf < (size_t)kFewRing ? (kFewSmem - win) / buf : kFewRing);
+    f.smem = (int32_t)(win + f.ring * buf);
+    const int64_t units = (int64_t)a.stage_events << f.ns_log;
+    // Lanes over an event's entries shorten its chain while the stage's warps are few; past
+    // some 8 warps their reductions cost more issue than they save (20,017 events in stages
+    // of 37: one sample a CTA 4 lanes 454 us, 1 lane 508; eight, 627 and 568).
+    f.lanes = units <= 64 ? 4 : 1;
+    f.threads = (int32_t)(units * f.lanes >= 992 ? 992 : (units * f.lanes + 31) / 32 * 32) + 32;
+    return true;
+}
+
+cudaError_t launch_few(const KArgs &a, const FewArgs &f, cudaStream_t st) {
+    // CTAs along y: a warp for each item of the largest stage, up to 64 CTAs an SM in all
+    const int64_t lanes = f.n >= 32 ? 32 : f.n, run = f.n >= 32 ? kFewDrawRun : 1;
+    const int64_t items = ((int64_t)a.stage_entries * lanes + 32 * run - 1) / (32 * run) * ((f.n + 31) / 32);
+    const int64_t per = (items + kFewDrawThreads / 32 - 1) / (kFewDrawThreads / 32);
+    const int64_t most = (int64_t)64 * sm_count() / a.n_stages + 1;
+    const unsigned gy = (unsigned)(per < 1 ? 1 : per < most ? per : most);
+    const int64_t aux = f.durations && a.n_aux > 0 ? ((int64_t)a.n_aux * f.n + 128 * run * gy - 1) / (128 * run * gy) : 0;
+    void (*draw)(const KArgs, const FewArgs) = f.dur_in ? k_few_draw<true> : k_few_draw<false>;
+    draw<<<dim3((unsigned)(a.n_stages + (aux < 64 ? aux : 64)), gy), kFewDrawThreads, 0, st>>>(a, f);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    const bool pos = a.positive && !f.dur_in;
+    void (*fn)(const KArgs, const FewArgs) =
+        f.lanes == 4 ? pos ? k_few<true, 4> : k_few<false, 4> : pos ? k_few<true, 1> : k_few<false, 1>;
+    e = raise_smem_limit((const void *)fn, (size_t)f.smem);
+    if (e != cudaSuccess) return e;
+    fn<<<(unsigned)f.ctas, (unsigned)f.threads, (size_t)f.smem, st>>>(a, f);
+    return cudaGetLastError();
+}
+
+}  // namespace mcd

@@ -214,6 +214,8 @@ struct KArgs {
     int32_t n_warps;
     int32_t max_units;        // most and mean work units of a stage, by which the single-DAG launches choose
     int32_t avg_units;        // their warps per CTA (pick_warps); 0: n_warps is the caller's choice
+    int32_t stage_events, stage_entries;  // most events and precedence entries of a stage
+    int32_t n_events, n_entries;
     int32_t n_aux;
     int32_t window_slots;
     int32_t n_dist, n_alias;
@@ -273,6 +275,32 @@ struct KArgs {
 constexpr int32_t kAdjObjective = 1;  // forward: add (realized - earliest) to the objective sum
 constexpr int32_t kAdjCntLoad = 2;    // backward: start from the counts in cnt_ckpt (else zero)
 constexpr int32_t kAdjCntSave = 4;    // backward: leave the counts in cnt_ckpt for the next block
+
+// Few samples of one DAG (mcd_few.cu).
+constexpr int kFewInline = 8;   // seeds that travel with the launch
+constexpr int64_t kFewDirect = 40000;  // events times samples up to which they are written straight to the host
+constexpr int kFewRing = 8;     // most stage buffers
+constexpr size_t kFewSmem = 225 * 1024;
+constexpr size_t kFewScratch = (size_t)8 << 30;  // most scratch of a launch, and what a handle's pool keeps
+
+// Arguments beside the DAG's.  Element (row, sample) of an output lies at
+// row * out_row + sample * out_col, of durations at link * dur_row + sample * dur_col.
+struct FewArgs {
+    int64_t seed[kFewInline];
+    const int64_t *seeds;          // [n] on the device, or null: seed
+    int32_t n, ns_log;             // samples; log2 of a CTA's
+    int64_t out_row, out_col, dur_row, dur_col;
+    const double *dur_in;          // given durations, or null: drawn
+    double *realized, *durations;  // each may be null
+    int32_t *cause;                // may be null
+    double *entry_dur;             // scratch [ctas * cta_entries]: a CTA's durations in entry order
+    int64_t cta_entries;
+    size_t scratch;                // its bytes
+    // shared memory of the propagation: window, then `ring` buffers of a stage's event
+    // and predecessor records and durations
+    int32_t ring_off, ring, buf_bytes, pred_off, dur_off, smem;
+    int32_t ctas, threads, lanes;
+};
 
 // Arguments of the persistent batch kernel.
 struct BatchArgs {

@@ -164,7 +164,7 @@ cudaError_t raise_smem_limit(const void *fn, size_t smem) {
 }
 
 // SMs of the current device, 0 on error (looked up once per device).
-static int sm_count() {
+int sm_count() {
     static std::atomic<int> known[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
