@@ -183,31 +183,33 @@ static int64_t ctas_fit(int64_t smem) {
 }
 
 // Warps take a stage's units from a counter, so a CTA may have any number of them.
-// An SM's warps (sm_warps) are dealt out over the c CTAs it holds at a time, nw each,
-// a multiple of four (warps go to the four sub-partitions in turn; six or ten leave
-// two of them short).  c CTAs then take sm_warps / nw for their work and a tail at
-// each stage's barrier, half a unit's time or so: 0.55 sm_warps / U with U units a
-// stage (fitted to 30-130 events a level, 4 to 24 warps).  Several small CTAs hide
-// each other's barriers where many tiles queue for an SM; a launch of a tile or two an
-// SM wants every warp on them.
-// Measured against the compiler's choice, a sixth of the level width: one sample of
-// 1,000 events 250 -> 172 us (4 -> 16 warps), 20,017 events x 3,001 samples 2.95 ->
-// 1.75 ms (7 -> 24), 45 events a level x 30,000 samples, the statistics, 1.79 -> 1.58
-// (9 -> 8, three CTAs an SM where two fitted).
+// An SM's warps (sm_warps) are dealt out over the c CTAs it holds at a time, nw each.
+// With the issue time of a tile's stage as the unit and U work units a stage, a stage
+// takes k CTAs of nw warps D + max(k, 0.42 + 0.58 sm_warps / nw): D = 1.1 sm_warps / U, its
+// barrier and chain, which the CTAs share, and what nw warps need for a tile alone.
+// Tiles queue for an SM in rounds of c, the last of them with what is left.
+// (Fitted to 12-100 events a level, 1-17 tiles an SM, 4-24 warps: within 4 % of the
+// fastest, where multiples of four alone, and the last round as long as the others, lost
+// up to 13 %: 30 events a level, four tiles an SM 403 -> 356 us with four CTAs of six.)
+// Measured against the compiler's choice, a sixth of the level width: 20,017 events x
+// 3,001 samples 2.95 -> 1.75 ms (7 -> 24 warps), 45 events a level x 30,000 samples, the
+// statistics, 1.79 -> 1.58 (9 -> 12).
 int pick_warps(const KArgs &a, int64_t tiles, int sm_warps, int cta_warps) {
     const int sms = sm_count();
     if (a.max_units <= 0 || !sms) return a.n_warps;
     const int64_t per_sm = (tiles + sms - 1) / sms;
     const int64_t fit = ctas_fit(a.smem_total);
     const int most = (a.max_units + 3) / 4 * 4 < cta_warps ? (a.max_units + 3) / 4 * 4 : cta_warps;
-    const double tail = 0.55 * sm_warps / (a.avg_units > 0 ? a.avg_units : 1);
+    const double chain = 1.1 * sm_warps / (a.avg_units > 0 ? a.avg_units : 1);
     int best = 4;
     double best_cost = 0.0;
     for (int c = 1; c <= 8 && (c == 1 || (c <= fit && c <= per_sm)); ++c) {
-        int nw = sm_warps / c / 4 * 4;
+        int nw = sm_warps / c;
         nw = nw > most ? most : nw;
         if (nw < 4) break;
-        const double cost = (double)((per_sm + c - 1) / c) * ((double)sm_warps / nw + tail);
+        const double alone = 0.42 + 0.58 * sm_warps / nw;
+        auto round = [&](int64_t k) { return k ? chain + (k > alone ? (double)k : alone) : 0.0; };
+        const double cost = (double)(per_sm / c) * round(c) + round(per_sm % c);
         if (c == 1 || cost < best_cost) {
             best = nw;
             best_cost = cost;
