@@ -542,10 +542,52 @@ bool run_few(mcd_dag *g, const int64_t *seeds, const double *dur_in, int64_t n, 
     return true;
 }
 
+// Scratch of few-sample launches on callers' streams: one pool a device, made with the
+// first handle (so that no run waits for it).  It keeps what a launch may need, and
+// kFewIdle once no handle that used it is left.
+struct FewPool {
+    std::mutex mu;
+    bool made = false;
+    cudaMemPool_t pool = nullptr;  // null: not to be had
+    int users = 0;                 // handles that took from it
+};
+FewPool g_few_pool[64];
+constexpr size_t kFewIdle = (size_t)32 << 20;
+
+cudaMemPool_t few_pool(mcd_dag *g, bool use) {
+    if (g->device < 0 || g->device >= 64) return nullptr;
+    FewPool &fp = g_few_pool[g->device];
+    std::lock_guard<std::mutex> lk(fp.mu);
+    if (!fp.made) {
+        fp.made = true;
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = g->device;
+        uint64_t keep = kFewScratch;
+        void *p = nullptr;
+        if (cudaMemPoolCreate(&fp.pool, &props) != cudaSuccess ||
+            cudaMemPoolSetAttribute(fp.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess)
+            fp.pool = nullptr;
+        else if (cudaMallocFromPoolAsync(&p, kFewIdle, fp.pool, g->stream[0]) == cudaSuccess)
+            cudaFreeAsync(p, g->stream[0]);
+        (void)cudaGetLastError();
+    }
+    if (use && fp.pool && !g->few_used.exchange(true)) ++fp.users;
+    return fp.pool;
+}
+
+void few_pool_leave(mcd_dag *g) {
+    if (!g->few_used.exchange(false)) return;
+    FewPool &fp = g_few_pool[g->device];
+    std::lock_guard<std::mutex> lk(fp.mu);
+    if (--fp.users == 0 && cudaMemPoolTrimTo(fp.pool, kFewIdle) != cudaSuccess) (void)cudaGetLastError();
+}
+
 // The same with device buffers (a: the launch's arguments, sample-minor rows).  The
-// scratch comes from the handle's pool in the stream's order, so that calls on several
-// streams and threads share nothing; a stream that is being captured, and one whose
-// scratch cannot be had, keeps the general launch.
+// scratch is taken in the stream's order, so that calls on several streams and threads
+// share nothing; a stream that is being captured, and a launch whose scratch cannot be
+// had, keep the general kernels.
 bool run_few_device(mcd_dag *g, const KArgs &a, cudaStream_t st) {
     FewArgs f{};
     if (!few_layout(a, a.n, false, f)) return false;
@@ -554,24 +596,10 @@ bool run_few_device(mcd_dag *g, const KArgs &a, cudaStream_t st) {
         (void)cudaGetLastError();
         return false;
     }
-    {
-        std::lock_guard<std::mutex> lk(g->few_mu);
-        if (!g->few_pool) {
-            cudaMemPoolProps props{};
-            props.allocType = cudaMemAllocationTypePinned;
-            props.location.type = cudaMemLocationTypeDevice;
-            props.location.id = g->device;
-            uint64_t keep = kFewScratch;
-            if (cudaMemPoolCreate(&g->few_pool, &props) != cudaSuccess) {
-                (void)cudaGetLastError();
-                g->few_pool = nullptr;
-                return false;
-            }
-            cuda_check(cudaMemPoolSetAttribute(g->few_pool, cudaMemPoolAttrReleaseThreshold, &keep), "scratch pool");
-        }
-    }
+    const cudaMemPool_t pool = few_pool(g, true);
+    if (!pool) return false;
     void *p = nullptr;
-    if (cudaMallocFromPoolAsync(&p, f.scratch, g->few_pool, st) != cudaSuccess) {
+    if (cudaMallocFromPoolAsync(&p, f.scratch, pool, st) != cudaSuccess) {
         (void)cudaGetLastError();
         return false;
     }
@@ -699,6 +727,7 @@ int mcd_dag_create_ex(const mcd_dag_desc *desc, const mcd_generator *gen, const 
             cuda_check(cudaStreamCreateWithFlags(&g->stream[k], cudaStreamNonBlocking), "stream create");
         cuda_check(cudaMalloc(&g->d_err, 256), "error flag allocation");
         cuda_check(cudaMemset(g->d_err, 0, sizeof(int32_t)), "error flag init");
+        few_pool(g, false);
         *out = g;
     });
     if (rc != MCD_OK && g) {
@@ -720,7 +749,7 @@ void mcd_dag_destroy(mcd_dag *g) {
             cudaStreamDestroy(g->stream[k]);
         }
     if (g->ws) cudaFree(g->ws);
-    if (g->few_pool) cudaMemPoolDestroy(g->few_pool);  // (what is in use goes with its last cudaFreeAsync)
+    few_pool_leave(g);
     if (g->d_err) cudaFree(g->d_err);
     cudaSetDevice(prev);
     delete g;  // the image goes with its last handle

@@ -569,9 +569,8 @@ __device__ __forceinline__ void source(const TileCtx<S> &t, const double *win, i
 // clamp t = std::min(t, ub), and if (t >= latest) { latest = t; cause = src; } --
 // true when the entry takes the maximum over.
 template <bool POSITIVE>
-__device__ __forceinline__ bool relax(double src, double dur, long long ub_key, long long ub_bits, long long &lk,
-                                      long long &lbits, bool &clamp) {
-    const double tt = src + dur;
+__device__ __forceinline__ bool relax_time(double tt, long long ub_key, long long ub_bits, long long &lk,
+                                           long long &lbits, bool &clamp) {
     long long tb = __double_as_longlong(tt);
     long long tk = order_key<POSITIVE>(tb);
     clamp = ub_key < tk;
@@ -583,6 +582,11 @@ __device__ __forceinline__ bool relax(double src, double dur, long long ub_key, 
     lk = tk;
     lbits = POSITIVE ? tk : tb;
     return true;
+}
+template <bool POSITIVE>
+__device__ __forceinline__ bool relax(double src, double dur, long long ub_key, long long ub_bits, long long &lk,
+                                      long long &lbits, bool &clamp) {
+    return relax_time<POSITIVE>(src + dur, ub_key, ub_bits, lk, lbits, clamp);
 }
 
 // One stage's events under given durations, one at a time from the stage's counter

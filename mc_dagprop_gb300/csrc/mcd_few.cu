@@ -9,9 +9,9 @@
 // durations come through a ring of stage buffers that a warp of its own fills by bulk
 // copies several stages ahead.  It is bound by that chain, about 1,800 clocks a stage of
 // 100 events, and by the draws' instructions as the samples grow.
-// Measured, before and after: 1,000 events, one seed through host buffers 168 -> 68 us;
-// 200,000 events, one seed 13.1 -> 1.9 ms; on the device, 10,000 events x 152 samples
-// 642 -> 129 us, 20,017 x 608 1,757 -> 692, 200,000 x 608 12.8 -> 4.5 ms.
+// Measured, before and after: 1,000 events, one seed through host buffers 168 -> 63 us;
+// 200,000 events, one seed 13.1 -> 1.6 ms; on the device, 10,000 events x 152 samples
+// 642 -> 113 us, 20,017 x 608 1,757 -> 589, 200,000 x 608 12.8 -> 4.0 ms.
 #include "mcd_device.cuh"
 
 namespace mcd {
@@ -103,11 +103,20 @@ __global__ void __launch_bounds__(kFewDrawThreads) k_few_draw(const KArgs a, con
 // list decides ties as in the sequential loop (_core.cpp:338-347: a later equal time
 // takes over), so the maximum over (key, place), taken where its key reaches the event's
 // own, is the loop's result.
+// One lane an event: entries are read kAhead at a time, their loads and adds overlapping
+// (20,017 events x 608 samples 692 -> 589 us).  Several lanes: a thread's first unit of a
+// stage is read before the barrier that ends the stage before, so that the chain is the
+// window's read, the add, the maximum and the window's write (x 32 397 -> 358; one lane an
+// event gained nothing by it).  The copies of two stages ahead have then landed at each
+// barrier, of a ring of three buffers at least.
 template <bool POSITIVE, int G>
-__global__ void __launch_bounds__(1024, 1) k_few(const KArgs a, const FewArgs f) {
+__global__ void __launch_bounds__(G == 1 ? 1024 : 544, 1) k_few(const KArgs a, const FewArgs f) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t bars[kFewRing];
     __shared__ int2 head[kFewRing];  // of the stage in a buffer: events, first entry
+    constexpr int kAhead = 4;
+    constexpr bool kEarly = G > 1;
+    constexpr int ahead = kEarly ? 2 : 1; // stages whose copies have landed at a barrier
     double *win = reinterpret_cast<double *>(smem);
     unsigned char *ring = smem + f.ring_off;
     const int lane = threadIdx.x & 31, R = f.ring, NS = a.n_stages, ns = 1 << f.ns_log;
@@ -131,6 +140,10 @@ __global__ void __launch_bounds__(1024, 1) k_few(const KArgs a, const FewArgs f)
         if (m.w) bulk_g2s(buf + f.pred_off, a.pred + m.z, pr_bytes, &bars[b]);
         if (m.w) bulk_g2s(buf + f.dur_off, entry_dur + (few_first(l, m.z) << f.ns_log), du_bytes, &bars[b]);
     };
+    // (the workers are a multiple of G * ns: a thread's units are all of one sample)
+    const int j = ((int)threadIdx.x / G) & (ns - 1), s = (blockIdx.x << f.ns_log) + j;
+    double *wcol = win + j, *rcol = f.realized && s < f.n ? f.realized + s * f.out_col : nullptr;
+    int32_t *ccol = f.cause && s < f.n ? f.cause + s * f.out_col : nullptr;
     bool ok = true;
     int issued = 0, waits = 0;  // the producer's: stages copied, and the one last waited for
     if (producer) {
@@ -139,69 +152,107 @@ __global__ void __launch_bounds__(1024, 1) k_few(const KArgs a, const FewArgs f)
         for (; issued < R && issued < NS; ++issued) fill(issued, __ldg(meta + kVecs * issued));
         for (int k = 0; k < 2; ++k)
             if (R + k < NS) m_next[k] = __ldg(meta + kVecs * (R + k));
-        if (NS > 0) ok = stage_wait(&bars[0], 0u, a.err);
+        for (; waits < ahead && waits < NS && ok; ++waits) ok = stage_wait(&bars[waits], 0u, a.err);
+        --waits;
     }
-    if (!__syncthreads_or(!ok)) {
-        int b = 0;
-        uint32_t phase = 0;
-        for (int l = 0; l < NS; ++l) {
-            if ((int)threadIdx.x < workers) {
-                const int2 h = head[b];
-                const unsigned char *buf = ring + b * f.buf_bytes;
-                const EvRec *sev = reinterpret_cast<const EvRec *>(buf);
-                const PredRec *pred = reinterpret_cast<const PredRec *>(buf + f.pred_off);
-                const double *durs = reinterpret_cast<const double *>(buf + f.dur_off);
-                const unsigned group = G == 32 ? 0xFFFFFFFFu : ((1u << G) - 1u) << (lane & ~(G - 1));
-                for (int u = threadIdx.x; u < (h.x * G) << f.ns_log; u += workers) {
-                    const int j = (u / G) & (ns - 1);
-                    const EvRec ev = load_ev(sev + ((u / G) >> f.ns_log));
-                    const long long init_key = POSITIVE ? ev.init_bits : ev.init_key;
-                    const long long ub_key = POSITIVE ? ev.ub_bits : ev.ub_key;
-                    const int pb = ev.pred_begin - h.y, pe = ev.pred_end - h.y;
-                    long long key = (long long)0x8000000000000000ull, bits = 0;  // (below any event's own key)
-                    int place = -1, cause = -1;
-                    for (int p = pb + (u & (G - 1)); p < pe; p += G) {
-                        const int2 src = *reinterpret_cast<const int2 *>(pred + p);  // src_slot, src_user
-                        bool clamp;
-                        if (relax<POSITIVE>(win[(window_row<1>(src.x) << f.ns_log) + j], durs[(p << f.ns_log) + j], ub_key,
-                                            ev.ub_bits, key, bits, clamp)) {
-                            place = p;
-                            cause = src.y;
-                        }
-                    }
-                    long long best = key;
-                    int at = place;
+    // A thread's unit: its event, and its first entry with its duration (kEarly).
+    EvRec ev{};
+    int2 src{};  // src_slot, src_user
+    double dur = 0.0;
+    int p0 = 0, pe = 0;  // its first entry, and its event's end, in the stage's entries
+    const PredRec *pred = nullptr;
+    const double *dcol = nullptr;
+    auto fetch = [&](int b, int u) {  // unit u of the stage in buffer b
+        const unsigned char *buf = ring + b * f.buf_bytes;
+        pred = reinterpret_cast<const PredRec *>(buf + f.pred_off);
+        dcol = reinterpret_cast<const double *>(buf + f.dur_off) + j;
+        ev = load_ev(reinterpret_cast<const EvRec *>(buf) + ((u / G) >> f.ns_log));
+        p0 = ev.pred_begin - head[b].y + (u & (G - 1));
+        pe = ev.pred_end - head[b].y;
+        if (kEarly && p0 < pe) {
+            src = *reinterpret_cast<const int2 *>(pred + p0);
+            dur = dcol[p0 << f.ns_log];
+        }
+    };
+    const unsigned group = ((1u << G) - 1u) << (lane & ~(G - 1));
+    auto run = [&]() {
+        const long long init_key = POSITIVE ? ev.init_bits : ev.init_key;
+        const long long ub_key = POSITIVE ? ev.ub_bits : ev.ub_key;
+        long long key = (long long)0x8000000000000000ull, bits = 0;  // (below any event's own key)
+        int place = -1, cause = -1;
+        if constexpr (kEarly) {
+            for (int p = p0;;) {
+                bool clamp;
+                if (p < pe && relax_time<POSITIVE>(wcol[window_row<1>(src.x) << f.ns_log] + dur, ub_key, ev.ub_bits, key,
+                                                   bits, clamp)) {
+                    place = p;
+                    cause = src.y;
+                }
+                p += G;
+                if (p >= pe) break;
+                src = *reinterpret_cast<const int2 *>(pred + p);
+                dur = dcol[p << f.ns_log];
+            }
+        } else {
+            for (int p = p0; p < pe; p += kAhead) {
+                int2 from[kAhead];
+                double t[kAhead];
 #pragma unroll
-                    for (int m = 1; m < G; m *= 2) {
-                        const long long k = __shfl_xor_sync(group, best, m);
-                        const int q = __shfl_xor_sync(group, at, m);
-                        if (k > best || (k == best && q > at)) {
-                            best = k;
-                            at = q;
-                        }
+                for (int k = 0; k < kAhead; ++k)
+                    if (p + k < pe) {
+                        from[k] = *reinterpret_cast<const int2 *>(pred + p + k);
+                        t[k] = wcol[window_row<1>(from[k].x) << f.ns_log] + dcol[(p + k) << f.ns_log];
                     }
-                    const bool taken = at >= 0 && best >= init_key;
-                    if (G == 1 || (taken ? place == at : (u & (G - 1)) == 0)) {
-                        if (!taken) {
-                            cause = -1;
-                            bits = ub_key < init_key ? ev.ub_bits : ev.init_bits;  // realized = std::min(latest, ub)
-                        }
-                        const double v = __longlong_as_double(bits);
-                        const int slot = window_row<1>(ev.slot);
-                        if (slot >= 0) win[(slot << f.ns_log) + j] = v;
-                        const int s = (blockIdx.x << f.ns_log) + j;
-                        if (s < f.n) {
-                            if (f.realized) f.realized[(int64_t)ev.user * f.out_row + s * f.out_col] = v;
-                            if (f.cause) f.cause[(int64_t)ev.user * f.out_row + s * f.out_col] = cause;
-                        }
-                    }
+#pragma unroll
+                for (int k = 0; k < kAhead; ++k) {
+                    bool clamp;
+                    if (p + k < pe && relax_time<POSITIVE>(t[k], ub_key, ev.ub_bits, key, bits, clamp)) cause = from[k].y;
                 }
             }
+        }
+        long long best = key;
+        int at = place;
+#pragma unroll
+        for (int m = 1; m < G; m *= 2) {
+            const long long k = __shfl_xor_sync(group, best, m);
+            const int q = __shfl_xor_sync(group, at, m);
+            if (k > best || (k == best && q > at)) {
+                best = k;
+                at = q;
+            }
+        }
+        const bool taken = best >= init_key;  // (an event without entries has none: its key is above)
+        if (G == 1 || (taken ? place == at : (lane & (G - 1)) == 0)) {
+            if (!taken) {
+                cause = -1;
+                bits = ub_key < init_key ? ev.ub_bits : ev.init_bits;  // realized = std::min(latest, ub)
+            }
+            const double v = __longlong_as_double(bits);
+            const int slot = window_row<1>(ev.slot);
+            if (slot >= 0) wcol[slot << f.ns_log] = v;
+            if (rcol) *at_row(rcol, ev.user, (uint32_t)f.out_row * 8u) = v;
+            if (ccol) *at_row(ccol, ev.user, (uint32_t)f.out_row * 4u) = cause;
+        }
+    };
+    if (!__syncthreads_or(!ok)) {
+        int b = 0, b2 = ahead;  // buffers of stages l and l + ahead
+        uint32_t phase2 = 0;    // phase of the latter
+        if (kEarly && (int)threadIdx.x < workers && (int)threadIdx.x < (head[0].x * G) << f.ns_log) fetch(0, threadIdx.x);
+        for (int l = 0; l < NS; ++l) {
             const int nb = b + 1 == R ? 0 : b + 1;
-            const uint32_t nphase = phase ^ (nb == 0 ? 1u : 0u);
-            if (producer && l + 1 < NS) {
-                waits = l + 1;
-                ok = stage_wait(&bars[nb], nphase, a.err);
+            if ((int)threadIdx.x < workers) {
+                const int units = (head[b].x * G) << f.ns_log;
+                if (kEarly && (int)threadIdx.x < units) run();
+                for (int u = threadIdx.x + (kEarly ? workers : 0); u < units; u += workers) {
+                    fetch(b, u);
+                    run();
+                }
+                // the next stage's first unit: its records have landed, and off its chain
+                if (kEarly && l + 1 < NS && (int)threadIdx.x < (head[nb].x * G) << f.ns_log) fetch(nb, threadIdx.x);
+            }
+            if (producer && l + ahead < NS) {
+                waits = l + ahead;
+                ok = stage_wait(&bars[b2], phase2, a.err);
             }
             if (__syncthreads_or(!ok)) break;
             if (producer && l + R < NS) {
@@ -211,7 +262,10 @@ __global__ void __launch_bounds__(1024, 1) k_few(const KArgs a, const FewArgs f)
                 if (l + R + 2 < NS) m_next[1] = __ldg(meta + kVecs * (l + R + 2));
             }
             b = nb;
-            phase = nphase;
+            if (++b2 == R) {
+                b2 = 0;
+                phase2 ^= 1u;
+            }
         }
     }
     if (producer && !ok)  // a copy that never landed: drain the others in flight, then leave
@@ -225,12 +279,12 @@ int sm_count();
 // kFewScratch, and sizes where it measured no faster.  With `work` the stages plus a 64th
 // of the events: samples drawn, general and few,
 //   100 events in 2 stages (work 4)   8.3 and 12.7 us: the second launch is not repaid
-//   203 in 11 (14)    x 152 24.7, 21.2   x 608 24.7, 22.7   x 2,432 24.7, 27.8
-//   600 in 20 (29)    x 152 59, 29       x 608 59, 37       x 2,432 59, 58
-//   20,017 in 545 (860) x 1,216 1,758, 934   x 2,432 1,760, 1,470   x 3,001 1,758, 1,857
+//   203 in 11 (14)    x 152 24.7, 20.5   x 608 24.7, 20.7   x 2,432 24.7, 27.8
+//   600 in 20 (29)    x 152 59, 27       x 608 59, 33       x 2,432 59, 58
+//   20,017 in 493 (805) x 1,216 1,758, 833   x 2,432 1,760, 1,366   x 3,001 1,758, 1,857
 // and durations given, whose general kernel has less to do a stage,
 //   203  x 152 20.6, 19.9   x 608 20.6, 23.1;  600  x 608 45, 38   x 1,216 45, 43
-//   20,017  x 1,216 1,427, 998   x 2,432 1,432, 1,475
+//   20,017  x 1,216 1,427, 867   x 2,432 1,432, 1,475
 // direct: the rows go straight to the host, which saves more launches than this adds.
 bool few_layout(const KArgs &a, int64_t n, bool direct, FewArgs &f) {
     const int sms = sm_count();
@@ -250,19 +304,20 @@ bool few_layout(const KArgs &a, int64_t n, bool direct, FewArgs &f) {
     const size_t ev = (size_t)a.stage_events * sizeof(EvRec), pred = (size_t)a.stage_entries * sizeof(PredRec);
     const size_t dur = ((size_t)(a.stage_entries + 1) / 2 * 2 << f.ns_log) * sizeof(double);
     const size_t buf = (ev + pred + dur + 127) / 128 * 128;
-    if (win + 2 * buf > kFewSmem) return false;
+    const int64_t units = (int64_t)a.stage_events << f.ns_log;
+    // Lanes over an event's entries shorten its chain while the stage's warps are few; past
+    // some 16 warps their reductions cost more issue than they save (50,000 events in stages
+    // of up to 128: one sample a CTA 1 lane 681 us, 4 lanes 594; 20,017 in stages of 37,
+    // eight samples: 1 lane 568, 4 lanes 627).
+    f.lanes = units <= 128 ? 4 : 1;
+    if (win + (f.lanes > 1 ? 3 : 2) * buf > kFewSmem) return false;
     f.ring_off = (int32_t)win;
     f.pred_off = (int32_t)ev;
     f.dur_off = (int32_t)(ev + pred);
     f.buf_bytes = (int32_t)buf;
     f.ring = (int32_t)((kFewSmem - win) / buf < (size_t)kFewRing ? (kFewSmem - win) / buf : kFewRing);
     f.smem = (int32_t)(win + f.ring * buf);
-    const int64_t units = (int64_t)a.stage_events << f.ns_log;
-    // Lanes over an event's entries shorten its chain while the stage's warps are few; past
-    // some 8 warps their reductions cost more issue than they save (20,017 events in stages
-    // of 37: one sample a CTA 4 lanes 454 us, 1 lane 508; eight, 627 and 568).
-    f.lanes = units <= 64 ? 4 : 1;
-    f.threads = (int32_t)(units * f.lanes >= 992 ? 992 : (units * f.lanes + 31) / 32 * 32) + 32;
+    f.threads = (int32_t)(units * f.lanes >= 960 ? 960 : (units * f.lanes + 63) / 64 * 64) + 32;  // (64: lanes << ns_log at most)
     return true;
 }
 

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <memory>
 #include <mutex>
 #include <new>
@@ -68,8 +69,7 @@ struct mcd_dag {
     int32_t *d_err = nullptr;  // latched kernel errors of this handle's launches
     char *ws = nullptr;        // workspace
     size_t ws_bytes = 0;
-    std::mutex few_mu;                   // guards the making of few_pool
-    cudaMemPool_t few_pool = nullptr;    // scratch of few-sample launches on the caller's streams
+    std::atomic<bool> few_used{false};  // counted among the users of the device's few-sample scratch pool
     int64_t last_adj_plan[3] = {0, 0, 0};  // the last gradient's samples per chunk, level blocks, buffer bytes
     explicit mcd_dag(std::shared_ptr<const mcd::DagImage> image)
         : img(std::move(image)), h(img->h), device(img->device), dbytes(img->dbytes), d_ev(img->d_ev),
