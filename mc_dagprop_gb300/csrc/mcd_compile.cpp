@@ -240,7 +240,7 @@ void verify_layout(const HostDag &H) {
                         fail("link table without a table");
                     }
                 }
-                if (!H.win_smem) {
+                if (!H.rows_planned) {
                     if (p.src_slot != -1) fail("window slot without a window");
                     continue;
                 }
@@ -259,7 +259,7 @@ void verify_layout(const HostDag &H) {
             }
             const int32_t er = narrow_row(r.slot);
             if (er >= 0) {
-                if (!H.win_smem || er >= H.window_slots || last_read[(size_t)er] >= st)
+                if (!H.rows_planned || er >= H.window_slots || last_read[(size_t)er] >= st)
                     fail("window slot reuse");
                 tenant[(size_t)er] = r.user;
             } else if (er != -1) {
@@ -799,6 +799,10 @@ void compile_dag(const mcd_dag_desc &d, const mcd_generator &g, HostDag &H, int3
     const size_t win_bytes = (size_t)H.window_slots * kTile * sizeof(double);
     H.win_smem = win_bytes <= kMaxWindowBytes && win_bytes + fixed_bytes + 2 * kMinStageBytes <= kSmemMax &&
                  window != MCD_WINDOW_GLOBAL && std::getenv("MCD_NO_SMEM_WINDOW") == nullptr;
+    // Few-sample launches have short rows, so their window is on chip also where 256-byte
+    // rows are too many (unless the caller wants it off chip).
+    H.rows_planned = H.win_smem || (H.window_slots <= 0x7FFF && window != MCD_WINDOW_GLOBAL &&
+                                    std::getenv("MCD_NO_SMEM_WINDOW") == nullptr);
     const size_t avail = kSmemMax - fixed_bytes - (H.win_smem ? win_bytes : 0);
     size_t budget = std::min(kMaxStageBytes, avail / 2 > 256 ? avail / 2 - 256 : avail / 2);  // room for padding
 
@@ -1002,7 +1006,7 @@ void compile_dag(const mcd_dag_desc &d, const mcd_generator &g, HostDag &H, int3
         }
         EvRec r{};
         r.user = e;
-        r.slot = H.win_smem ? slot_word(slot[e], slot[e]) : -1;
+        r.slot = H.rows_planned ? slot_word(slot[e], slot[e]) : -1;
         r.pred_begin = (int32_t)H.pred.size();
         const double earliest = d.earliest[e];
         const double ub = earliest + d.max_delay;  // _core.cpp:334
@@ -1014,7 +1018,7 @@ void compile_dag(const mcd_dag_desc &d, const mcd_generator &g, HostDag &H, int3
             const int32_t src = d.pred_src[tstart[e] + k];
             const int32_t l = d.pred_act[tstart[e] + k];
             PredRec p{};
-            p.src_slot = H.win_smem ? slot_word(slot[src], slot[src]) : -1;
+            p.src_slot = H.rows_planned ? slot_word(slot[src], slot[src]) : -1;
             p.src_user = src;
             if (l >= L) {
                 // Past the last link the reference reads beyond its duration

@@ -274,10 +274,12 @@ __global__ void __launch_bounds__(G == 1 ? 1024 : 544, 1) k_few(const KArgs a, c
 
 int sm_count();
 
-// The layout of a launch of n samples; false where this path does not apply: windows off
-// chip, warps per CTA that the caller fixed, stages that leave no ring, more scratch than
-// kFewScratch, and sizes where it measured no faster.  With `work` the stages plus a 64th
-// of the events: samples drawn, general and few,
+// The layout of a launch of n samples; false where this path does not apply: a window that
+// the caller wants off chip, warps per CTA that the caller fixed, stages that leave no
+// ring, more scratch than kFewScratch, and sizes where it measured no faster.  (A window
+// too large for rows of 32 samples is no obstacle: 50,000 events in levels of 200 x 152
+// samples 3,690 -> 645 us.)  With `work` the stages plus a 64th of the events: samples
+// drawn, general and few,
 //   100 events in 2 stages (work 4)   8.3 and 12.7 us: the second launch is not repaid
 //   203 in 11 (14)    x 152 24.7, 20.5   x 608 24.7, 20.7   x 2,432 24.7, 27.8
 //   600 in 20 (29)    x 152 59, 27       x 608 59, 33       x 2,432 59, 58
@@ -288,7 +290,7 @@ int sm_count();
 // direct: the rows go straight to the host, which saves more launches than this adds.
 bool few_layout(const KArgs &a, int64_t n, bool direct, FewArgs &f) {
     const int sms = sm_count();
-    if (n < 1 || !a.win_smem || a.avg_units <= 0 || a.n_stages <= 0 || sms <= 0) return false;
+    if (n < 1 || !a.rows_planned || a.avg_units <= 0 || a.n_stages <= 0 || sms <= 0) return false;
     const int64_t work = a.n_stages + a.n_events / 64;
     if (!direct && work < (a.dur_in ? 24 : 8)) return false;
     const int most = work < 32 ? 2 : a.dur_in ? 3 : 4;

@@ -60,6 +60,7 @@ constexpr size_t kSmemMax = 226 * 1024;  // 227 KB per CTA, less room for static
 struct HostDag {
     int32_t E = 0, L = 0, n_levels = 0, n_warps = 1, window_slots = 0;
     bool win_smem = true;
+    bool rows_planned = true;     // slot words hold window rows (also where the general kernels' window is off chip)
     bool positive = false;        // all times non-negative and finite
     int64_t max_preds = 0;        // largest predecessor list
     bool tables_in_smem = true;

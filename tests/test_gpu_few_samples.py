@@ -1,6 +1,6 @@
 """A handful of samples (lanes over predecessors) against the general kernels and the
 oracle, bit for bit: every sampler, lists longer than the lanes, stages with more units
-than threads, one stage, times of both signs, sample counts around the steps of a CTA's
+than threads, one stage, a window too large for tiles of 32, times of both signs, sample counts around the steps of a CTA's
 samples and past the last, page-locked, ordinary and device buffers, two streams at once,
 a captured stream."""
 from __future__ import annotations
@@ -22,7 +22,8 @@ def _bits(a):
 
 
 @pytest.mark.parametrize("layers,width,preds,shift,big", [(6, 150, 12, 0.0, False), (40, 7, 4, -500.0, False),
-                                                          (1, 3, 1, 0.0, False), (5, 900, 4, 0.0, True)])
+                                                          (1, 3, 1, 0.0, False), (5, 900, 4, 0.0, True),
+                                                          (9, 1100, 4, 0.0, False)])
 @pytest.mark.parametrize("n", [1, 3, 8, 9, 153, 1217, 2433])
 def test_rows_equal_the_general_kernels_and_the_oracle(cuda, layers, width, preds, shift, big, n):
     flat, gen = kitchen_sink(seed=6, n_layers=layers, width=width, big_table=big, max_preds=preds)
