@@ -134,7 +134,8 @@ int mcd_dag_create(const mcd_dag_desc *desc, const mcd_generator *gen, mcd_dag *
 /* Compile options (the same call with explicit choices). */
 #define MCD_WARPS_BATCH_CLASS (-1)
 typedef struct mcd_dag_options {
-    int32_t n_warps; /* warps per CTA, 1..24; 0 = chosen from the DAG's level width;
+    int32_t n_warps; /* warps per CTA, 1..24 (kept by every launch); 0 = chosen from the
+                        DAG's level width and, per launch, its samples;
                         MCD_WARPS_BATCH_CLASS = chosen, then rounded up to 2, 4, 8, 12 or 24 */
     int32_t no_cache; /* 0: share the compiled records of a live handle created from
                          identical inputs (same arrays, generator, options and device);
@@ -182,7 +183,9 @@ int mcd_propagate_host(mcd_dag *dag, const double *durations, int64_t n, double 
 /* ---- Device buffers, sample-minor, asynchronous on `stream` (NULL = the handle's stream) ----
  * seeds[n] on the device; outputs realized[E*ld], durations[L*ld], cause_event[E*ld]
  * (any may be NULL).  Kernel errors are latched on the handle and reported by
- * mcd_dag_check(). */
+ * mcd_dag_check().  Runs of few samples take scratch memory from a pool in the
+ * stream's order (not while the stream is captured, nor where it cannot be had: the
+ * same results by the general kernels). */
 int mcd_run_device(mcd_dag *dag, const int64_t *seeds, int64_t n, double *realized, double *durations,
                    int32_t *cause_event, int64_t ld, void *stream);
 /* Propagation alone from device durations[L*ld_in] (sample-minor). */

@@ -4,14 +4,14 @@
 // its levels are then a chain: an event's entries one after another, each a Philox block
 // and a sampler, some 5,000 clocks a stage.  Here the draws come first, on all SMs
 // (k_few_draw), into a scratch in the order in which the propagation reads them; then a
-// CTA of one to sixteen samples walks the stages (k_few).  What is left of a stage is a
+// CTA of one to twenty samples walks the stages (k_few).  What is left of a stage is a
 // barrier, one add and a maximum, and nothing else may lie on that path: records and
 // durations come through a ring of stage buffers that a warp of its own fills by bulk
 // copies several stages ahead.  It is bound by that chain, about 1,800 clocks a stage of
 // 100 events, and by the draws' instructions as the samples grow.
-// Measured, before and after: 1,000 events, one seed through host buffers 168 -> 63 us;
-// 200,000 events, one seed 13.1 -> 1.6 ms; on the device, 10,000 events x 152 samples
-// 642 -> 113 us, 20,017 x 608 1,757 -> 589, 200,000 x 608 12.8 -> 4.0 ms.
+// Measured, before and after: 1,000 events, one seed through host buffers 168 -> 62 us;
+// 200,000 events, one seed 13.1 -> 1.5 ms; on the device, 10,000 events x 152 samples
+// 642 -> 111 us, 20,017 x 608 1,757 -> 560, 200,000 x 608 12.8 -> 3.8 ms.
 #include "mcd_device.cuh"
 
 namespace mcd {
@@ -25,81 +25,118 @@ __device__ __forceinline__ int64_t few_first(int stage, int first_entry) {
     return (int64_t)((uint32_t)(first_entry + stage + 1) & ~1u);
 }
 
-// Durations of the stage blockIdx.x.  A warp's lanes are the samples of a block of up to
-// 32 and, when n is smaller, several entries; a lane takes kFewDrawRun entries one after
-// another where n fills the lanes (one otherwise: latency), drawing a Philox block once
-// for the entries that share it.  The last CTAs draw the links no entry references.  The
-// draws are the sampled propagation's own (same records, blocks, words and arithmetic):
-// equal bits.
+// Durations of the stage blockIdx.x.  A warp's lanes are the samples of a block of 32 S
+// (S a lane: a record is read and decoded once for them, and their chains overlap) and,
+// when n is smaller, several entries; a lane takes kFewDrawRun entries one after another
+// where n fills the lanes (one otherwise: latency), drawing a Philox block once for the
+// entries that share it.  The last CTAs draw the links no entry references.  The draws are
+// the sampled propagation's own (same records, blocks, words and arithmetic): equal bits.
+// Bound by instructions (148 per 32 draws at one sample a lane, 60 % issue active).  Both
+// kernels, 20,017 events: x 1,216 832 us with one sample a lane, 750 with two, 742 with
+// four; x 2,432 1,388, 1,256, 1,197; x 152 412, 411, 419.
 constexpr int kFewDrawRun = 4;
-template <bool GIVEN>
+template <bool GIVEN, int S>
 __global__ void __launch_bounds__(kFewDrawThreads) k_few_draw(const KArgs a, const FewArgs f) {
-    const int stage = blockIdx.x, n = f.n, ns = 1 << f.ns_log, lane = threadIdx.x & 31;
+    const int stage = blockIdx.x, n = f.n, ns = f.ns, lane = threadIdx.x & 31;
     const DistParam *dists = a.dist;
     const AliasEntry *alias = reinterpret_cast<const AliasEntry *>(dists + a.n_dist);
     const AliasPick *picks = reinterpret_cast<const AliasPick *>(alias + a.n_alias);
     const int lanes_log = n > 16 ? 5 : n > 8 ? 4 : n > 4 ? 3 : n > 2 ? 2 : n > 1 ? 1 : 0;  // of a lane's samples
     const int run = n >= 32 ? kFewDrawRun : 1;
-    const int blocks = (n + 31) >> 5, per_warp = run << (5 - lanes_log);  // sample blocks; entries a warp takes
-    U4 words{};
+    const int blocks = (n + 32 * S - 1) / (32 * S), per_warp = run << (5 - lanes_log);  // sample blocks; entries a warp takes
+    U4 words[S];
     uint32_t drawn = 0xFFFFFFFFu;  // the block `words` are of (no block has this number)
-    uint64_t seed = 0;
-    auto draw = [&](int kd, double v, const double *vt, uint32_t block, uint32_t link) {
+    uint64_t seed[S];
+    auto draw = [&](int kd, double v, const double *vt, uint32_t block, uint32_t link, double (&d)[S]) {
         const int kind = kd & KD_KIND_MASK;
-        if (kind == K_FIXED) return v;
+#pragma unroll
+        for (int j = 0; j < S; ++j) d[j] = v;
+        if (kind == K_FIXED) return;
         const DistParam &p = dists[kd >> 8];
         float dfac;
-        if (kind == K_GAMMA && !p.erlang) return draw_gamma(p, v, block, seed, a.err, &dfac);
-        if (block != drawn) words = draw_words(seed, block, 0u, 0u);
+        if (kind == K_GAMMA && !p.erlang) {
+#pragma unroll
+            for (int j = 0; j < S; ++j) d[j] = draw_gamma(p, v, block, seed[j], a.err, &dfac);
+            return;
+        }
+        if (block != drawn) {
+#pragma unroll
+            for (int j = 0; j < S; ++j) words[j] = draw_words(seed[j], block, 0u, 0u);
+        }
         drawn = block;
         const int w = (kd >> KD_WORD_SHIFT) & 3;
-        if (kind == K_GAMMA) return draw_erlang(p, v, link, seed, words, w, a.err, &dfac);
-        if (kind == K_EXP) return draw_exponential(p, v, word_of(words, w), dfac);
-        return draw_empirical(p, alias, picks, vt, v, kind == K_EMP_REL, word_of(words, w), words.y,
-                              (kd & KD_TWO_WORD) != 0, dfac);
+        if (kind == K_GAMMA) {
+#pragma unroll
+            for (int j = 0; j < S; ++j) d[j] = draw_erlang(p, v, link, seed[j], words[j], w, a.err, &dfac);
+        } else if (kind == K_EXP) {
+#pragma unroll
+            for (int j = 0; j < S; ++j) d[j] = draw_exponential(p, v, word_of(words[j], w), dfac);
+        } else {
+#pragma unroll
+            for (int j = 0; j < S; ++j)
+                d[j] = draw_empirical(p, alias, picks, vt, v, kind == K_EMP_REL, word_of(words[j], w), words[j].y,
+                                      (kd & KD_TWO_WORD) != 0, dfac);
+        }
     };
     const bool aux = stage >= a.n_stages;
     const int4 meta = aux ? make_int4(0, 0, 0, a.n_aux) : __ldg(reinterpret_cast<const int4 *>(a.stage_meta + kStageMetaInts * stage));
     const int4 mv = aux ? meta : __ldg(reinterpret_cast<const int4 *>(a.stage_meta + kStageMetaInts * stage) + 1);
-    double *out = aux ? nullptr : f.entry_dur + (few_first(stage, meta.z) << f.ns_log);
+    double *out = aux ? nullptr : f.entry_dur + few_first(stage, meta.z) * ns;
     const int cta = blockIdx.y + (aux ? (stage - a.n_stages) * gridDim.y : 0);
     const int ctas = aux ? (gridDim.x - a.n_stages) * gridDim.y : gridDim.y;
     const int items = (meta.w + per_warp - 1) / per_warp * blocks;
     for (int item = cta * (kFewDrawThreads / 32) + (threadIdx.x >> 5); item < items; item += ctas * (kFewDrawThreads / 32)) {
         const int g = item / blocks;
-        const int s = ((item - g * blocks) << 5) + (lane & ((1 << lanes_log) - 1));
+        const int s = (item - g * blocks) * (32 * S) + (lane & ((1 << lanes_log) - 1));
         if (s >= n) continue;
-        seed = f.seeds ? (uint64_t)__ldg(f.seeds + s) : (uint64_t)f.seed[s & (kFewInline - 1)];
+        int64_t of_cta[S], col[S];  // (a CTA of the propagation reads its own samples)
+        bool in[S];
+#pragma unroll
+        for (int j = 0; j < S; ++j) {
+            const int sj = s + 32 * j;
+            in[j] = sj < n;
+            seed[j] = !in[j] ? 0 : f.seeds ? (uint64_t)__ldg(f.seeds + sj) : (uint64_t)f.seed[sj & (kFewInline - 1)];
+            of_cta[j] = (int64_t)(sj / ns) * f.cta_entries + sj % ns;
+            col[j] = sj * f.dur_col;
+        }
         drawn = 0xFFFFFFFFu;
         const int first = g * per_warp + (lane >> lanes_log) * run;
         for (int i = first; i < first + run && i < meta.w; ++i) {
+            double dur[S];
             if (aux) {
                 const LinkRec lr = a.aux[i];  // (owns its block)
-                f.durations[(int64_t)lr.link * f.dur_row + s * f.dur_col] =
-                    draw(lr.kd, lr.v, nullptr, (uint32_t)lr.link, (uint32_t)lr.link);
+                draw(lr.kd, lr.v, nullptr, (uint32_t)lr.link, (uint32_t)lr.link, dur);
+#pragma unroll
+                for (int j = 0; j < S; ++j)
+                    if (in[j]) f.durations[(int64_t)lr.link * f.dur_row + col[j]] = dur[j];
                 continue;
             }
             const int4 *q = reinterpret_cast<const int4 *>(a.pred + meta.z + i);
             const int4 r0 = __ldg(q);  // src_slot, src_user, link, kd
-            double dur = 0.0;
             if (GIVEN) {
-                if (r0.z >= 0) dur = __ldg(f.dur_in + (int64_t)r0.z * f.dur_row + s * f.dur_col);
+#pragma unroll
+                for (int j = 0; j < S; ++j) dur[j] = r0.z >= 0 && in[j] ? __ldg(f.dur_in + (int64_t)r0.z * f.dur_row + col[j]) : 0.0;
             } else {
                 const int4 r1 = __ldg(q + 1);  // v, dvo, block
                 const double *vt = nullptr;
                 if (r1.z >= 0 && (r0.w & KD_KIND_MASK) != K_FIXED)
                     vt = meta.y >= 0 ? a.vals + mv.x + (r1.z - mv.w) / (int)sizeof(double) : a.vals + (r1.z ^ kVtGlobal);
-                dur = draw(r0.w, __hiloint2double(r1.y, r1.x), vt, (uint32_t)r1.w, (uint32_t)r0.z);
-                if (f.durations && (r0.w & KD_WRITE)) f.durations[(int64_t)r0.z * f.dur_row + s * f.dur_col] = dur;
+                draw(r0.w, __hiloint2double(r1.y, r1.x), vt, (uint32_t)r1.w, (uint32_t)r0.z, dur);
+                if (f.durations && (r0.w & KD_WRITE)) {
+#pragma unroll
+                    for (int j = 0; j < S; ++j)
+                        if (in[j]) f.durations[(int64_t)r0.z * f.dur_row + col[j]] = dur[j];
+                }
             }
-            // (CTA s / ns of the propagation reads its samples alone)
-            out[(int64_t)(s >> f.ns_log) * f.cta_entries + ((int64_t)i << f.ns_log) + (s & (ns - 1))] = dur;
+#pragma unroll
+            for (int j = 0; j < S; ++j)
+                if (in[j]) out[of_cta[j] + (int64_t)i * ns] = dur[j];
         }
     }
 }
 
-// One CTA for 2^ns_log samples, its last warp the producer: unit u of a stage is lane
-// u % G of sample (u / G) % 2^ns_log of event u / G / 2^ns_log.  An entry's place in its
+// One CTA for ns samples, its last warp the producer.  Of the others' threads, G lanes
+// take a sample of an event, and every step-th event of a stage.  An entry's place in its
 // list decides ties as in the sequential loop (_core.cpp:338-347: a later equal time
 // takes over), so the maximum over (key, place), taken where its key reaches the event's
 // own, is the loop's result.
@@ -110,7 +147,7 @@ __global__ void __launch_bounds__(kFewDrawThreads) k_few_draw(const KArgs a, con
 // event gained nothing by it).  The copies of two stages ahead have then landed at each
 // barrier, of a ring of three buffers at least.
 template <bool POSITIVE, int G>
-__global__ void __launch_bounds__(G == 1 ? 1024 : 544, 1) k_few(const KArgs a, const FewArgs f) {
+__global__ void __launch_bounds__(G == 1 ? 896 : 544, 1) k_few(const KArgs a, const FewArgs f) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t bars[kFewRing];
     __shared__ int2 head[kFewRing];  // of the stage in a buffer: events, first entry
@@ -119,9 +156,8 @@ __global__ void __launch_bounds__(G == 1 ? 1024 : 544, 1) k_few(const KArgs a, c
     constexpr int ahead = kEarly ? 2 : 1; // stages whose copies have landed at a barrier
     double *win = reinterpret_cast<double *>(smem);
     unsigned char *ring = smem + f.ring_off;
-    const int lane = threadIdx.x & 31, R = f.ring, NS = a.n_stages, ns = 1 << f.ns_log;
-    const int workers = blockDim.x - 32;
-    const bool producer = (int)threadIdx.x == workers;
+    const int lane = threadIdx.x & 31, R = f.ring, NS = a.n_stages, ns = f.ns;
+    const bool producer = threadIdx.x == blockDim.x - 32, worker = (int)threadIdx.x < f.workers;
     const double *entry_dur = f.entry_dur + (int64_t)blockIdx.x * f.cta_entries;
     const int4 *meta = reinterpret_cast<const int4 *>(a.stage_meta);
     constexpr int kVecs = kStageMetaInts / 4;
@@ -132,16 +168,17 @@ __global__ void __launch_bounds__(G == 1 ? 1024 : 544, 1) k_few(const KArgs a, c
         head[b] = make_int2(n_ev, m.z);
         const uint32_t ev_bytes = (uint32_t)n_ev * (uint32_t)sizeof(EvRec);
         const uint32_t pr_bytes = (uint32_t)m.w * (uint32_t)sizeof(PredRec);
-        const uint32_t du_bytes = (((uint32_t)(m.w + 1) & ~1u) << f.ns_log) * (uint32_t)sizeof(double);
+        const uint32_t du_bytes = ((uint32_t)(m.w + 1) & ~1u) * (uint32_t)ns * (uint32_t)sizeof(double);
         unsigned char *buf = ring + b * f.buf_bytes;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         mbar_expect_tx(&bars[b], ev_bytes + pr_bytes + du_bytes);
         bulk_g2s(buf, a.ev + m.x, ev_bytes, &bars[b]);
         if (m.w) bulk_g2s(buf + f.pred_off, a.pred + m.z, pr_bytes, &bars[b]);
-        if (m.w) bulk_g2s(buf + f.dur_off, entry_dur + (few_first(l, m.z) << f.ns_log), du_bytes, &bars[b]);
+        if (m.w) bulk_g2s(buf + f.dur_off, entry_dur + few_first(l, m.z) * ns, du_bytes, &bars[b]);
     };
     // (the workers are a multiple of G * ns: a thread's units are all of one sample)
-    const int j = ((int)threadIdx.x / G) & (ns - 1), s = (blockIdx.x << f.ns_log) + j;
+    const int j = ((int)threadIdx.x / G) % ns, s = blockIdx.x * ns + j;
+    const int first = (int)threadIdx.x / (G * ns), step = f.workers / (G * ns);
     double *wcol = win + j, *rcol = f.realized && s < f.n ? f.realized + s * f.out_col : nullptr;
     int32_t *ccol = f.cause && s < f.n ? f.cause + s * f.out_col : nullptr;
     bool ok = true;
@@ -162,16 +199,16 @@ __global__ void __launch_bounds__(G == 1 ? 1024 : 544, 1) k_few(const KArgs a, c
     int p0 = 0, pe = 0;  // its first entry, and its event's end, in the stage's entries
     const PredRec *pred = nullptr;
     const double *dcol = nullptr;
-    auto fetch = [&](int b, int u) {  // unit u of the stage in buffer b
+    auto fetch = [&](int b, int e) {  // event e of the stage in buffer b
         const unsigned char *buf = ring + b * f.buf_bytes;
         pred = reinterpret_cast<const PredRec *>(buf + f.pred_off);
         dcol = reinterpret_cast<const double *>(buf + f.dur_off) + j;
-        ev = load_ev(reinterpret_cast<const EvRec *>(buf) + ((u / G) >> f.ns_log));
-        p0 = ev.pred_begin - head[b].y + (u & (G - 1));
+        ev = load_ev(reinterpret_cast<const EvRec *>(buf) + e);
+        p0 = ev.pred_begin - head[b].y + (lane & (G - 1));
         pe = ev.pred_end - head[b].y;
         if (kEarly && p0 < pe) {
             src = *reinterpret_cast<const int2 *>(pred + p0);
-            dur = dcol[p0 << f.ns_log];
+            dur = dcol[p0 * ns];
         }
     };
     const unsigned group = ((1u << G) - 1u) << (lane & ~(G - 1));
@@ -183,7 +220,7 @@ __global__ void __launch_bounds__(G == 1 ? 1024 : 544, 1) k_few(const KArgs a, c
         if constexpr (kEarly) {
             for (int p = p0;;) {
                 bool clamp;
-                if (p < pe && relax_time<POSITIVE>(wcol[window_row<1>(src.x) << f.ns_log] + dur, ub_key, ev.ub_bits, key,
+                if (p < pe && relax_time<POSITIVE>(wcol[window_row<1>(src.x) * ns] + dur, ub_key, ev.ub_bits, key,
                                                    bits, clamp)) {
                     place = p;
                     cause = src.y;
@@ -191,7 +228,7 @@ __global__ void __launch_bounds__(G == 1 ? 1024 : 544, 1) k_few(const KArgs a, c
                 p += G;
                 if (p >= pe) break;
                 src = *reinterpret_cast<const int2 *>(pred + p);
-                dur = dcol[p << f.ns_log];
+                dur = dcol[p * ns];
             }
         } else {
             for (int p = p0; p < pe; p += kAhead) {
@@ -201,7 +238,7 @@ __global__ void __launch_bounds__(G == 1 ? 1024 : 544, 1) k_few(const KArgs a, c
                 for (int k = 0; k < kAhead; ++k)
                     if (p + k < pe) {
                         from[k] = *reinterpret_cast<const int2 *>(pred + p + k);
-                        t[k] = wcol[window_row<1>(from[k].x) << f.ns_log] + dcol[(p + k) << f.ns_log];
+                        t[k] = wcol[window_row<1>(from[k].x) * ns] + dcol[(p + k) * ns];
                     }
 #pragma unroll
                 for (int k = 0; k < kAhead; ++k) {
@@ -229,7 +266,7 @@ __global__ void __launch_bounds__(G == 1 ? 1024 : 544, 1) k_few(const KArgs a, c
             }
             const double v = __longlong_as_double(bits);
             const int slot = window_row<1>(ev.slot);
-            if (slot >= 0) wcol[slot << f.ns_log] = v;
+            if (slot >= 0) wcol[slot * ns] = v;
             if (rcol) *at_row(rcol, ev.user, (uint32_t)f.out_row * 8u) = v;
             if (ccol) *at_row(ccol, ev.user, (uint32_t)f.out_row * 4u) = cause;
         }
@@ -237,18 +274,18 @@ __global__ void __launch_bounds__(G == 1 ? 1024 : 544, 1) k_few(const KArgs a, c
     if (!__syncthreads_or(!ok)) {
         int b = 0, b2 = ahead;  // buffers of stages l and l + ahead
         uint32_t phase2 = 0;    // phase of the latter
-        if (kEarly && (int)threadIdx.x < workers && (int)threadIdx.x < (head[0].x * G) << f.ns_log) fetch(0, threadIdx.x);
+        if (kEarly && worker && first < head[0].x) fetch(0, first);
         for (int l = 0; l < NS; ++l) {
             const int nb = b + 1 == R ? 0 : b + 1;
-            if ((int)threadIdx.x < workers) {
-                const int units = (head[b].x * G) << f.ns_log;
-                if (kEarly && (int)threadIdx.x < units) run();
-                for (int u = threadIdx.x + (kEarly ? workers : 0); u < units; u += workers) {
-                    fetch(b, u);
+            if (worker) {
+                const int n_ev = head[b].x;
+                if (kEarly && first < n_ev) run();
+                for (int e = first + (kEarly ? step : 0); e < n_ev; e += step) {
+                    fetch(b, e);
                     run();
                 }
                 // the next stage's first unit: its records have landed, and off its chain
-                if (kEarly && l + 1 < NS && (int)threadIdx.x < (head[nb].x * G) << f.ns_log) fetch(nb, threadIdx.x);
+                if (kEarly && l + 1 < NS && first < head[nb].x) fetch(nb, first);
             }
             if (producer && l + ahead < NS) {
                 waits = l + ahead;
@@ -280,33 +317,34 @@ int sm_count();
 // too large for rows of 32 samples is no obstacle: 50,000 events in levels of 200 x 152
 // samples 3,690 -> 645 us.)  With `work` the stages plus a 64th of the events: samples
 // drawn, general and few,
-//   100 events in 2 stages (work 4)   8.3 and 12.7 us: the second launch is not repaid
-//   203 in 11 (14)    x 152 24.7, 20.5   x 608 24.7, 20.7   x 2,432 24.7, 27.8
-//   600 in 20 (29)    x 152 59, 27       x 608 59, 33       x 2,432 59, 58
-//   20,017 in 493 (805) x 1,216 1,758, 833   x 2,432 1,760, 1,366   x 3,001 1,758, 1,857
+//   100 events in 2 stages (work 4)    8.3 and 12.7 us: the second launch is not repaid
+//   150 in 7 (10)        x 40 18.6, 17.0    x 608 18.6, 20.6
+//   203 in 11 (14)       x 152 24.7, 20.5   x 608 24.7, 22.6   x 2,432 24.7, 26.1
+//   2,000 in 34 (65)     x 608 122, 51      x 2,432 123, 111   x 3,001 123, 130
+//   20,017 in 493 (805)  x 608 1,755, 560   x 2,432 1,757, 1,196   x 3,001 1,758, 1,506
+//   2,000 in 45 (76)     x 3,040 135, 141: stages of some 42 events divide the last two
 // and durations given, whose general kernel has less to do a stage,
-//   203  x 152 20.6, 19.9   x 608 20.6, 23.1;  600  x 608 45, 38   x 1,216 45, 43
-//   20,017  x 1,216 1,427, 867   x 2,432 1,432, 1,475
+//   203  x 608 20.6, 23.1;  600 in 20 (29)  x 608 45, 31   x 1,824 45, 39   x 2,432 45, 46
+//   20,017  x 1,216 1,424, 769   x 1,824 1,426, 1,017;  50,000 in 833  x 2,432 2,889, 2,929
 // direct: the rows go straight to the host, which saves more launches than this adds.
 bool few_layout(const KArgs &a, int64_t n, bool direct, FewArgs &f) {
     const int sms = sm_count();
     if (n < 1 || !a.rows_planned || a.avg_units <= 0 || a.n_stages <= 0 || sms <= 0) return false;
     const int64_t work = a.n_stages + a.n_events / 64;
     if (!direct && work < (a.dur_in ? 24 : 8)) return false;
-    const int most = work < 32 ? 2 : a.dur_in ? 3 : 4;
-    f.ns_log = 0;
-    while (f.ns_log <= most && ((int64_t)sms << f.ns_log) < n) ++f.ns_log;
-    if (f.ns_log > most) return false;
+    const int most = a.dur_in ? 12 : work < 12 ? 1 : work < 24 ? 4 : a.n_events <= 42 * (int64_t)a.n_stages ? 20 : 16;
+    if (n > (int64_t)most * sms) return false;
     f.n = (int32_t)n;
-    f.ctas = (int32_t)((n + (1 << f.ns_log) - 1) >> f.ns_log);
-    f.cta_entries = ((int64_t)a.n_entries + a.n_stages + 2) / 2 * 2 << f.ns_log;
+    f.ns = (int32_t)((n + sms - 1) / sms);
+    f.ctas = (int32_t)((n + f.ns - 1) / f.ns);
+    f.cta_entries = ((int64_t)a.n_entries + a.n_stages + 2) / 2 * 2 * f.ns;
     f.scratch = (size_t)f.ctas * (size_t)f.cta_entries * sizeof(double);
     if (f.scratch > kFewScratch) return false;
-    const size_t win = (((size_t)a.window_slots << f.ns_log) * sizeof(double) + 127) / 128 * 128;
+    const size_t win = ((size_t)a.window_slots * f.ns * sizeof(double) + 127) / 128 * 128;
     const size_t ev = (size_t)a.stage_events * sizeof(EvRec), pred = (size_t)a.stage_entries * sizeof(PredRec);
-    const size_t dur = ((size_t)(a.stage_entries + 1) / 2 * 2 << f.ns_log) * sizeof(double);
+    const size_t dur = (size_t)(a.stage_entries + 1) / 2 * 2 * f.ns * sizeof(double);
     const size_t buf = (ev + pred + dur + 127) / 128 * 128;
-    const int64_t units = (int64_t)a.stage_events << f.ns_log;
+    const int64_t units = (int64_t)a.stage_events * f.ns;
     // Lanes over an event's entries shorten its chain while the stage's warps are few; past
     // some 16 warps their reductions cost more issue than they save (50,000 events in stages
     // of up to 128: one sample a CTA 1 lane 681 us, 4 lanes 594; 20,017 in stages of 37,
@@ -319,19 +357,25 @@ bool few_layout(const KArgs &a, int64_t n, bool direct, FewArgs &f) {
     f.buf_bytes = (int32_t)buf;
     f.ring = (int32_t)((kFewSmem - win) / buf < (size_t)kFewRing ? (kFewSmem - win) / buf : kFewRing);
     f.smem = (int32_t)(win + f.ring * buf);
-    f.threads = (int32_t)(units * f.lanes >= 960 ? 960 : (units * f.lanes + 63) / 64 * 64) + 32;  // (64: lanes << ns_log at most)
+    const int unit = f.lanes * f.ns;  // threads an event
+    const int64_t all = (int64_t)a.stage_events * unit;
+    f.workers = (int32_t)(all < 864 ? all : 864 / unit * unit);
+    f.threads = (f.workers + 31) / 32 * 32 + 32;
     return true;
 }
 
 cudaError_t launch_few(const KArgs &a, const FewArgs &f, cudaStream_t st) {
     // CTAs along y: a warp for each item of the largest stage, up to 64 CTAs an SM in all
     const int64_t lanes = f.n >= 32 ? 32 : f.n, run = f.n >= 32 ? kFewDrawRun : 1;
-    const int64_t items = ((int64_t)a.stage_entries * lanes + 32 * run - 1) / (32 * run) * ((f.n + 31) / 32);
+    const int per_lane = f.n <= 64 ? 1 : f.n <= 1024 || f.dur_in ? 2 : 4;  // samples a lane
+    const int64_t items = ((int64_t)a.stage_entries * lanes + 32 * run - 1) / (32 * run) * ((f.n + 32 * per_lane - 1) / (32 * per_lane));
     const int64_t per = (items + kFewDrawThreads / 32 - 1) / (kFewDrawThreads / 32);
     const int64_t most = (int64_t)64 * sm_count() / a.n_stages + 1;
     const unsigned gy = (unsigned)(per < 1 ? 1 : per < most ? per : most);
     const int64_t aux = f.durations && a.n_aux > 0 ? ((int64_t)a.n_aux * f.n + 128 * run * gy - 1) / (128 * run * gy) : 0;
-    void (*draw)(const KArgs, const FewArgs) = f.dur_in ? k_few_draw<true> : k_few_draw<false>;
+    void (*draw)(const KArgs, const FewArgs) = 
+        f.dur_in ? per_lane == 1 ? k_few_draw<true, 1> : k_few_draw<true, 2>
+                 : per_lane == 1 ? k_few_draw<false, 1> : per_lane == 2 ? k_few_draw<false, 2> : k_few_draw<false, 4>;
     draw<<<dim3((unsigned)(a.n_stages + (aux < 64 ? aux : 64)), gy), kFewDrawThreads, 0, st>>>(a, f);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;

@@ -289,7 +289,7 @@ constexpr size_t kFewScratch = (size_t)8 << 30;  // most scratch of a launch, an
 struct FewArgs {
     int64_t seed[kFewInline];
     const int64_t *seeds;          // [n] on the device, or null: seed
-    int32_t n, ns_log;             // samples; log2 of a CTA's
+    int32_t n, ns;                 // samples, and those of a CTA
     int64_t out_row, out_col, dur_row, dur_col;
     const double *dur_in;          // given durations, or null: drawn
     double *realized, *durations;  // each may be null
@@ -300,7 +300,7 @@ struct FewArgs {
     // shared memory of the propagation: window, then `ring` buffers of a stage's event
     // and predecessor records and durations
     int32_t ring_off, ring, buf_bytes, pred_off, dur_off, smem;
-    int32_t ctas, threads, lanes;
+    int32_t ctas, threads, workers, lanes;
 };
 
 // Arguments of the persistent batch kernel.

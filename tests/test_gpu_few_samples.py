@@ -24,7 +24,7 @@ def _bits(a):
 @pytest.mark.parametrize("layers,width,preds,shift,big", [(6, 150, 12, 0.0, False), (40, 7, 4, -500.0, False),
                                                           (1, 3, 1, 0.0, False), (5, 900, 4, 0.0, True),
                                                           (9, 1100, 4, 0.0, False)])
-@pytest.mark.parametrize("n", [1, 3, 8, 9, 153, 1217, 2433])
+@pytest.mark.parametrize("n", [1, 3, 8, 9, 153, 800, 1217, 3040, 3041])
 def test_rows_equal_the_general_kernels_and_the_oracle(cuda, layers, width, preds, shift, big, n):
     flat, gen = kitchen_sink(seed=6, n_layers=layers, width=width, big_table=big, max_preds=preds)
     flat = dict(flat, earliest=flat["earliest"] + shift)
