@@ -87,6 +87,32 @@ int mcd_batch_create(mcd_dag *const *dags, int32_t n_dags, const int64_t *seed0,
         }
         cuda_check(cudaSetDevice(B->device), "cudaSetDevice");
         cuda_check(cudaStreamCreateWithFlags(&B->stream, cudaStreamNonBlocking), "stream create");
+        int sms = 0;
+        cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, B->device), "SM count");
+        auto cost = [&](int32_t i) { return (double)B->dags[i]->h.pred.size() + 2.0 * B->dags[i]->h.E; };
+        // Wide tiles pay where an SM has the work of several of the costliest tiles (a wide
+        // one takes 1.77 times as long, and the last of them set the end): three where a
+        // narrow CTA has its SM to itself; nine where several hide each other's barriers,
+        // and then only if many entries draw nothing, their cost being the records that
+        // two samples share.  Measured (tiles of work an SM: narrow, wide): one
+        // CTA an SM, 9.7: 29.2, 24.2 ms; several, half the entries fixed, 18: 20.9, 19.1;
+        // a fifth of them fixed, 15: 9.7, 11.1; 32 networks of two delay types 45.8, 39.6,
+        // of five 94.7, 94.9, by this rule 89.2.
+        double work = 0.0, most = 0.0, entries = 0.0, sampled = 0.0;
+        size_t narrow_smem = 0;
+        for (int32_t i = 0; i < n_dags; ++i) {
+            const HostDag &h = B->dags[i]->h;
+            const double tiles = (double)((B->n[i] + kTile - 1) / kTile);
+            work += cost(i) * tiles;
+            most = std::max(most, cost(i));
+            entries += (double)h.pred.size() * tiles;
+            sampled += (double)h.sampled_entries * tiles;
+            if (h.win_smem) narrow_smem = std::max(narrow_smem, (size_t)h.smem_total);
+        }
+        const int64_t narrow_fit = std::min<int64_t>((228 * 1024) / ((int64_t)narrow_smem + 1024),
+                                                     kMaxBatchWarps / std::max(1, B->n_warps));
+        const double tiles_deep = work / (std::max(most, 1.0) * std::max(1, sms));
+        const bool wide_pays = narrow_fit <= 1 ? tiles_deep >= 3.0 : tiles_deep >= 9.0 && sampled < 0.65 * entries;
         // layout of the batch's device memory; launches by kernel variant
         B->ev_off.resize((size_t)n_dags + 1, 0);
         std::vector<int32_t> launch_of((size_t)n_dags);
@@ -95,7 +121,7 @@ int mcd_batch_create(mcd_dag *const *dags, int32_t n_dags, const int64_t *seed0,
             B->max_E = std::max(B->max_E, h.E);
             B->ev_off[i + 1] = B->ev_off[i] + h.E;
             // (more than one narrow tile of samples fills a wide one)
-            const bool wide = h.wide_rows > 0 && B->n[i] > kTile;
+            const bool wide = wide_pays && h.wide_rows > 0 && B->n[i] > kTile;
             Launch *L = nullptr;
             for (Launch &x : B->launches)
                 if (x.win_smem == h.win_smem && x.positive == h.positive && x.tsmem == h.tables_in_smem && x.wide == wide)
@@ -116,10 +142,7 @@ int mcd_batch_create(mcd_dag *const *dags, int32_t n_dags, const int64_t *seed0,
             B->n_items += (B->n[i] + kTile - 1) / kTile;
         }
         B->total_E = B->ev_off[n_dags];
-        int sms = 0;
-        cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, B->device), "SM count");
         // items: within each launch, DAGs by cost per tile, most expensive first; every tile of a DAG
-        auto cost = [&](int32_t i) { return (double)B->dags[i]->h.pred.size() + 2.0 * B->dags[i]->h.E; };
         std::vector<int32_t> items;
         std::vector<size_t> item_off;  // first item of each launch
         int64_t scratch_all = 0;  // doubles; launches run one after another

@@ -1148,8 +1148,12 @@ void compile_dag(const mcd_dag_desc &d, const mcd_generator &g, HostDag &H, int3
     }
     if (H.max_units > 0) H.avg_units = std::max<int32_t>(1, (H.E - H.n_pairs) / H.n_stages);
     H.block_draws = 0;
+    H.sampled_entries = 0;
     for (const PredRec &p : H.pred)
-        if ((p.kd & KD_KIND_MASK) != K_FIXED && !(p.kd & KD_REUSE)) ++H.block_draws;
+        if ((p.kd & KD_KIND_MASK) != K_FIXED) {
+            ++H.sampled_entries;
+            if (!(p.kd & KD_REUSE)) ++H.block_draws;
+        }
 }
 
 // The links by Philox block, for a kernel that draws durations without propagating:

@@ -65,6 +65,7 @@ struct HostDag {
     int64_t max_preds = 0;        // largest predecessor list
     bool tables_in_smem = true;
     int32_t max_units = 0, avg_units = 0;  // most and mean work units of a stage (0: warps per CTA fixed by the caller)
+    int64_t sampled_entries = 0;  // precedence entries whose link draws
     int32_t stage_events = 0, stage_entries = 0;  // most events and precedence entries of a stage
     int32_t n_stages = 0, stage_bytes = 0;
     int32_t smem_stage_off = 0, smem_tables_off = 0, smem_bar_off = 0, smem_total = 0;
