@@ -899,7 +899,7 @@ def main():
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
                          "algorithmic_bytes_per_launch": alg_bytes,
-                         "kernel": "k_propagate<GIVEN=0, WIN_SMEM=1, STATS=0, POSITIVE=1, TS=smem> (fused Philox sampler + FP64 "
+                         "kernel": "k_propagate<WIN_SMEM=1, STATS=0, POSITIVE=1, TS=smem, S=2> (fused Philox sampler + FP64 "
                                    "propagation)",
                          "kernel_ms": float(np.mean(kernel_ms))},
             "cpu_baseline": cpu, "e2e": e2e, "e2e_dropin": e2e_dropin, "gpu_launches": args.steps, "clocks": ck,

@@ -1,13 +1,12 @@
 // mcd_batch.cpp -- many DAGs, each with its own samples, in one persistent launch.
 //
-// The work is a queue of (DAG, tile of 32 samples, or 64 where the DAG has wide
-// tiles) items, most expensive DAG first
-// (longest-processing-time order), consumed by a persistent grid of CTAs that
+// The work is a queue of (DAG, tile of 32 samples, or 64 where wide tiles pay) items,
+// most expensive DAG first (longest-processing-time order), consumed by a persistent grid of CTAs that
 // fills every SM whatever the DAGs' sizes -- a plain per-DAG launch of a DAG
 // with 1,000 samples keeps 32 CTAs busy and leaves the rest of the GPU idle.
 // DAGs are grouped by kernel variant (window on chip or not, tables in shared
-// memory or not, positive times or not, wide tiles or not); each group is one launch with its own
-// queue.  Each run is one CUDA
+// memory or not, positive times or not, wide tiles or not); each group is one launch
+// with its own queue.  Each run is one CUDA
 // graph: reset the accumulators and the queue heads, the persistent statistics
 // launches, the batched finish.  The graph is recorded on the first run and
 // replayed afterwards.

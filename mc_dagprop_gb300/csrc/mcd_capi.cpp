@@ -519,7 +519,8 @@ bool run_few(mcd_dag *g, const int64_t *seeds, const double *dur_in, int64_t n, 
     if (dur_in) {
         f.dur_in = in_dv ? in_dv : du_major;
         if (!in_dv && L > 0)
-            cuda_check(cudaMemcpyAsync(du_major, dur_in, (size_t)(n * L) * 8, cudaMemcpyHostToDevice, st), "durations upload");
+            cuda_check(cudaMemcpyAsync(du_major, dur_in, (size_t)(n * L) * 8, cudaMemcpyHostToDevice, st),
+                       "durations upload");
     } else if (n <= kFewInline) {
         std::copy(seeds, seeds + n, f.seed);
     } else {

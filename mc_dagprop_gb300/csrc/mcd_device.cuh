@@ -1,8 +1,8 @@
 // mcd_device.cuh -- device code of the Monte Carlo DAG-propagation path (sm_103a).
 //
 // k_propagate: one CTA owns a tile of 32 samples (one per lane), or a wide tile of
-// 64 (two per lane; use_wide), and walks the whole compiled DAG stage by stage (a stage is a level, or a slice of a wide
-// level); the warps of the CTA split each stage's events and meet at a barrier
+// 64 (two per lane; use_wide), and walks the whole compiled DAG stage by stage (a
+// stage is a level, or a slice of a wide level); the warps of the CTA split each stage's events and meet at a barrier
 // between stages.  The records of the next stage are copied into shared memory
 // by the TMA bulk-copy engine (cp.async.bulk + mbarrier, double-buffered) while
 // the current one is processed, so no warp waits on L2 for DAG records.

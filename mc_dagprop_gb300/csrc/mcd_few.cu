@@ -31,7 +31,7 @@ __device__ __forceinline__ int64_t few_first(int stage, int first_entry) {
 // where n fills the lanes (one otherwise: latency), drawing a Philox block once for the
 // entries that share it.  The last CTAs draw the links no entry references.  The draws are
 // the sampled propagation's own (same records, blocks, words and arithmetic): equal bits.
-// Bound by instructions (148 per 32 draws at one sample a lane, 60 % issue active).  Both
+// Bound by instructions (per 32 draws 148 at one sample a lane, 109 at four).  Both
 // kernels, 20,017 events: x 1,216 832 us with one sample a lane, 750 with two, 742 with
 // four; x 2,432 1,388, 1,256, 1,197; x 152 412, 411, 419.
 constexpr int kFewDrawRun = 4;
@@ -43,7 +43,8 @@ __global__ void __launch_bounds__(kFewDrawThreads) k_few_draw(const KArgs a, con
     const AliasPick *picks = reinterpret_cast<const AliasPick *>(alias + a.n_alias);
     const int lanes_log = n > 16 ? 5 : n > 8 ? 4 : n > 4 ? 3 : n > 2 ? 2 : n > 1 ? 1 : 0;  // of a lane's samples
     const int run = n >= 32 ? kFewDrawRun : 1;
-    const int blocks = (n + 32 * S - 1) / (32 * S), per_warp = run << (5 - lanes_log);  // sample blocks; entries a warp takes
+    const int blocks = (n + 32 * S - 1) / (32 * S);  // of samples
+    const int per_warp = run << (5 - lanes_log);     // entries a warp takes
     U4 words[S];
     uint32_t drawn = 0xFFFFFFFFu;  // the block `words` are of (no block has this number)
     uint64_t seed[S];
@@ -79,13 +80,14 @@ __global__ void __launch_bounds__(kFewDrawThreads) k_few_draw(const KArgs a, con
         }
     };
     const bool aux = stage >= a.n_stages;
-    const int4 meta = aux ? make_int4(0, 0, 0, a.n_aux) : __ldg(reinterpret_cast<const int4 *>(a.stage_meta + kStageMetaInts * stage));
-    const int4 mv = aux ? meta : __ldg(reinterpret_cast<const int4 *>(a.stage_meta + kStageMetaInts * stage) + 1);
+    const int4 *sm = reinterpret_cast<const int4 *>(a.stage_meta + kStageMetaInts * stage);
+    const int4 meta = aux ? make_int4(0, 0, 0, a.n_aux) : __ldg(sm), mv = aux ? meta : __ldg(sm + 1);
     double *out = aux ? nullptr : f.entry_dur + few_first(stage, meta.z) * ns;
     const int cta = blockIdx.y + (aux ? (stage - a.n_stages) * gridDim.y : 0);
     const int ctas = aux ? (gridDim.x - a.n_stages) * gridDim.y : gridDim.y;
     const int items = (meta.w + per_warp - 1) / per_warp * blocks;
-    for (int item = cta * (kFewDrawThreads / 32) + (threadIdx.x >> 5); item < items; item += ctas * (kFewDrawThreads / 32)) {
+    constexpr int kWarps = kFewDrawThreads / 32;
+    for (int item = cta * kWarps + (threadIdx.x >> 5); item < items; item += ctas * kWarps) {
         const int g = item / blocks;
         const int s = (item - g * blocks) * (32 * S) + (lane & ((1 << lanes_log) - 1));
         if (s >= n) continue;
@@ -115,7 +117,8 @@ __global__ void __launch_bounds__(kFewDrawThreads) k_few_draw(const KArgs a, con
             const int4 r0 = __ldg(q);  // src_slot, src_user, link, kd
             if (GIVEN) {
 #pragma unroll
-                for (int j = 0; j < S; ++j) dur[j] = r0.z >= 0 && in[j] ? __ldg(f.dur_in + (int64_t)r0.z * f.dur_row + col[j]) : 0.0;
+                for (int j = 0; j < S; ++j)
+                    dur[j] = r0.z >= 0 && in[j] ? __ldg(f.dur_in + (int64_t)r0.z * f.dur_row + col[j]) : 0.0;
             } else {
                 const int4 r1 = __ldg(q + 1);  // v, dvo, block
                 const double *vt = nullptr;
@@ -368,12 +371,14 @@ cudaError_t launch_few(const KArgs &a, const FewArgs &f, cudaStream_t st) {
     // CTAs along y: a warp for each item of the largest stage, up to 64 CTAs an SM in all
     const int64_t lanes = f.n >= 32 ? 32 : f.n, run = f.n >= 32 ? kFewDrawRun : 1;
     const int per_lane = f.n <= 64 ? 1 : f.n <= 1024 || f.dur_in ? 2 : 4;  // samples a lane
-    const int64_t items = ((int64_t)a.stage_entries * lanes + 32 * run - 1) / (32 * run) * ((f.n + 32 * per_lane - 1) / (32 * per_lane));
+    const int64_t blocks = (f.n + 32 * per_lane - 1) / (32 * per_lane);
+    const int64_t items = ((int64_t)a.stage_entries * lanes + 32 * run - 1) / (32 * run) * blocks;
     const int64_t per = (items + kFewDrawThreads / 32 - 1) / (kFewDrawThreads / 32);
     const int64_t most = (int64_t)64 * sm_count() / a.n_stages + 1;
     const unsigned gy = (unsigned)(per < 1 ? 1 : per < most ? per : most);
-    const int64_t aux = f.durations && a.n_aux > 0 ? ((int64_t)a.n_aux * f.n + 128 * run * gy - 1) / (128 * run * gy) : 0;
-    void (*draw)(const KArgs, const FewArgs) = 
+    const int64_t per_cta = kFewDrawThreads * run * gy;
+    const int64_t aux = f.durations && a.n_aux > 0 ? ((int64_t)a.n_aux * f.n + per_cta - 1) / per_cta : 0;
+    void (*draw)(const KArgs, const FewArgs) =
         f.dur_in ? per_lane == 1 ? k_few_draw<true, 1> : k_few_draw<true, 2>
                  : per_lane == 1 ? k_few_draw<false, 1> : per_lane == 2 ? k_few_draw<false, 2> : k_few_draw<false, 4>;
     draw<<<dim3((unsigned)(a.n_stages + (aux < 64 ? aux : 64)), gy), kFewDrawThreads, 0, st>>>(a, f);
