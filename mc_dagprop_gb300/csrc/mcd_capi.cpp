@@ -20,7 +20,7 @@
 
 namespace mcd {
 cudaError_t launch_propagate(const KArgs &a, bool given, bool win_smem, bool stats, cudaStream_t st);
-bool few_layout(const KArgs &a, int64_t n, bool direct, FewArgs &f);
+bool few_layout(const KArgs &a, int64_t n, bool given, bool direct, FewArgs &f);
 cudaError_t launch_few(const KArgs &a, const FewArgs &f, cudaStream_t st);
 cudaError_t launch_stats_finish(const FArgs &f, cudaStream_t st);
 cudaError_t launch_event_ticks(const double *earliest, int32_t E, int32_t q, long long *te, cudaStream_t st);
@@ -460,19 +460,20 @@ void move_rows(const T *minor, int64_t C, T *dv, T *host, T *major, int64_t rows
 }
 
 // Few samples through host buffers (mcd_few.cu); false where that path does not apply.
-// seeds, or dur_in: what the samples are.  Few rows (kFewInline, kFewDirect) are written
-// sample-major, straight into pinned memory (or to the device and copied), which saves
-// the seeds' copy and the transposes; others are transposed (move_rows): their scattered
-// 8-byte writes cost more over the host link (1,000 events x 1 68 against 80 us, x 20 80
-// and 85, x 32 93 and 89; 10,000 x 4 138 and 143, x 8 159 and 151).
+// seeds, or (null) given durations, which a DAG without links may leave out.  Few rows
+// (kFewInline, kFewDirect) are written sample-major, straight into pinned memory (or to
+// the device and copied), which saves the seeds' copy and the transposes; others are
+// transposed (move_rows): their scattered 8-byte writes cost more over the host link
+// (1,000 events x 1 68 against 80 us, x 20 80 and 85, x 32 93 and 89; 10,000 x 4 138 and
+// 143, x 8 159 and 151).
 bool run_few(mcd_dag *g, const int64_t *seeds, const double *dur_in, int64_t n, double *realized, double *durations,
              int32_t *cause) {
     const int64_t E = g->h.E, L = g->h.L;
     KArgs a = base_args(g);
     FewArgs f{};
-    a.dur_in = dur_in;  // (which rule applies)
+    const bool given = !seeds;
     const bool direct = n <= kFewInline && n * E <= kFewDirect;
-    if (!few_layout(a, n, direct, f)) return false;
+    if (!few_layout(a, n, given, direct, f)) return false;
     double *real_dv = device_view(realized), *dur_dv = device_view(durations);
     const double *in_dv = device_view(dur_in);
     int32_t *cause_dv = device_view(cause);
@@ -513,14 +514,16 @@ bool run_few(mcd_dag *g, const int64_t *seeds, const double *dur_in, int64_t n, 
     f.cause = !cause ? nullptr : !direct ? ca : cause_dv ? cause_dv : ca_major;
     f.out_row = direct ? 1 : n;
     f.out_col = direct ? E : 1;
-    f.dur_row = direct || dur_in ? 1 : n;
-    f.dur_col = direct || dur_in ? L : 1;
+    f.dur_row = direct ? 1 : n;
+    f.dur_col = direct ? L : 1;
     cudaStream_t st = g->stream[0];
-    if (dur_in) {
-        f.dur_in = in_dv ? in_dv : du_major;
-        if (!in_dv && L > 0)
+    if (given) {
+        const double *in = in_dv ? in_dv : du_major;
+        if (dur_in && !in_dv && L > 0)
             cuda_check(cudaMemcpyAsync(du_major, dur_in, (size_t)(n * L) * 8, cudaMemcpyHostToDevice, st),
                        "durations upload");
+        if (!direct && L > 0) cuda_check(launch_transpose_f64(in, L, du, n, n, L, st), "transpose");
+        f.dur_in = direct ? in : du;
     } else if (n <= kFewInline) {
         std::copy(seeds, seeds + n, f.seed);
     } else {
@@ -590,9 +593,9 @@ void few_pool_leave(mcd_dag *g) {
 // scratch is taken in the stream's order, so that calls on several streams and threads
 // share nothing; a stream that is being captured, and a launch whose scratch cannot be
 // had, keep the general kernels.
-bool run_few_device(mcd_dag *g, const KArgs &a, cudaStream_t st) {
+bool run_few_device(mcd_dag *g, const KArgs &a, bool given, cudaStream_t st) {
     FewArgs f{};
-    if (!few_layout(a, a.n, false, f)) return false;
+    if (!few_layout(a, a.n, given, false, f)) return false;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) {
         (void)cudaGetLastError();
@@ -612,7 +615,7 @@ bool run_few_device(mcd_dag *g, const KArgs &a, cudaStream_t st) {
     f.durations = a.durations;
     f.dur_in = a.dur_in;
     f.out_row = a.ld;
-    f.dur_row = a.dur_in ? a.ld_in : a.ld;
+    f.dur_row = given ? a.ld_in : a.ld;
     f.out_col = f.dur_col = 1;
     const cudaError_t e = launch_few(a, f, st);
     cudaFreeAsync(p, st);
@@ -857,7 +860,7 @@ int mcd_run_device(mcd_dag *g, const int64_t *seeds, int64_t n, double *realized
             ensure_ws(g, (size_t)g->h.E * (size_t)ld * 8);
             a.scratch = (double *)g->ws;
         }
-        if (run_few_device(g, a, st)) return;
+        if (run_few_device(g, a, false, st)) return;
         cuda_check(launch_propagate(a, false, g->h.win_smem, false, st), "propagate launch");
     });
 }
@@ -882,7 +885,7 @@ int mcd_propagate_device(mcd_dag *g, const double *dur, int64_t ld_in, int64_t n
             ensure_ws(g, (size_t)g->h.E * (size_t)ld * 8);
             a.scratch = (double *)g->ws;
         }
-        if (run_few_device(g, a, st)) return;
+        if (run_few_device(g, a, true, st)) return;
         cuda_check(launch_propagate(a, true, g->h.win_smem, false, st), "propagate launch");
     });
 }

@@ -330,13 +330,14 @@ int sm_count();
 //   203  x 608 20.6, 23.1;  600 in 20 (29)  x 608 45, 31   x 1,824 45, 39   x 2,432 45, 46
 //   20,017  x 1,216 1,424, 769   x 1,824 1,426, 1,017;  50,000 in 833  x 2,432 2,889, 2,929
 // direct: the rows go straight to the host, which saves more launches than this adds.
-bool few_layout(const KArgs &a, int64_t n, bool direct, FewArgs &f) {
+bool few_layout(const KArgs &a, int64_t n, bool given, bool direct, FewArgs &f) {
     const int sms = sm_count();
     if (n < 1 || !a.rows_planned || a.avg_units <= 0 || a.n_stages <= 0 || sms <= 0) return false;
     const int64_t work = a.n_stages + a.n_events / 64;
-    if (!direct && work < (a.dur_in ? 24 : 8)) return false;
-    const int most = a.dur_in ? 12 : work < 12 ? 1 : work < 24 ? 4 : a.n_events <= 42 * (int64_t)a.n_stages ? 20 : 16;
+    if (!direct && work < (given ? 24 : 8)) return false;
+    const int most = given ? 12 : work < 12 ? 1 : work < 24 ? 4 : a.n_events <= 42 * (int64_t)a.n_stages ? 20 : 16;
     if (n > (int64_t)most * sms) return false;
+    f.given = given;
     f.n = (int32_t)n;
     f.ns = (int32_t)((n + sms - 1) / sms);
     f.ctas = (int32_t)((n + f.ns - 1) / f.ns);
@@ -370,7 +371,7 @@ bool few_layout(const KArgs &a, int64_t n, bool direct, FewArgs &f) {
 cudaError_t launch_few(const KArgs &a, const FewArgs &f, cudaStream_t st) {
     // CTAs along y: a warp for each item of the largest stage, up to 64 CTAs an SM in all
     const int64_t lanes = f.n >= 32 ? 32 : f.n, run = f.n >= 32 ? kFewDrawRun : 1;
-    const int per_lane = f.n <= 64 ? 1 : f.n <= 1024 || f.dur_in ? 2 : 4;  // samples a lane
+    const int per_lane = f.n <= 64 ? 1 : f.n <= 1024 || f.given ? 2 : 4;  // samples a lane
     const int64_t blocks = (f.n + 32 * per_lane - 1) / (32 * per_lane);
     const int64_t items = ((int64_t)a.stage_entries * lanes + 32 * run - 1) / (32 * run) * blocks;
     const int64_t per = (items + kFewDrawThreads / 32 - 1) / (kFewDrawThreads / 32);
@@ -379,12 +380,12 @@ cudaError_t launch_few(const KArgs &a, const FewArgs &f, cudaStream_t st) {
     const int64_t per_cta = kFewDrawThreads * run * gy;
     const int64_t aux = f.durations && a.n_aux > 0 ? ((int64_t)a.n_aux * f.n + per_cta - 1) / per_cta : 0;
     void (*draw)(const KArgs, const FewArgs) =
-        f.dur_in ? per_lane == 1 ? k_few_draw<true, 1> : k_few_draw<true, 2>
+        f.given ? per_lane == 1 ? k_few_draw<true, 1> : k_few_draw<true, 2>
                  : per_lane == 1 ? k_few_draw<false, 1> : per_lane == 2 ? k_few_draw<false, 2> : k_few_draw<false, 4>;
     draw<<<dim3((unsigned)(a.n_stages + (aux < 64 ? aux : 64)), gy), kFewDrawThreads, 0, st>>>(a, f);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    const bool pos = a.positive && !f.dur_in;
+    const bool pos = a.positive && !f.given;
     void (*fn)(const KArgs, const FewArgs) =
         f.lanes == 4 ? pos ? k_few<true, 4> : k_few<false, 4> : pos ? k_few<true, 1> : k_few<false, 1>;
     e = raise_smem_limit((const void *)fn, (size_t)f.smem);

@@ -291,7 +291,8 @@ struct FewArgs {
     const int64_t *seeds;          // [n] on the device, or null: seed
     int32_t n, ns;                 // samples, and those of a CTA
     int64_t out_row, out_col, dur_row, dur_col;
-    const double *dur_in;          // given durations, or null: drawn
+    int32_t given;                 // durations: given in dur_in (null without links), else drawn
+    const double *dur_in;
     double *realized, *durations;  // each may be null
     int32_t *cause;                // may be null
     double *entry_dur;             // scratch [ctas * cta_entries]: a CTA's durations in entry order

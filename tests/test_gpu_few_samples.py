@@ -95,3 +95,18 @@ def test_device_buffers_streams_and_capture(cuda, n):
         assert torch.equal(again[k][0], want[k][0]) and torch.equal(again[k][2], want[k][2])
     for a, b in zip(graphed, want[0]):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("n", [1, 40])
+def test_a_dag_without_links_may_leave_the_durations_out(cuda, n):
+    E = 700
+    flat = dict(earliest=np.arange(E, dtype=np.float64), act_idx=np.zeros(0, np.int32), act_duration=np.zeros(0),
+                act_type=np.zeros(0, np.int32), target=np.arange(1, E, dtype=np.int32),
+                pred_offsets=np.arange(E, dtype=np.int64), pred_src=np.arange(E - 1, dtype=np.int32),
+                pred_act=np.zeros(E - 1, np.int32), max_delay=1000.0)  # a chain over links past the last
+    prop = batching.compile_dag(flat, [], 0, "auto")
+    real, cause = np.empty((n, E)), np.empty((n, E), np.int32)
+    assert lib().mcd_propagate_host(C.c_void_p(prop._handle()), None, n, real.ctypes.data, cause.ctypes.data) == 0
+    assert np.array_equal(real, np.tile(flat["earliest"], (n, 1)))
+    # a later event's own time exceeds its predecessor's: no cause
+    assert (cause == -1).all()
