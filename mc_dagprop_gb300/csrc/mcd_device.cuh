@@ -591,13 +591,20 @@ __device__ __forceinline__ bool relax(double src, double dur, long long ub_key, 
 
 // One stage's events under given durations, one at a time from the stage's counter
 // (no draws, so no pairs).  The durations are uncached DRAM reads: an event's first
-// kGivenAhead entries are read while the event before it runs, later ones when
-// reached.  Without the sampler the kernel fits 64 registers, so 32 warps an SM.
+// kGivenAhead entries are read while the event before it runs.  Without the sampler the
+// kernel runs at 64 registers (those of wide tiles spill 64 bytes), so 32 warps an SM.
 // 200,000 events x 4,864 samples: reads four at a time when reached, 24 warps 13.2 ms
 // (2.3 TB/s); one event ahead, 32 warps 9.6 (3.2 TB/s).  20,017 events x 3,001
-// samples 3.5 -> 1.45 ms.  Prefetching the next stage's rows into L2 gained 2 %.
+// samples 3.5 -> 1.30 ms.  Prefetching the next stage's rows into L2 gained 2 %.
+// LONG: events of many predecessors, whose later entries are read kGivenAhead together
+// (one by one, each waits for DRAM: 4,000 events of 12.5 predecessors x 4,864 samples at
+// 8 warps 3,160 us, together 2,190; of 2.5, where the other form's registers serve
+// better, 503 against 460).  With the window off chip the sources are L2 reads, and read
+// together too (4,000 events of 2.5, 8 warps 681 -> 603 us); LONG then reads nothing
+// ahead, for want of registers (of 12.5: 2,900 -> 2,190; reading ahead as well spilled,
+// 2,830, and 1,415 against 884 of 4.5).
 constexpr int kGivenAhead = 4;
-template <bool WIN_SMEM, int S>
+template <bool WIN_SMEM, int S, bool LONG>
 __device__ __forceinline__ void stage_given(const KArgs &a, const EvRec *sev, const PredRec *spred, int pred0, int n_ev,
                                             uint32_t ctr, const TileCtx<S> &t, unsigned char *smem) {
     double *win = reinterpret_cast<double *>(smem);
@@ -615,8 +622,9 @@ __device__ __forceinline__ void stage_given(const KArgs &a, const EvRec *sev, co
         for (int j = 0; j < S; ++j)
             if (t.active[j]) d[j] = __ldcs(row + 32 * j);
     };
+    constexpr bool kAhead = WIN_SMEM || !LONG;
     auto read = [&](int i, double (&d)[kGivenAhead][S]) {
-        if (i >= n_ev) return;
+        if (!kAhead || i >= n_ev) return;
         const int4 e = reinterpret_cast<const int4 *>(sev + i)[0];  // user, slot, pred_begin, pred_end
 #pragma unroll
         for (int k = 0; k < kGivenAhead; ++k)
@@ -643,23 +651,62 @@ __device__ __forceinline__ void stage_given(const KArgs &a, const EvRec *sev, co
             cause[j] = -1;
         }
         const int pb = ev.pred_begin - pred0, np = ev.pred_end - ev.pred_begin;
-        auto entry = [&](int4 rec, const double (&dur)[S]) {
-            double src[S];
-            source<WIN_SMEM, S>(t, win, rec.x, rec.y, src);
+        auto relaxed = [&](const double (&src)[S], const double (&dur)[S], int32_t user) {
 #pragma unroll
             for (int j = 0; j < S; ++j) {
                 bool clamp;
-                if (relax<false>(src[j], dur[j], ev.ub_key, ev.ub_bits, lk[j], lbits[j], clamp)) cause[j] = rec.y;
+                if (relax<false>(src[j], dur[j], ev.ub_key, ev.ub_bits, lk[j], lbits[j], clamp)) cause[j] = user;
             }
         };
+        auto entry = [&](int4 rec, const double (&dur)[S]) {
+            double src[S];
+            source<WIN_SMEM, S>(t, win, rec.x, rec.y, src);
+            relaxed(src, dur, rec.y);
+        };
+        // entries p to p + kGivenAhead - 1; sources that lie off chip are read together
+        auto entries = [&](int p, const double (&dur)[kGivenAhead][S]) {
+            const int4 *recs = reinterpret_cast<const int4 *>(spred + pb + p);
+            double src[kGivenAhead][S];
 #pragma unroll
-        for (int k = 0; k < kGivenAhead; ++k)
-            if (k < np) entry(reinterpret_cast<const int4 *>(spred + pb + k)[0], d[k]);
-        for (int k = kGivenAhead; k < np; ++k) {
-            const int4 rec = reinterpret_cast<const int4 *>(spred + pb + k)[0];
-            double dur[S];
-            duration(rec.z, dur);
-            entry(rec, dur);
+            for (int k = 0; k < kGivenAhead; ++k)
+                if (p + k < np) source<WIN_SMEM, S>(t, win, recs[2 * k].x, recs[2 * k].y, src[k]);
+#pragma unroll
+            for (int k = 0; k < kGivenAhead; ++k)
+                if (p + k < np) relaxed(src[k], dur[k], recs[2 * k].y);
+        };
+        if constexpr (!kAhead) {
+            for (int p = 0; p < np; p += kGivenAhead) {
+                double now[kGivenAhead][S];
+#pragma unroll
+                for (int k = 0; k < kGivenAhead; ++k)
+                    if (p + k < np) duration(reinterpret_cast<const int4 *>(spred + pb + p + k)->z, now[k]);
+                entries(p, now);
+            }
+        } else if constexpr (!WIN_SMEM) {
+            entries(0, d);
+        } else {
+#pragma unroll
+            for (int k = 0; k < kGivenAhead; ++k)
+                if (k < np) entry(reinterpret_cast<const int4 *>(spred + pb + k)[0], d[k]);
+        }
+        if constexpr (LONG && kAhead) {
+            for (int p = kGivenAhead; p < np; p += kGivenAhead) {
+                const int4 *recs = reinterpret_cast<const int4 *>(spred + pb + p);
+                double rest[kGivenAhead][S];
+#pragma unroll
+                for (int k = 0; k < kGivenAhead; ++k)
+                    if (p + k < np) duration(recs[2 * k].z, rest[k]);
+#pragma unroll
+                for (int k = 0; k < kGivenAhead; ++k)
+                    if (p + k < np) entry(recs[2 * k], rest[k]);
+            }
+        } else if constexpr (!LONG) {
+            for (int k = kGivenAhead; k < np; ++k) {
+                const int4 rec = reinterpret_cast<const int4 *>(spred + pb + k)[0];
+                double dur[S];
+                duration(rec.z, dur);
+                entry(rec, dur);
+            }
         }
 #pragma unroll
         for (int j = 0; j < S; ++j)
@@ -846,7 +893,7 @@ __device__ __forceinline__ void stage_events(const KArgs &a, int buf, const EvRe
 // a.blk_start stages begins -- the checkpoints a level-block recomputation
 // starts from.
 template <bool GIVEN, bool WIN_SMEM, bool STATS, bool POSITIVE, bool ADJ = false, int TS = kTablesEither,
-          bool LANE_HIST = true, int S = 1>
+          bool LANE_HIST = true, int S = 1, bool LONG = false>
 __device__ __forceinline__ bool propagate_tile(const KArgs &a, int64_t tile, double *rows, int64_t rows_ld,
                                                bool rows_tile_local, unsigned char *smem, uint64_t *bars,
                                                bool reuse, double *spill = nullptr) {
@@ -956,7 +1003,7 @@ __device__ __forceinline__ bool propagate_tile(const KArgs &a, int64_t tile, dou
         if (meta.y >= 0) {  // records in the staging buffer (shared memory)
             const unsigned char *buf = smem + a.smem_stage_off + b * a.stage_bytes;
             if constexpr (GIVEN)
-                stage_given<WIN_SMEM, S>(a, reinterpret_cast<const EvRec *>(buf), reinterpret_cast<const PredRec *>(buf + mv.z),
+                stage_given<WIN_SMEM, S, LONG>(a, reinterpret_cast<const EvRec *>(buf), reinterpret_cast<const PredRec *>(buf + mv.z),
                                          meta.z, meta.y, ctr, t, smem);
             else
                 stage_events<WIN_SMEM, STATS, POSITIVE, ADJ, true, TS, LANE_HIST, S>(
@@ -964,7 +1011,7 @@ __device__ __forceinline__ bool propagate_tile(const KArgs &a, int64_t tile, dou
                 meta.x, meta.y, n_pair, ctr, t, smem, grp);
         } else {  // a stage whose records exceed the buffer is read from global memory
             if constexpr (GIVEN)
-                stage_given<WIN_SMEM, S>(a, a.ev + meta.x, a.pred + meta.z, meta.z, -meta.y, ctr, t, smem);
+                stage_given<WIN_SMEM, S, LONG>(a, a.ev + meta.x, a.pred + meta.z, meta.z, -meta.y, ctr, t, smem);
             else
                 stage_events<WIN_SMEM, STATS, POSITIVE, ADJ, false, TS, LANE_HIST, S>(
                 a, b, a.ev + meta.x, a.pred + meta.z, meta.z, meta.x, -meta.y, n_pair, ctr, t, smem, grp);
@@ -1007,10 +1054,10 @@ __global__ void __launch_bounds__(768, 1) k_propagate(const KArgs a) {
 
 // The same with given durations (a.dur_in), which may be anything.
 constexpr int kGivenWarps = 32;  // most warps of a CTA, and of an SM (64 registers a thread)
-template <bool WIN_SMEM, int S>
+template <bool WIN_SMEM, int S, bool LONG>
 __global__ void __launch_bounds__(kGivenWarps * 32, 1) k_propagate_given(const KArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
-    propagate_tile<true, WIN_SMEM, false, false, false, kTablesEither, true, S>(
+    propagate_tile<true, WIN_SMEM, false, false, false, kTablesEither, true, S, LONG>(
         a, (int64_t)blockIdx.x, a.realized ? a.realized : a.scratch, a.ld, false, smem,
         reinterpret_cast<uint64_t *>(smem + a.smem_bar_off), false);
 }
