@@ -53,6 +53,10 @@ __device__ __forceinline__ int quick_bin(float f, const DelayBins &d, int nb) {
     return q < 0.0f ? 0 : q > (float)nb ? nb + 1 : 1 + (int)q;
 }
 
+// Whether the square of base b or its reciprocal's is so far out that a link's relative
+// moments cannot be had from its absolute ones.
+__host__ __device__ inline bool far_base(double b) { return b != 0.0 && !(fabs(b) >= 1e-100 && fabs(b) <= 1e100); }
+
 struct HistArgs {
     const int32_t *cls;      // [L] class of each link, -1: none
     const double *base;      // [L]
@@ -82,11 +86,13 @@ constexpr int kHistLanes = 4;  // samples a lane draws at a time
 //                        bins in single precision, the exact quotient only where an
 //                        edge is near.
 // Relative sums follow per link from the absolute ones (the base divides out), so
-// they cost one division a link and item.
+// they cost one division a link and item; of bases beyond 1e-100 to 1e100 every delay
+// is divided (far_base).
 // 10,000 samples of 1,000 events (2,400 links, five kinds): 0.39 ms; as a
 // propagation with a durations output and a kernel that binned those with FP64
 // divisions and FP64 shared-memory atomics the whole call took 12.4 ms more.
-template <bool TSMEM>
+// FAR: some link has a far base (the check in the draws' loop costs the others 13 %).
+template <bool TSMEM, bool FAR>
 __global__ void __launch_bounds__(kHistThreads) k_delay_hist(const KArgs a, const HistArgs h) {
     extern __shared__ __align__(16) unsigned char sm[];
     const int nh = h.nc * 2 * (h.nb + 2);
@@ -167,6 +173,7 @@ __global__ void __launch_bounds__(kHistThreads) k_delay_hist(const KArgs a, cons
                     }
                     const double b = __ldg(h.base + r0.x);
                     // (NaN, so every bin exact, where the base is no finite float)
+                    const bool far = FAR && far_base(b);
                     const float invb = fabsf((float)b) < 3e38f ? 1.0f / (float)b : __int_as_float(0x7FC00000);
                     double sum = 0.0, sq = 0.0;
 #pragma unroll
@@ -193,6 +200,11 @@ __global__ void __launch_bounds__(kHistThreads) k_delay_hist(const KArgs a, cons
                             k = quick_bin(f * invb, bins[c * 2 + 1], h.nb);
                             if (k < 0) k = exact(c, 1, delta / b);
                             count(c, 1, k, 1u);
+                            if (far) {
+                                const double x = delta / b;
+                                atomicAdd(&smom[c * 6 + 4], x);
+                                atomicAdd(&smom[c * 6 + 5], x * x);
+                            }
                         }
                     }
                     if (c >= 0) {
@@ -212,8 +224,8 @@ __global__ void __launch_bounds__(kHistThreads) k_delay_hist(const KArgs a, cons
                 if (c < 0) continue;
                 const double b = __ldg(h.base + r0.x);
                 const double m = (double)(end - block0);
-                double sum, sq;
-                const bool fixed = kind == K_FIXED;
+                double sum, sq, rel = 0.0, rel_sq = 0.0;  // (the latter two of far bases)
+                const bool fixed = kind == K_FIXED, far = FAR && far_base(b);
                 if (fixed || (vt >= 0 && dists[r0.y >> 8].tab_n <= 32)) {
                     unsigned n_k;  // this lane's value and how often it was drawn
                     double delta = 0.0;
@@ -231,6 +243,11 @@ __global__ void __launch_bounds__(kHistThreads) k_delay_hist(const KArgs a, cons
                     }
                     sum = (double)n_k * delta;
                     sq = sum * delta;
+                    if (far && n_k) {
+                        const double x = delta / b;
+                        rel = (double)n_k * x;
+                        rel_sq = rel * x;
+                    }
                 } else {
                     double2 &t = wacc[i * 32 + lane];
                     sum = t.x;
@@ -242,10 +259,18 @@ __global__ void __launch_bounds__(kHistThreads) k_delay_hist(const KArgs a, cons
                     sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
                     sq += __shfl_xor_sync(0xFFFFFFFFu, sq, o);
                 }
+                if (far) {
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) {
+                        rel += __shfl_xor_sync(0xFFFFFFFFu, rel, o);
+                        rel_sq += __shfl_xor_sync(0xFFFFFFFFu, rel_sq, o);
+                    }
+                }
                 if (lane < (b != 0.0 ? 6 : 3)) {  // lanes 0-2: count, sum, squares of the delays; 3-5: relative
                     const double s = lane >= 3 ? 1.0 / b : 1.0;
                     const int k = lane % 3;
-                    atomicAdd(&smom[c * 6 + lane], k == 0 ? m : k == 1 ? sum * s : sq * s * s);
+                    const double first = far && lane >= 3 ? rel : sum * s, second = far && lane >= 3 ? rel_sq : sq * s * s;
+                    atomicAdd(&smom[c * 6 + lane], k == 0 ? m : k == 1 ? first : second);
                 }
             }
             __syncwarp();
@@ -300,7 +325,11 @@ int mcd_delay_histograms(mcd_dag *g, const int64_t *seeds, int64_t n, const int3
         const size_t tables = hd.tables_in_smem ? hist_tables_bytes((int32_t)hd.dist.size(), (int32_t)hd.alias.size()) : 0;
         const size_t smem = tables + kHistWarps * kGroupLinks * 32 * (sizeof(double2) + 4) +
                             (size_t)n_classes * (48 + 2 * sizeof(DelayBins)) + nh * 4;
-        void (*fn)(const KArgs, const HistArgs) = hd.tables_in_smem ? k_delay_hist<true> : k_delay_hist<false>;
+        bool far = false;
+        for (int32_t l = 0; l < L; ++l) far = far || far_base(link_base[l]);
+        void (*fn)(const KArgs, const HistArgs) =
+            hd.tables_in_smem ? far ? k_delay_hist<true, true> : k_delay_hist<true, false>
+                              : far ? k_delay_hist<false, true> : k_delay_hist<false, false>;
         cuda_check(raise_smem_limit((const void *)fn, smem), "histogram shared memory");
         int sms = 0, per_sm = 0;
         cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device), "device query");
