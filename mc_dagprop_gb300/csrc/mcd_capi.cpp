@@ -77,6 +77,7 @@ KArgs base_args(const mcd_dag *g) {
     a.n_events = g->h.E;
     a.rows_planned = g->h.rows_planned ? 1 : 0;
     a.n_entries = (int32_t)g->h.pred.size();
+    a.n_sampled = (int32_t)g->h.sampled_entries;
     a.n_aux = (int32_t)g->h.aux.size();
     a.window_slots = g->h.window_slots;
     a.n_dist = (int32_t)g->h.dist.size();

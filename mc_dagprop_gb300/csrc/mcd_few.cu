@@ -323,19 +323,34 @@ int sm_count();
 //   100 events in 2 stages (work 4)    8.3 and 12.7 us: the second launch is not repaid
 //   150 in 7 (10)        x 40 18.6, 17.0    x 608 18.6, 20.6
 //   203 in 11 (14)       x 152 24.7, 20.5   x 608 24.7, 22.6   x 2,432 24.7, 26.1
-//   2,000 in 34 (65)     x 608 122, 51      x 2,432 123, 111   x 3,001 123, 130
+//   2,000 in 34 (65)     x 608 122, 51      x 2,432 123, 111
 //   20,017 in 493 (805)  x 608 1,755, 560   x 2,432 1,757, 1,196   x 3,001 1,758, 1,506
-//   2,000 in 45 (76)     x 3,040 135, 141: stages of some 42 events divide the last two
 // and durations given, whose general kernel has less to do a stage,
 //   203  x 608 20.6, 23.1;  600 in 20 (29)  x 608 45, 31   x 1,824 45, 39   x 2,432 45, 46
 //   20,017  x 1,216 1,424, 769   x 1,824 1,426, 1,017;  50,000 in 833  x 2,432 2,889, 2,929
+// What the last samples an SM gain, as the time of the general kernels over that of
+// these, at 12 to 100 events a level in 13 to 455 stages:
+//   drawn, up to 30 stages   16 an SM 1.02-1.29, 18 0.97-1.29;
+//                            20 up to 20 events a level 1.00-1.26, 30 to 100 0.93-1.06
+//   40 stages and more       18 1.01-1.97;
+//                            20 where four fifths of the entries draw 1.01-1.73; where half
+//                            of them do, up to 30 events a level 1.11-1.89, 44 to 100 0.94-1.03
+// (the draws are dealt out evenly here and lie on the stages' chain there; narrow levels
+// leave the general kernels' warps idle).
 // direct: the rows go straight to the host, which saves more launches than this adds.
 bool few_layout(const KArgs &a, int64_t n, bool given, bool direct, FewArgs &f) {
     const int sms = sm_count();
     if (n < 1 || !a.rows_planned || a.avg_units <= 0 || a.n_stages <= 0 || sms <= 0) return false;
     const int64_t work = a.n_stages + a.n_events / 64;
     if (!direct && work < (given ? 24 : 8)) return false;
-    const int most = given ? 12 : work < 12 ? 1 : work < 24 ? 4 : a.n_events <= 42 * (int64_t)a.n_stages ? 20 : 16;
+    const int64_t width = a.n_events / a.n_stages;
+    const bool drawing = 3 * (int64_t)a.n_sampled >= 2 * (int64_t)a.n_entries;
+    const int most = given             ? 12
+                     : work < 12       ? 1
+                     : work < 24       ? 4
+                     : width <= 24     ? 20
+                     : a.n_stages < 40 ? 16
+                     : width <= 36 || drawing ? 20 : 18;
     if (n > (int64_t)most * sms) return false;
     f.given = given;
     f.n = (int32_t)n;

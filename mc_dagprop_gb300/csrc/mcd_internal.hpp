@@ -216,6 +216,7 @@ struct KArgs {
     int32_t avg_units;        // their warps per CTA (pick_warps); 0: n_warps is the caller's choice
     int32_t stage_events, stage_entries;  // most events and precedence entries of a stage
     int32_t n_events, n_entries;
+    int32_t n_sampled;        // entries whose link draws
     int32_t rows_planned;     // slot words hold window rows
     int32_t n_aux;
     int32_t window_slots;
