@@ -183,9 +183,11 @@ int mcd_propagate_host(mcd_dag *dag, const double *durations, int64_t n, double 
 /* ---- Device buffers, sample-minor, asynchronous on `stream` (NULL = the handle's stream) ----
  * seeds[n] on the device; outputs realized[E*ld], durations[L*ld], cause_event[E*ld]
  * (any may be NULL).  Kernel errors are latched on the handle and reported by
- * mcd_dag_check().  Runs of few samples take scratch memory from a pool in the
- * stream's order (not while the stream is captured, nor where it cannot be had: the
- * same results by the general kernels). */
+ * mcd_dag_check().  Runs of few samples (at most 20 an SM) take up to 8 GiB of device
+ * memory from a pool in the stream's order (not while the stream is captured, nor where
+ * it cannot be had: the same results by the general kernels).  The pool, one a device,
+ * holds 32 MiB from the first handle on, keeps up to 2 GiB between such runs, and gives
+ * back what is above 32 MiB when the last handle that had one is destroyed. */
 int mcd_run_device(mcd_dag *dag, const int64_t *seeds, int64_t n, double *realized, double *durations,
                    int32_t *cause_event, int64_t ld, void *stream);
 /* Propagation alone from device durations[L*ld_in] (sample-minor). */

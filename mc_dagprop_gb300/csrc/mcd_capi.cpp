@@ -549,8 +549,11 @@ bool run_few(mcd_dag *g, const int64_t *seeds, const double *dur_in, int64_t n, 
 }
 
 // Scratch of few-sample launches on callers' streams: one pool a device, made with the
-// first handle (so that no run waits for it).  It keeps what a launch may need, and
-// kFewIdle once no handle that used it is left.
+// first handle (so that no run waits for it).  Between launches it keeps kFewKeep at most,
+// what is above goes back at the next synchronisation, and kFewIdle once no handle that
+// used it is left.  (What a launch has to take anew costs about a millisecond a GiB:
+// 200,000 events x 608 samples, 2.4 GiB, waited for each time 3.8 ms with all of it kept,
+// 4.6 with 2 GiB, 6.7 with 1, 8.8 with none; 20,017 x 3,001, 1.2 GiB, 1.5, 1.5, 2.0, 4.0.)
 struct FewPool {
     std::mutex mu;
     bool made = false;
@@ -558,6 +561,7 @@ struct FewPool {
     int users = 0;                 // handles that took from it
 };
 FewPool g_few_pool[64];
+constexpr size_t kFewKeep = (size_t)2 << 30;
 constexpr size_t kFewIdle = (size_t)32 << 20;
 
 cudaMemPool_t few_pool(mcd_dag *g, bool use) {
@@ -570,7 +574,7 @@ cudaMemPool_t few_pool(mcd_dag *g, bool use) {
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = g->device;
-        uint64_t keep = kFewScratch;
+        uint64_t keep = kFewKeep;
         void *p = nullptr;
         if (cudaMemPoolCreate(&fp.pool, &props) != cudaSuccess ||
             cudaMemPoolSetAttribute(fp.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess)

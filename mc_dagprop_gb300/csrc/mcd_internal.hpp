@@ -283,7 +283,7 @@ constexpr int kFewInline = 8;   // seeds that travel with the launch
 constexpr int64_t kFewDirect = 40000;  // events times samples up to which they are written straight to the host
 constexpr int kFewRing = 8;     // most stage buffers
 constexpr size_t kFewSmem = 225 * 1024;
-constexpr size_t kFewScratch = (size_t)8 << 30;  // most scratch of a launch, and what a handle's pool keeps
+constexpr size_t kFewScratch = (size_t)8 << 30;  // most scratch of a launch
 
 // Arguments beside the DAG's.  Element (row, sample) of an output lies at
 // row * out_row + sample * out_col, of durations at link * dur_row + sample * dur_col.
