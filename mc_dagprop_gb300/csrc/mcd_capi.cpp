@@ -26,6 +26,7 @@ cudaError_t launch_stats_finish(const FArgs &f, cudaStream_t st);
 cudaError_t launch_event_ticks(const double *earliest, int32_t E, int32_t q, long long *te, cudaStream_t st);
 cudaError_t launch_wait_selftest(int32_t *err, uint32_t limit, cudaStream_t st);
 cudaError_t noalloc_scratch(void **ptr, size_t *bytes);
+unsigned long long current_context_id();
 cudaError_t launch_transpose_f64(const double *in, int64_t ld_in, double *out, int64_t ld_out, int64_t rows,
                                  int64_t cols, cudaStream_t st);
 cudaError_t launch_transpose_i32(const int32_t *in, int64_t ld_in, int32_t *out, int64_t ld_out, int64_t rows,
@@ -548,8 +549,9 @@ bool run_few(mcd_dag *g, const int64_t *seeds, const double *dur_in, int64_t n, 
     return true;
 }
 
-// Scratch of few-sample launches on callers' streams: one pool a device, made with the
-// first handle (so that no run waits for it).  Between launches it keeps kFewKeep at most,
+// Scratch of few-sample launches on callers' streams: one pool a device and context (it
+// goes with its context at a device reset), made with the first handle (so that no run
+// waits for it).  Between launches it keeps kFewKeep at most,
 // what is above goes back at the next synchronisation, and kFewIdle once no handle that
 // used it is left.  (What a launch has to take anew costs about a millisecond a GiB:
 // 200,000 events x 608 samples, 2.4 GiB, waited for each time 3.8 ms with all of it kept,
@@ -557,8 +559,9 @@ bool run_few(mcd_dag *g, const int64_t *seeds, const double *dur_in, int64_t n, 
 struct FewPool {
     std::mutex mu;
     bool made = false;
-    cudaMemPool_t pool = nullptr;  // null: not to be had
-    int users = 0;                 // handles that took from it
+    unsigned long long context = 0;  // that the pool was made in
+    cudaMemPool_t pool = nullptr;    // null: not to be had
+    int users = 0;                   // handles that took from it
 };
 FewPool g_few_pool[64];
 constexpr size_t kFewKeep = (size_t)2 << 30;
@@ -568,8 +571,12 @@ cudaMemPool_t few_pool(mcd_dag *g, bool use) {
     if (g->device < 0 || g->device >= 64) return nullptr;
     FewPool &fp = g_few_pool[g->device];
     std::lock_guard<std::mutex> lk(fp.mu);
-    if (!fp.made) {
+    const unsigned long long context = current_context_id();
+    if (!fp.made || fp.context != context) {
         fp.made = true;
+        fp.context = context;
+        fp.pool = nullptr;
+        fp.users = 0;
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
@@ -583,7 +590,10 @@ cudaMemPool_t few_pool(mcd_dag *g, bool use) {
             cudaFreeAsync(p, g->stream[0]);
         (void)cudaGetLastError();
     }
-    if (use && fp.pool && !g->few_used.exchange(true)) ++fp.users;
+    if (use && fp.pool && !g->few_used.exchange(true)) {
+        g->few_context = context;
+        ++fp.users;
+    }
     return fp.pool;
 }
 
@@ -591,7 +601,7 @@ void few_pool_leave(mcd_dag *g) {
     if (!g->few_used.exchange(false)) return;
     FewPool &fp = g_few_pool[g->device];
     std::lock_guard<std::mutex> lk(fp.mu);
-    if (--fp.users == 0 && cudaMemPoolTrimTo(fp.pool, kFewIdle) != cudaSuccess) (void)cudaGetLastError();
+    if (g->few_context == fp.context && --fp.users == 0 && cudaMemPoolTrimTo(fp.pool, kFewIdle) != cudaSuccess) (void)cudaGetLastError();
 }
 
 // The same with device buffers (a: the launch's arguments, sample-minor rows).  The

@@ -287,7 +287,7 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratch
 // cuCtxGetCurrent and cuCtxGetId, found through the runtime so the library needs
 // no link to the driver library; ids are never reused within a process), or 0
 // when no context is current yet.
-static unsigned long long current_context_id() {
+unsigned long long current_context_id() {
     using CtxGetCurrent = int (*)(void **);
     using CtxGetId = int (*)(void *, unsigned long long *);
     static const std::pair<CtxGetCurrent, CtxGetId> fns = [] {
