@@ -20,6 +20,7 @@
 
 namespace mcd {
 cudaError_t launch_propagate(const KArgs &a, bool given, bool win_smem, bool stats, cudaStream_t st);
+bool wide_pays(const KArgs &a);
 bool few_layout(const KArgs &a, int64_t n, bool given, bool direct, FewArgs &f);
 cudaError_t launch_few(const KArgs &a, const FewArgs &f, cudaStream_t st);
 cudaError_t launch_stats_finish(const FArgs &f, cudaStream_t st);
@@ -1000,12 +1001,13 @@ int mcd_propagate_host(mcd_dag *g, const double *durations, int64_t n, double *r
 // How a statistics run of n samples uses the handle's workspace beside the
 // accumulators: samples per launch, and the rows that do not fit on chip --
 // realized rows when the window is off chip (512 MiB of them a launch), or the
-// off-chip window rows of wide tiles (256 MiB a launch).
+// off-chip window rows of wide tiles, where those run (256 MiB a launch).
 struct StatsChunk {
     int64_t C;
     size_t rows_bytes, spill_bytes;
 };
-static StatsChunk stats_chunk(const HostDag &h, int64_t n) {
+static StatsChunk stats_chunk(const mcd_dag *g, int64_t n) {
+    const HostDag &h = g->h;
     StatsChunk c{n, 0, 0};
     if (!h.win_smem) {
         const size_t row = std::max<size_t>((size_t)h.E * 8, 1);
@@ -1013,7 +1015,10 @@ static StatsChunk stats_chunk(const HostDag &h, int64_t n) {
         c.rows_bytes = align_up((size_t)h.E * (size_t)c.C * 8, 256);
     } else if (h.wide_rows > 0 && h.window_spill > 0) {
         const size_t tile = (size_t)h.window_spill * kWideTile * sizeof(double);
-        c.C = std::min<int64_t>(n, (int64_t)((256ull << 20) / tile) * kWideTile);
+        KArgs a = base_args(g);
+        a.n = std::min<int64_t>(n, (int64_t)((256ull << 20) / tile) * kWideTile);
+        if (!wide_pays(a)) return c;
+        c.C = a.n;
         c.spill_bytes = align_up((size_t)((c.C + kWideTile - 1) / kWideTile) * tile, 256);
     }
     return c;
@@ -1026,7 +1031,7 @@ static void stats_device(mcd_dag *g, const int64_t *seeds, int64_t seed0, int64_
     const HostDag &h = g->h;
     const size_t E = (size_t)h.E;
     const StatsParams sp = stats_params(h, n);
-    const StatsChunk ch = stats_chunk(h, n);
+    const StatsChunk ch = stats_chunk(g, n);
     const int64_t C = ch.C;
     const size_t acc_bytes = align_up(E * 8, 256), hist_bytes = align_up(E * kHistStride * 4, 256),
                  te_bytes = align_up(E * 8, 256);
@@ -1104,7 +1109,7 @@ int mcd_stats_host(mcd_dag *g, const int64_t *seeds, int64_t seed0, int64_t n, c
         const size_t hist_out = out->hist ? hist_bytes : 0;
         // reserve: [accumulators | hist | ticks | scratch] ... [outputs (5 x E doubles) | hist copy | seeds]
         const size_t head = 5 * out_bytes + hist_out + seeds_bytes;
-        const StatsChunk ch = stats_chunk(g->h, n);
+        const StatsChunk ch = stats_chunk(g, n);
         ensure_ws(g, acc_bytes + hist_bytes + te_bytes + ch.rows_bytes + ch.spill_bytes + head);
         // stats_device carves its regions from the start of the workspace, so the
         // staging area goes at the end

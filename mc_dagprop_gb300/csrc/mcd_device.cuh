@@ -42,8 +42,10 @@ cudaError_t raise_smem_limit(const void *fn, size_t smem);
 // SM and a CTA hold at the kernel's registers).
 int pick_warps(const KArgs &a, int64_t tiles, int sm_warps = 24, int cta_warps = 24);
 
-// Wide tiles (two samples a lane) of a sampled launch: whether they run it, and the
-// arguments with their layout in place.
+// Wide tiles (two samples a lane) of a launch: whether they are the faster ones, whether
+// they run it (they need a place for their off-chip rows), and the arguments with their
+// layout in place.
+bool wide_pays(const KArgs &a);
 bool use_wide(const KArgs &a);
 KArgs wide_args(const KArgs &a);
 

@@ -232,14 +232,18 @@ int pick_warps(const KArgs &a, int64_t tiles, int sm_warps, int cta_warps) {
 // three narrow tiles against two wide ones.
 // Measured (narrow, wide): 200,000 events x 9,728 samples, outputs 24.0, 21.4 ms;
 // statistics of 10,000 events x 65,536 samples 10.2, 8.6 ms.
-bool use_wide(const KArgs &a) {
+bool wide_pays(const KArgs &a) {
     if (a.wide_rows <= 0 || !a.positive || !a.tables_in_smem || ctas_fit(a.smem_total) > 1) return false;
-    if (a.window_spill > 0 && !a.spill && !a.realized) return false;  // no place for the off-chip rows
     const int sms = sm_count();
     if (!sms) return false;
     const int64_t narrow = (a.n + (int64_t)sms * kTile - 1) / ((int64_t)sms * kTile);
     const int64_t wide = (a.n + (int64_t)sms * kWideTile - 1) / ((int64_t)sms * kWideTile);
     return 9 * narrow >= 16 * wide;
+}
+
+bool use_wide(const KArgs &a) {
+    if (a.window_spill > 0 && !a.spill && !a.realized) return false;  // no place for the off-chip rows
+    return wide_pays(a);
 }
 
 KArgs wide_args(const KArgs &a) {
