@@ -24,6 +24,7 @@
 #include "mcd_handle.hpp"
 
 namespace mcd {
+bool wide_pays(const KArgs &a);
 cudaError_t launch_adjoint_forward(const KArgs &a, cudaStream_t st);
 cudaError_t launch_adjoint_backward(const KArgs &a, cudaStream_t st);
 cudaError_t launch_event_ticks(const double *earliest, int32_t E, int32_t q, long long *te, cudaStream_t st);
@@ -150,11 +151,16 @@ extern "C" int mcd_gradient_host(mcd_dag *g, int64_t seed0, int64_t n, double *o
                      s_cck = (h.win_smem && blocks) ? align_up(tiles * win_n * 4, 256) : 0,
                      s_rows = h.win_smem ? 0 : align_up(E * (size_t)C * 8, 256),
                      s_crow = h.win_smem ? 0 : align_up(E * (size_t)C * 4, 256),
-                     s_blk = align_up(n_blk * 4 + 4, 256),
-                     // off-chip window rows of the forward's wide tiles (level blocks run narrow ones)
-                     s_spill = (h.wide_rows > 0 && !blocks) ? align_up((size_t)((C + kWideTile - 1) / kWideTile) *
-                                                                           h.window_spill * kWideTile * 8, 256)
-                                                            : 0;
+                     s_blk = align_up(n_blk * 4 + 4, 256);
+        // off-chip window rows of the forward's wide tiles, where those run (level blocks run
+        // narrow ones) and the budget has room beside the plan's buffers
+        size_t s_spill = 0;
+        if (h.window_spill > 0 && !blocks) {
+            KArgs a = base_args(g);
+            a.n = std::min(C, n);
+            s_spill = align_up((size_t)((C + kWideTile - 1) / kWideTile) * h.window_spill * kWideTile * 8, 256);
+            if (!wide_pays(a) || plan.bytes + s_spill > budget) s_spill = 0;
+        }
         ensure_ws(g, s_code + s_dfac + s_acc + s_ge + s_gl + s_out + s_te + s_wck + s_cck + s_rows + s_crow + s_blk +
                          s_spill);
         char *p = g->ws;
@@ -253,7 +259,7 @@ extern "C" int mcd_gradient_host(mcd_dag *g, int64_t seed0, int64_t n, double *o
         check_device_error(g);
         g->last_adj_plan[0] = (int64_t)C;
         g->last_adj_plan[1] = (int64_t)n_blk;
-        g->last_adj_plan[2] = (int64_t)plan.bytes;
+        g->last_adj_plan[2] = (int64_t)(plan.bytes + s_spill);
     });
 }
 
