@@ -134,8 +134,9 @@ int mcd_dag_create(const mcd_dag_desc *desc, const mcd_generator *gen, mcd_dag *
 /* Compile options (the same call with explicit choices). */
 #define MCD_WARPS_BATCH_CLASS (-1)
 typedef struct mcd_dag_options {
-    int32_t n_warps; /* warps per CTA, 1..24 (kept by every launch); 0 = chosen from the
-                        DAG's level width and, per launch, its samples;
+    int32_t n_warps; /* warps per CTA, 1..24 (kept by every launch but a batch's wide tiles,
+                        mcd_batch_plan); 0 = chosen from the DAG's level width and, per
+                        launch, its samples;
                         MCD_WARPS_BATCH_CLASS = chosen, then rounded up to 2, 4, 8, 12 or 24 */
     int32_t no_cache; /* 0: share the compiled records of a live handle created from
                          identical inputs (same arrays, generator, options and device);
@@ -260,8 +261,13 @@ int mcd_batch_run(mcd_batch *batch);
 int mcd_batch_sync(mcd_batch *batch);
 int mcd_batch_download(mcd_batch *batch, int32_t i, const mcd_stats *host);
 void *mcd_batch_stream(const mcd_batch *batch);
-int64_t mcd_batch_items(const mcd_batch *batch);
+int64_t mcd_batch_items(const mcd_batch *batch); /* 32-sample tiles over all DAGs */
 int32_t mcd_batch_grid(const mcd_batch *batch);
+/* What the launches consume: the items queued (a DAG that runs wide tiles queues one
+ * for 64 samples), the DAGs that run wide tiles, and the most warps per CTA of a launch
+ * (more than the DAGs' n_warps where wide tiles leave room for fewer CTAs an SM).  Any
+ * may be NULL. */
+int mcd_batch_plan(const mcd_batch *batch, int64_t *queued_items, int32_t *wide_dags, int32_t *most_warps);
 /* CTAs of the persistent batch kernel one SM holds at n_warps warps per CTA and
  * smem_bytes of dynamic shared memory (the largest mcd_dag_info.smem_bytes of the
  * batch): DAGs with equal values share a launch without lowering each other's

@@ -1,8 +1,8 @@
 """Batched runs of many DAGs in persistent launches, with a small autotuner.
 
 A ``Batch`` compiles every DAG with the same number of warps per CTA (the CTA
-size of its persistent launch) and runs all (DAG, 32-sample tile) work items in
-one CUDA graph.  The warps per CTA trade work per stage against barrier and idle
+size of its persistent launch) and runs all (DAG, tile of 32 or 64 samples) work
+items in one CUDA graph (``Batch.plan`` says which).  The warps per CTA trade work per stage against barrier and idle
 time: wide DAGs want many warps, narrow ones few (and more CTAs per SM); where
 the propagation window lives trades shared memory (fewer CTAs per SM) against
 global-memory reads of predecessor times.
@@ -193,7 +193,8 @@ class BatchRunner:
 
     @property
     def classes(self) -> list:
-        """(warps per CTA, CTAs per SM, DAG count, work items) of each class batch."""
+        """(warps per CTA its DAGs are compiled with, CTAs per SM, DAG count, 32-sample
+        tiles) of each class batch."""
         return [(w, per_sm, len(idx), b.items) for w, per_sm, idx, b in self.batches]
 
     def run(self, wait: bool = True) -> None:

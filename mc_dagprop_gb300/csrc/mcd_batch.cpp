@@ -328,6 +328,22 @@ void *mcd_batch_stream(const mcd_batch *B) { return B ? (void *)B->stream : null
 int64_t mcd_batch_items(const mcd_batch *B) { return B ? B->n_items : -1; }
 int32_t mcd_batch_grid(const mcd_batch *B) { return B ? B->grid : -1; }
 
+int mcd_batch_plan(const mcd_batch *B, int64_t *queued_items, int32_t *wide_dags, int32_t *most_warps) {
+    return guarded([&] {
+        if (!B) throw McdError(MCD_ERR_INVALID, "null batch");
+        int64_t queued = 0;
+        int32_t wide = 0, warps = 0;
+        for (const Launch &L : B->launches) {
+            queued += L.args.n_items;
+            if (L.wide) wide += (int32_t)L.dags.size();
+            warps = std::max(warps, L.n_warps);
+        }
+        if (queued_items) *queued_items = queued;
+        if (wide_dags) *wide_dags = wide;
+        if (most_warps) *most_warps = warps;
+    });
+}
+
 int mcd_batch_download(mcd_batch *B, int32_t i, const mcd_stats *host) {
     return guarded([&] {
         if (!B || !host || i < 0 || i >= (int32_t)B->dags.size()) throw McdError(MCD_ERR_INVALID, "bad arguments");

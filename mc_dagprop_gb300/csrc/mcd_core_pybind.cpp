@@ -503,6 +503,16 @@ class Batch {
         }
         raise_status(rc);
     }
+    py::dict plan() const {
+        int64_t queued = 0;
+        int32_t wide = 0, warps = 0;
+        raise_status(mcd_batch_plan(b_.get(), &queued, &wide, &warps));
+        py::dict d;
+        d["queued_items"] = queued;
+        d["wide_dags"] = wide;
+        d["most_warps"] = warps;
+        return d;
+    }
     py::dict stats(int i, bool hist) {
         if (i < 0 || i >= (int)props_.size()) throw py::index_error("batch index out of range");
         const int64_t E = props_[i]->node_count();
@@ -838,7 +848,9 @@ PYBIND11_MODULE(_core, m) {
         .def("run", &Batch::run, py::arg("wait") = true, "Run the batch (one CUDA graph launch)")
         .def("sync", &Batch::sync, "Wait for the last run and report kernel errors")
         .def("stats", &Batch::stats, py::arg("i"), py::arg("hist") = false, "Statistics of propagator i")
-        .def_property_readonly("items", &Batch::items, "Work items (DAG, 32-sample tile)")
+        .def_property_readonly("items", &Batch::items, "32-sample tiles over all DAGs")
+        .def_property_readonly("plan", &Batch::plan,
+                               "What the launches consume: {queued_items, wide_dags, most_warps}")
         .def_property_readonly("grid", &Batch::grid, "CTAs of the persistent launch")
         .def_static(
             "occupancy",
