@@ -61,6 +61,18 @@ void ensure_ws(mcd_dag *g, size_t bytes) {
     g->ws_bytes = bytes;
 }
 
+// The same; false where the device has no memory for it (calls that run with less).
+static bool try_ws(mcd_dag *g, size_t bytes) {
+    try {
+        ensure_ws(g, bytes);
+    } catch (const McdError &e) {
+        if (e.code != MCD_ERR_NOMEM) throw;
+        (void)cudaGetLastError();
+        return false;
+    }
+    return true;
+}
+
 KArgs base_args(const mcd_dag *g) {
     KArgs a{};
     a.ev = g->d_ev;
@@ -491,7 +503,7 @@ bool run_few(mcd_dag *g, const int64_t *seeds, const double *dur_in, int64_t n, 
         cuda_check(cudaMemGetInfo(&free_b, &total_b), "device memory query");
         if (bytes > std::min((free_b + g->ws_bytes) / 4, (size_t)32 << 30)) return false;
     }
-    ensure_ws(g, bytes);
+    if (!try_ws(g, bytes)) return false;
     char *p = g->ws;
     auto take = [&](size_t bytes) {
         char *q = p;
@@ -1024,18 +1036,30 @@ static StatsChunk stats_chunk(const mcd_dag *g, int64_t n) {
     return c;
 }
 
+// Reserves the workspace of a statistics run and `extra` bytes: per-event accumulators
+// and the chunk's rows.  Without memory for a wide plan's off-chip rows, narrow tiles.
+static StatsChunk stats_reserve(mcd_dag *g, int64_t n, size_t extra) {
+    const size_t E = (size_t)g->h.E;
+    const size_t rest = 2 * align_up(E * 8, 256) + align_up(E * kHistStride * 4, 256) + extra;
+    const StatsChunk c = stats_chunk(g, n);
+    if (c.spill_bytes && !try_ws(g, rest + c.spill_bytes)) {
+        ensure_ws(g, rest);
+        return StatsChunk{n, 0, 0};
+    }
+    ensure_ws(g, rest + c.rows_bytes + c.spill_bytes);
+    return c;
+}
+
 // Statistics of n samples into device outputs, asynchronously on st.  The
-// handle's workspace holds the per-event accumulators (and what stats_chunk says).
+// handle's workspace holds what stats_reserve took (ch).
 static void stats_device(mcd_dag *g, const int64_t *seeds, int64_t seed0, int64_t n, const mcd_stats *out,
-                         cudaStream_t st) {
+                         const StatsChunk &ch, cudaStream_t st) {
     const HostDag &h = g->h;
     const size_t E = (size_t)h.E;
     const StatsParams sp = stats_params(h, n);
-    const StatsChunk ch = stats_chunk(g, n);
     const int64_t C = ch.C;
     const size_t acc_bytes = align_up(E * 8, 256), hist_bytes = align_up(E * kHistStride * 4, 256),
                  te_bytes = align_up(E * 8, 256);
-    ensure_ws(g, acc_bytes + hist_bytes + te_bytes + ch.rows_bytes + ch.spill_bytes);
     auto *acc = reinterpret_cast<unsigned long long *>(g->ws);
     auto *hist = reinterpret_cast<uint32_t *>(g->ws + acc_bytes);
     auto *te = reinterpret_cast<long long *>(g->ws + acc_bytes + hist_bytes);
@@ -1088,7 +1112,8 @@ int mcd_stats_device(mcd_dag *g, const int64_t *seeds, int64_t seed0, int64_t n,
         if (!g || !out) throw McdError(MCD_ERR_INVALID, "null argument");
         if (n <= 0 || n > (int64_t)1 << 31) throw McdError(MCD_ERR_INVALID, "need 0 < n <= 2^31 samples");
         cuda_check(cudaSetDevice(g->device), "cudaSetDevice");
-        stats_device(g, seeds, seed0, n, out, stream ? (cudaStream_t)stream : g->stream[0]);
+        const StatsChunk ch = stats_reserve(g, n, 0);
+        stats_device(g, seeds, seed0, n, out, ch, stream ? (cudaStream_t)stream : g->stream[0]);
     });
 }
 
@@ -1102,15 +1127,13 @@ int mcd_stats_host(mcd_dag *g, const int64_t *seeds, int64_t seed0, int64_t n, c
         // device copies of the seeds and the outputs live after every region
         // stats_device carves (accumulators, histograms, earliest ticks, off-chip rows),
         // so none of them aliases
-        const size_t acc_bytes = align_up(E * 8, 256), hist_bytes = align_up(E * kHistStride * 4, 256),
-                     te_bytes = align_up(E * 8, 256);
+        const size_t hist_bytes = align_up(E * kHistStride * 4, 256);
         const size_t seeds_bytes = seeds ? align_up((size_t)n * 8, 256) : 0;
         const size_t out_bytes = align_up(E * 8, 256);
         const size_t hist_out = out->hist ? hist_bytes : 0;
         // reserve: [accumulators | hist | ticks | scratch] ... [outputs (5 x E doubles) | hist copy | seeds]
         const size_t head = 5 * out_bytes + hist_out + seeds_bytes;
-        const StatsChunk ch = stats_chunk(g, n);
-        ensure_ws(g, acc_bytes + hist_bytes + te_bytes + ch.rows_bytes + ch.spill_bytes + head);
+        const StatsChunk ch = stats_reserve(g, n, head);
         // stats_device carves its regions from the start of the workspace, so the
         // staging area goes at the end
         char *tail = g->ws + g->ws_bytes - head;
@@ -1121,7 +1144,7 @@ int mcd_stats_host(mcd_dag *g, const int64_t *seeds, int64_t seed0, int64_t n, c
         if (seeds) cuda_check(cudaMemcpyAsync(ds, seeds, (size_t)n * 8, cudaMemcpyHostToDevice, st), "seed upload");
         mcd_stats dev{out->mean ? o[0] : nullptr, out->p50 ? o[1] : nullptr, out->p90 ? o[2] : nullptr,
                       out->p99 ? o[3] : nullptr, out->p_on_time ? o[4] : nullptr, dh};
-        stats_device(g, ds, seed0, n, &dev, st);
+        stats_device(g, ds, seed0, n, &dev, ch, st);
         double *host_out[5] = {out->mean, out->p50, out->p90, out->p99, out->p_on_time};
         for (int k = 0; k < 5; ++k)
             if (host_out[k])
