@@ -60,10 +60,11 @@ struct mcd_batch {
     cudaGraphExec_t exec = nullptr;
 };
 
-extern "C" {
+extern "C" void mcd_batch_destroy(mcd_batch *B);
 
-int mcd_batch_create(mcd_dag *const *dags, int32_t n_dags, const int64_t *seed0, const int64_t *n_samples,
-                     mcd_batch **out) {
+// The batch with wide tiles where they pay, or without any.
+static int create_batch(mcd_dag *const *dags, int32_t n_dags, const int64_t *seed0, const int64_t *n_samples,
+                        bool may_be_wide, mcd_batch **out) {
     mcd_batch *B = nullptr;
     int rc = guarded([&] {
         if (!dags || !seed0 || !n_samples || !out || n_dags <= 0) throw McdError(MCD_ERR_INVALID, "bad arguments");
@@ -111,7 +112,7 @@ int mcd_batch_create(mcd_dag *const *dags, int32_t n_dags, const int64_t *seed0,
         const int64_t narrow_fit = std::min<int64_t>((228 * 1024) / ((int64_t)narrow_smem + 1024),
                                                      kMaxBatchWarps / std::max(1, B->n_warps));
         const double tiles_deep = work / (std::max(most, 1.0) * std::max(1, sms));
-        const bool wide_pays = narrow_fit <= 1 ? tiles_deep >= 3.0 : tiles_deep >= 9.0 && sampled < 0.65 * entries;
+        const bool wide_pays = may_be_wide && (narrow_fit <= 1 ? tiles_deep >= 3.0 : tiles_deep >= 9.0 && sampled < 0.65 * entries);
         // layout of the batch's device memory; launches by kernel variant
         B->ev_off.resize((size_t)n_dags + 1, 0);
         std::vector<int32_t> launch_of((size_t)n_dags);
@@ -267,6 +268,17 @@ int mcd_batch_create(mcd_dag *const *dags, int32_t n_dags, const int64_t *seed0,
         set_last_error(keep);
     }
     return rc;
+}
+
+extern "C" {
+
+int mcd_batch_create(mcd_dag *const *dags, int32_t n_dags, const int64_t *seed0, const int64_t *n_samples,
+                     mcd_batch **out) {
+    const int rc = create_batch(dags, n_dags, seed0, n_samples, true, out);
+    if (rc != MCD_ERR_NOMEM) return rc;
+    (void)cudaGetLastError();
+    // (no memory for the off-chip rows of wide tiles: 32-sample tiles need none)
+    return create_batch(dags, n_dags, seed0, n_samples, false, out);
 }
 
 void mcd_batch_destroy(mcd_batch *B) {

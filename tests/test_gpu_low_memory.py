@@ -9,7 +9,7 @@ from contextlib import contextmanager
 import numpy as np
 import pytest
 
-from mc_dagprop_gb300 import batching
+from mc_dagprop_gb300 import _core, batching
 from mc_dagprop_gb300 import workloads as W
 from mcd_testlib import kitchen_sink, lib
 
@@ -80,3 +80,29 @@ def test_statistics_without_room_for_off_chip_rows(cuda):
     with only(64 * MIB):
         got = prop.run_stats(n=n, seed0=5)
     assert all(np.array_equal(got[k], want[k]) for k in KEYS)
+
+
+def test_batches_without_room_for_off_chip_rows(cuda):
+    import torch
+
+    deep = 100 * torch.cuda.get_device_properties(0).multi_processor_count
+    dags = [kitchen_sink(seed=30 + i, n_layers=5, width=130) for i in range(3)]
+    props = [batching.compile_dag(f, g, 24) for f, g in dags]
+    wide = _core.Batch(props, [0, 1, 2], [deep] * 3)
+    assert wide.plan["wide_dags"] == 3
+    wide.run()
+    small = _core.Batch(props, [0, 1, 2], [100] * 3)  # (narrow tiles, loaded)
+    small.run()
+    narrow = None
+    for left in range(4, 64, 2):  # the first that leaves room for anything leaves none for the rows
+        with only(left * MIB):
+            try:
+                narrow = _core.Batch(props, [0, 1, 2], [deep] * 3)
+                break
+            except (RuntimeError, MemoryError):
+                pass
+    assert narrow.plan["wide_dags"] == 0
+    narrow.run()
+    for i in range(3):
+        a, b = wide.stats(i), narrow.stats(i)
+        assert all(np.array_equal(a[k], b[k]) for k in KEYS)
