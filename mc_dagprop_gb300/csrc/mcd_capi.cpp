@@ -885,6 +885,8 @@ int mcd_run_device(mcd_dag *g, const int64_t *seeds, int64_t n, double *realized
         a.durations = durations;
         a.cause = cause;
         if (!g->h.win_smem && !realized) {
+            // (also for few samples: a captured call runs the general kernels, and finds here
+            // what a call before the capture reserved)
             ensure_ws(g, (size_t)g->h.E * (size_t)ld * 8);
             a.scratch = (double *)g->ws;
         }

@@ -424,7 +424,8 @@ __device__ __forceinline__ long long tick_count(long long b, int q) {
 // Sum over the warp of non-negative 64-bit tick counts below 2^54: two 27-bit
 // limbs summed with one redux.sync each (a limb's sum stays below 2^32), then
 // recombined -- the exact sum.  The host's choice of tick keeps every per-sample
-// count below 2^54 (and the sum over all samples below 2^63).
+// count below 2^53, so a lane's two of a wide tile below 2^54 (and the sum over all
+// samples below 2^63).
 __device__ __forceinline__ long long warp_sum_ticks(long long d) {
     const unsigned long long u = (unsigned long long)d;
     const unsigned s0 = __reduce_add_sync(0xFFFFFFFFu, (unsigned)(u & 0x7FFFFFFu));

@@ -1,8 +1,9 @@
 // mcd_kernels.cu -- launch dispatch, statistics finish, earliest-tick tables and
 // layout kernels.
 //
-// The propagation kernel itself (k_propagate, mcd_device.cuh) is instantiated in
-// mcd_prop_sample.cu, mcd_prop_sample_gt.cu and mcd_prop_given.cu.
+// The propagation kernels themselves (mcd_device.cuh) are instantiated in
+// mcd_prop_sample.cu, mcd_prop_sample_gt.cu and mcd_prop_wide.cu (k_propagate) and in
+// mcd_prop_given.cu (k_propagate_given); few samples run those of mcd_few.cu.
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -222,7 +223,7 @@ int pick_warps(const KArgs &a, int64_t tiles, int sm_warps, int cta_warps) {
 }
 
 // A wide tile reads each record, decodes its kind and forms its addresses once for
-// 64 samples instead of 32 (121 -> 105 warp instructions per 32 sample-edges) and
+// 64 samples instead of 32 (121 -> 107 warp instructions per 32 sample-edges) and
 // its two samples' chains fill each other's latencies, so a CTA of 24 warps takes
 // 1.77 times as long for twice the samples.  It pays where a narrow CTA has its SM to
 // itself anyway: with two or three narrow CTAs an SM these hide each other's barriers
@@ -262,7 +263,8 @@ cudaError_t launch_prop_sample(const KArgs &a, bool win_smem, bool stats, bool p
                                size_t smem, cudaStream_t st);
 cudaError_t launch_prop_given(const KArgs &a, bool win_smem, cudaStream_t st);
 
-// One launch of the propagation kernel over a.n samples: one CTA per tile of 32.
+// One launch of the propagation kernel over a.n samples: one CTA per tile of 32, or of
+// 64 where wide tiles pay.
 // The shared-memory layout is fixed by the host compiler (KArgs::smem_*).
 cudaError_t launch_propagate(const KArgs &a, bool given, bool win_smem, bool stats, cudaStream_t st) {
     if (a.n <= 0) return cudaSuccess;
