@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -570,26 +571,24 @@ bool run_few(mcd_dag *g, const int64_t *seeds, const double *dur_in, int64_t n, 
 // 200,000 events x 608 samples, 2.4 GiB, waited for each time 3.8 ms with all of it kept,
 // 4.6 with 2 GiB, 6.7 with 1, 8.8 with none; 20,017 x 3,001, 1.2 GiB, 1.5, 1.5, 2.0, 4.0.)
 struct FewPool {
-    std::mutex mu;
     bool made = false;
-    unsigned long long context = 0;  // that the pool was made in
-    cudaMemPool_t pool = nullptr;    // null: not to be had
-    int users = 0;                   // handles that took from it
+    unsigned long long context = 0;
+    cudaMemPool_t pool = nullptr;  // null: not to be had
+    int users = 0;                 // handles that took from it
 };
-FewPool g_few_pool[64];
+std::mutex g_few_mu;
+// by device and context; never destroyed (a handle may outlive the statics)
+std::map<std::pair<int, unsigned long long>, FewPool> &g_few_pools = *new std::map<std::pair<int, unsigned long long>, FewPool>;
 constexpr size_t kFewKeep = (size_t)2 << 30;
 constexpr size_t kFewIdle = (size_t)32 << 20;
 
 cudaMemPool_t few_pool(mcd_dag *g, bool use) {
-    if (g->device < 0 || g->device >= 64) return nullptr;
-    FewPool &fp = g_few_pool[g->device];
-    std::lock_guard<std::mutex> lk(fp.mu);
     const unsigned long long context = current_context_id();
-    if (!fp.made || fp.context != context) {
+    std::lock_guard<std::mutex> lk(g_few_mu);
+    FewPool &fp = g_few_pools[{g->device, context}];
+    if (!fp.made) {
         fp.made = true;
         fp.context = context;
-        fp.pool = nullptr;
-        fp.users = 0;
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
@@ -603,18 +602,22 @@ cudaMemPool_t few_pool(mcd_dag *g, bool use) {
             cudaFreeAsync(p, g->stream[0]);
         (void)cudaGetLastError();
     }
-    if (use && fp.pool && !g->few_used.exchange(true)) {
-        g->few_context = context;
+    if (use && fp.pool && !g->few) {
+        g->few = &fp;
         ++fp.users;
     }
     return fp.pool;
 }
 
 void few_pool_leave(mcd_dag *g) {
-    if (!g->few_used.exchange(false)) return;
-    FewPool &fp = g_few_pool[g->device];
-    std::lock_guard<std::mutex> lk(fp.mu);
-    if (g->few_context == fp.context && --fp.users == 0 && cudaMemPoolTrimTo(fp.pool, kFewIdle) != cudaSuccess) (void)cudaGetLastError();
+    const unsigned long long context = current_context_id();
+    std::lock_guard<std::mutex> lk(g_few_mu);
+    FewPool *fp = static_cast<FewPool *>(g->few);
+    if (!fp) return;
+    g->few = nullptr;
+    // (a pool whose context is not the current one may be gone with it)
+    if (--fp->users == 0 && fp->context == context && cudaMemPoolTrimTo(fp->pool, kFewIdle) != cudaSuccess)
+        (void)cudaGetLastError();
 }
 
 // The same with device buffers (a: the launch's arguments, sample-minor rows).  The

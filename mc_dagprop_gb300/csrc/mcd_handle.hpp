@@ -3,7 +3,6 @@
 
 #include <cuda_runtime.h>
 
-#include <atomic>
 #include <memory>
 #include <mutex>
 #include <new>
@@ -69,8 +68,7 @@ struct mcd_dag {
     int32_t *d_err = nullptr;  // latched kernel errors of this handle's launches
     char *ws = nullptr;        // workspace
     size_t ws_bytes = 0;
-    std::atomic<bool> few_used{false};  // counted among the users of the device's few-sample scratch pool
-    unsigned long long few_context = 0; // and the context of that pool (both change under the pool's lock)
+    void *few = nullptr;       // the few-sample scratch pool it is counted a user of (under the pools' lock)
     int64_t last_adj_plan[3] = {0, 0, 0};  // the last gradient's samples per chunk, level blocks, buffer bytes
     explicit mcd_dag(std::shared_ptr<const mcd::DagImage> image)
         : img(std::move(image)), h(img->h), device(img->device), dbytes(img->dbytes), d_ev(img->d_ev),
