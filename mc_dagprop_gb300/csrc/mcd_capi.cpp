@@ -565,9 +565,8 @@ bool run_few(mcd_dag *g, const int64_t *seeds, const double *dur_in, int64_t n, 
 
 // Scratch of few-sample launches on callers' streams: one pool a device and context (it
 // goes with its context at a device reset), made with the first handle (so that no run
-// waits for it).  Between launches it keeps kFewKeep at most,
-// what is above goes back at the next synchronisation, and kFewIdle once no handle that
-// used it is left.  (What a launch has to take anew costs about a millisecond a GiB:
+// waits for it).  Between launches it keeps kFewKeep at most, what is above goes back at
+// the next synchronisation, and kFewIdle once no handle that used it is left.  (What a launch has to take anew costs about a millisecond a GiB:
 // 200,000 events x 608 samples, 2.4 GiB, waited for each time 3.8 ms with all of it kept,
 // 4.6 with 2 GiB, 6.7 with 1, 8.8 with none; 20,017 x 3,001, 1.2 GiB, 1.5, 1.5, 2.0, 4.0.)
 struct FewPool {
