@@ -91,16 +91,18 @@ static int create_batch(mcd_dag *const *dags, int32_t n_dags, const int64_t *see
         cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, B->device), "SM count");
         auto cost = [&](int32_t i) { return (double)B->dags[i]->h.pred.size() + 2.0 * B->dags[i]->h.E; };
         // Wide tiles pay where an SM has the work of several of the costliest tiles (a wide
-        // one takes 1.77 times as long, and the last of them set the end): three where a
-        // narrow CTA has its SM to itself; nine where several hide each other's barriers,
+        // one takes 1.77 times as long, and the last of them set the end): above three where a
+        // narrow CTA has its SM to itself (at three of one DAG, two rounds of wide tiles take
+        // 1,477 us where three of narrow ones take 1,344; one tile more, four rounds of narrow
+        // ones, 1,753); above nine where several hide each other's barriers,
         // and then only if many entries draw nothing, their cost being the records that
         // two samples share.  Measured (tiles of work an SM: narrow, wide): one
         // CTA an SM, 9.7: 29.2, 24.2 ms; several, half the entries fixed, 18: 20.9, 19.1;
         // a fifth of them fixed, 15: 9.7, 11.1; 32 networks of two delay types 45.8, 39.6,
         // of five 94.7, 94.9, by this rule 89.2.  Over 48 batches (2 to 24 networks of 20 to
         // 200 events a level, two and five types) the rule is within 1 % of narrow tiles where
-        // wide ones lose (three tiles of work, one CTA an SM: 1,427, 1,547 us; two networks:
-        // 557, 850) and takes or misses up to 1.26 where they win.
+        // wide ones lose (two networks: 557, 850 us) and takes or misses up to 1.26 where they
+        // win.
         double work = 0.0, most = 0.0, entries = 0.0, sampled = 0.0;
         size_t narrow_smem = 0;
         for (int32_t i = 0; i < n_dags; ++i) {
@@ -115,7 +117,7 @@ static int create_batch(mcd_dag *const *dags, int32_t n_dags, const int64_t *see
         const int64_t narrow_fit = std::min<int64_t>((228 * 1024) / ((int64_t)narrow_smem + 1024),
                                                      kMaxBatchWarps / std::max(1, B->n_warps));
         const double tiles_deep = work / (std::max(most, 1.0) * std::max(1, sms));
-        const bool wide_pays = may_be_wide && (narrow_fit <= 1 ? tiles_deep >= 3.0 : tiles_deep >= 9.0 && sampled < 0.65 * entries);
+        const bool wide_pays = may_be_wide && (narrow_fit <= 1 ? tiles_deep > 3.0 : tiles_deep > 9.0 && sampled < 0.65 * entries);
         // layout of the batch's device memory; launches by kernel variant
         B->ev_off.resize((size_t)n_dags + 1, 0);
         std::vector<int32_t> launch_of((size_t)n_dags);

@@ -38,3 +38,14 @@ def test_deep_batches_run_wide_tiles(cuda, n_warps):
         alone = batching.compile_dag(f, g, 0, "global").run_stats(n=n, seed0=i, hist=True)
         got = batch.stats(i, True)
         assert all(np.array_equal(alone[k], got[k]) for k in KEYS), i
+
+
+def test_whole_rounds_of_narrow_tiles_stay_narrow(cuda):
+    """Three 32-sample tiles an SM of one DAG take less time than two rounds of wide ones; a
+    tile more is a fourth round."""
+    import torch
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    prop = batching.compile_dag(*kitchen_sink(seed=40, n_layers=5, width=130), 24)
+    wide = [_core.Batch([prop], [0], [n]).plan["wide_dags"] for n in (96 * sms - 31, 96 * sms, 96 * sms + 1)]
+    assert wide == [0, 0, 1]
