@@ -224,13 +224,14 @@ __device__ __forceinline__ int pick_bin(const DistParam &p, const AliasPick *pic
 __device__ __forceinline__ double draw_empirical(const DistParam &p, const AliasEntry *alias, const AliasPick *picks,
                                                  const double *vt, double base, bool relative, uint32_t r,
                                                  uint32_t r2, bool two_word, float &dfac) {
+    const uint32_t j = __umulhi(r, (uint32_t)p.tab_n);
+    const uint32_t u = two_word ? r2 : r * (uint32_t)p.tab_n;
     if (vt) {
-        const int k = pick_bin(p, picks, r, r2, two_word);
+        const AliasPick pk = picks[p.tab_off + j];
+        const int k = u < pk.thresh ? (int)j : pk.alias;
         dfac = relative ? 1.0f + (float)alias[p.tab_off + k].v_self : 1.0f;
         return vt[k];
     }
-    const uint32_t j = __umulhi(r, (uint32_t)p.tab_n);
-    const uint32_t u = two_word ? r2 : r * (uint32_t)p.tab_n;
     const AliasEntry &e = alias[p.tab_off + j];
     const double val = u < e.thresh ? e.v_self : e.v_alias;
     dfac = relative ? 1.0f + (float)val : 1.0f;
@@ -503,6 +504,13 @@ __device__ __forceinline__ T *at_row(T *col, int32_t row, uint32_t ld_bytes) {
     using Byte = std::conditional_t<std::is_const<T>::value, const char, char>;
     return reinterpret_cast<T *>(reinterpret_cast<Byte *>(col) + (uint64_t)(uint32_t)row * ld_bytes);
 }
+// The same by integer arithmetic, for the sampled kernel: its loops compile to 1-2 % less
+// time so (5,600 events x 4,864 samples 339.9 -> 334.6 us, 200,000 x 9,728 21.5 -> 21.3 ms),
+// those of given durations and of few samples to 3 and 2 % more (9.57 -> 9.90 ms).
+template <typename T>
+__device__ __forceinline__ T *row_at(T *col, int32_t row, uint32_t ld_bytes) {
+    return reinterpret_cast<T *>(reinterpret_cast<uintptr_t>(col) + (uint64_t)(uint32_t)row * ld_bytes);
+}
 
 // The window row of a slot word (PredRec::src_slot, EvRec::slot): the low half for
 // tiles of 32 samples, the high half, signed, for wide tiles (negative: no row on
@@ -547,7 +555,7 @@ __device__ __forceinline__ int take_next(uint32_t ctr) {
 // tile's predecessor without one (see window_row) from its off-chip window row
 // or, where the realized times are an output, from that; window off chip: from
 // the realized rows.
-template <bool WIN_SMEM, int S>
+template <bool WIN_SMEM, int S, bool GIVEN>
 __device__ __forceinline__ void source(const TileCtx<S> &t, const double *win, int32_t slots, int32_t user,
                                        double (&v)[S]) {
     if (WIN_SMEM) {
@@ -563,7 +571,7 @@ __device__ __forceinline__ void source(const TileCtx<S> &t, const double *win, i
             return;
         }
     }
-    const double *row = at_row(t.rcol, user, t.rows_ld8);
+    const double *row = GIVEN ? at_row(t.rcol, user, t.rows_ld8) : row_at(t.rcol, user, t.rows_ld8);
 #pragma unroll
     for (int j = 0; j < S; ++j) v[j] = t.active[j] ? row[32 * j] : 0.0;
 }
@@ -663,7 +671,7 @@ __device__ __forceinline__ void stage_given(const KArgs &a, const EvRec *sev, co
         };
         auto entry = [&](int4 rec, const double (&dur)[S]) {
             double src[S];
-            source<WIN_SMEM, S>(t, win, rec.x, rec.y, src);
+            source<WIN_SMEM, S, true>(t, win, rec.x, rec.y, src);
             relaxed(src, dur, rec.y);
         };
         // entries p to p + kGivenAhead - 1; sources that lie off chip are read together
@@ -672,7 +680,7 @@ __device__ __forceinline__ void stage_given(const KArgs &a, const EvRec *sev, co
             double src[kGivenAhead][S];
 #pragma unroll
             for (int k = 0; k < kGivenAhead; ++k)
-                if (p + k < np) source<WIN_SMEM, S>(t, win, recs[2 * k].x, recs[2 * k].y, src[k]);
+                if (p + k < np) source<WIN_SMEM, S, true>(t, win, recs[2 * k].x, recs[2 * k].y, src[k]);
 #pragma unroll
             for (int k = 0; k < kGivenAhead; ++k)
                 if (p + k < np) relaxed(src[k], dur[k], recs[2 * k].y);
@@ -795,16 +803,16 @@ __device__ __forceinline__ void stage_events(const KArgs &a, int buf, const EvRe
             const PredRec pr = load_pred(spred + p);
             double src[S], dur[S];
             float dfac[S];
-            if (S > 1) source<WIN_SMEM, S>(t, win, pr.src_slot, pr.src_user, src);  // (may come from L2: ahead of the draws)
+            if (S > 1) source<WIN_SMEM, S, false>(t, win, pr.src_slot, pr.src_user, src);  // (may come from L2: ahead of the draws)
             link_duration<STAGED, TS, S>(a, pr.kd, pr.v, pr.dvo, (uint32_t)pr.block, (uint32_t)pr.link, t.seed, grp, smem,
                                          buf, dur, dfac);
             if (!STATS && !ADJ && (pr.kd & KD_WRITE) && t.dcol) {
-                double *row = at_row(t.dcol, pr.link, t.ld8);
+                double *row = row_at(t.dcol, pr.link, t.ld8);
 #pragma unroll
                 for (int j = 0; j < S; ++j)
                     if (j == 0 || t.active[j]) row[32 * j] = dur[j];
             }
-            if (S == 1) source<WIN_SMEM, S>(t, win, pr.src_slot, pr.src_user, src);
+            if (S == 1) source<WIN_SMEM, S, false>(t, win, pr.src_slot, pr.src_user, src);
 #pragma unroll
             for (int j = 0; j < S; ++j) {
                 bool clamp;
@@ -850,13 +858,13 @@ __device__ __forceinline__ void stage_events(const KArgs &a, int buf, const EvRe
             }
         }
         if (t.rcol && t.active[0]) {
-            double *row = at_row(t.rcol, ev.user, t.rows_ld8);
+            double *row = row_at(t.rcol, ev.user, t.rows_ld8);
 #pragma unroll
             for (int j = 0; j < S; ++j)
                 if (j == 0 || t.active[j]) row[32 * j] = __longlong_as_double(lbits[j]);
         }
         if (!STATS && !ADJ && t.ccol) {
-            int32_t *row = at_row(t.ccol, ev.user, t.ld4);
+            int32_t *row = row_at(t.ccol, ev.user, t.ld4);
 #pragma unroll
             for (int j = 0; j < S; ++j)
                 if (j == 0 || t.active[j]) row[32 * j] = cause[j];
@@ -1033,7 +1041,7 @@ __device__ __forceinline__ bool propagate_tile(const KArgs &a, int64_t tile, dou
             link_duration<false, TS, S>(a, lr.kd, lr.v, -1, (uint32_t)lr.link, (uint32_t)lr.link, t.seed, own, smem, 0, dur,
                                         dfac);
             if (t.dcol) {
-                double *row = at_row(t.dcol, lr.link, t.ld8);
+                double *row = row_at(t.dcol, lr.link, t.ld8);
 #pragma unroll
                 for (int j = 0; j < S; ++j)
                     if (j == 0 || t.active[j]) row[32 * j] = dur[j];
