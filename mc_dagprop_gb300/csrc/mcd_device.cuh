@@ -504,9 +504,10 @@ __device__ __forceinline__ T *at_row(T *col, int32_t row, uint32_t ld_bytes) {
     using Byte = std::conditional_t<std::is_const<T>::value, const char, char>;
     return reinterpret_cast<T *>(reinterpret_cast<Byte *>(col) + (uint64_t)(uint32_t)row * ld_bytes);
 }
-// The same by integer arithmetic, for the sampled kernel: its loops compile to 1-2 % less
-// time so (5,600 events x 4,864 samples 339.9 -> 334.6 us, 200,000 x 9,728 21.5 -> 21.3 ms),
-// those of given durations and of few samples to 3 and 2 % more (9.57 -> 9.90 ms).
+// The same by integer arithmetic, for the sampled kernel and the grouped forms of given
+// durations: their loops compile to 1-2 and 3 % less time so (5,600 events x 4,864 samples
+// 339.9 -> 334.6 us, 200,000 x 9,728 21.5 -> 21.3 ms), those that read given durations
+// ahead and those of few samples to 3 and 2 % more (9.57 -> 9.90 ms).
 template <typename T>
 __device__ __forceinline__ T *row_at(T *col, int32_t row, uint32_t ld_bytes) {
     return reinterpret_cast<T *>(reinterpret_cast<uintptr_t>(col) + (uint64_t)(uint32_t)row * ld_bytes);
@@ -555,7 +556,7 @@ __device__ __forceinline__ int take_next(uint32_t ctr) {
 // tile's predecessor without one (see window_row) from its off-chip window row
 // or, where the realized times are an output, from that; window off chip: from
 // the realized rows.
-template <bool WIN_SMEM, int S, bool GIVEN>
+template <bool WIN_SMEM, int S, bool AHEAD>
 __device__ __forceinline__ void source(const TileCtx<S> &t, const double *win, int32_t slots, int32_t user,
                                        double (&v)[S]) {
     if (WIN_SMEM) {
@@ -571,7 +572,7 @@ __device__ __forceinline__ void source(const TileCtx<S> &t, const double *win, i
             return;
         }
     }
-    const double *row = GIVEN ? at_row(t.rcol, user, t.rows_ld8) : row_at(t.rcol, user, t.rows_ld8);
+    const double *row = AHEAD ? at_row(t.rcol, user, t.rows_ld8) : row_at(t.rcol, user, t.rows_ld8);
 #pragma unroll
     for (int j = 0; j < S; ++j) v[j] = t.active[j] ? row[32 * j] : 0.0;
 }
@@ -601,23 +602,29 @@ __device__ __forceinline__ bool relax(double src, double dur, long long ub_key, 
 }
 
 // One stage's events under given durations, one at a time from the stage's counter
-// (no draws, so no pairs).  The durations are uncached DRAM reads: an event's first
-// kGivenAhead entries are read while the event before it runs.  Without the sampler the
-// kernel runs at 64 registers (those of wide tiles spill 64 bytes), so 32 warps an SM.
-// 200,000 events x 4,864 samples: reads four at a time when reached, 24 warps 13.2 ms
-// (2.3 TB/s); one event ahead, 32 warps 9.6 (3.2 TB/s).  20,017 events x 3,001
-// samples 3.5 -> 1.30 ms.  Prefetching the next stage's rows into L2 gained 2 %.
-// LONG: events of many predecessors, whose later entries are read kGivenAhead together
-// (one by one, each waits for DRAM: 4,000 events of 12.5 predecessors x 4,864 samples at
-// 8 warps 3,160 us, together 2,190; of 2.5, where the other form's registers serve
-// better, 503 against 460).  With the window off chip the sources are L2 reads, and read
-// together too (4,000 events of 2.5, 8 warps 681 -> 603 us); LONG then reads nothing
-// ahead, for want of registers (of 12.5: 2,900 -> 2,190; reading ahead as well spilled,
-// 2,830, and 1,415 against 884 of 4.5).
+// (no draws, so no pairs).  Large runs wait for DRAM at every duration.  Three forms
+// (launch_prop_given chooses):
+//   ahead  an event's first kGivenAhead entries are read while the event before it runs,
+//          later ones as they are reached.  Without the sampler the kernel runs at 64
+//          registers (those of wide tiles spill 64 bytes), so 32 warps an SM.  200,000
+//          events x 4,864 samples: reads four at a time when reached, 24 warps 13.2 ms
+//          (2.3 TB/s); one event ahead, 32 warps 9.6 (3.2 TB/s).  20,017 events x 3,001
+//          samples 3.5 -> 1.30 ms.  Prefetching the next stage's rows into L2 gained 2 %.
+//   groups entries are read kGivenAhead together as they are reached, their sources, with
+//          the window off chip, as well: for long lists, whose later entries would each
+//          wait (4,000 events of 6.5 predecessors x 4,864 samples at 8 warps 1,317 us,
+//          in groups 1,065), and for windows off chip (of 2.5: 596 us, in groups 572)
+//   hot    the same for durations that L2 holds, as a caller's that were just written or
+//          are propagated again do: loads that stay there (evict-first ones of 32 to 90 MB
+//          take up to 1.5 times as long, larger ones 2 % less), nothing ahead and sources
+//          one by one (sources together 1.15 times as long): 2,000 events x 1,000 samples
+//          in levels of 50 at 8 warps 197 us, ahead 228.
 constexpr int kGivenAhead = 4;
-template <bool WIN_SMEM, int S, bool LONG>
+enum : int { kGivenAheadOnce = 0, kGivenGroups = 1, kGivenGroupsHot = 2 };
+template <bool WIN_SMEM, int S, int FORM>
 __device__ __forceinline__ void stage_given(const KArgs &a, const EvRec *sev, const PredRec *spred, int pred0, int n_ev,
                                             uint32_t ctr, const TileCtx<S> &t, unsigned char *smem) {
+    constexpr bool kAhead = FORM == kGivenAheadOnce;
     double *win = reinterpret_cast<double *>(smem);
     auto take = [&]() {
         int i = 0;
@@ -628,12 +635,11 @@ __device__ __forceinline__ void stage_given(const KArgs &a, const EvRec *sev, co
 #pragma unroll
         for (int j = 0; j < S; ++j) d[j] = 0.0;
         if (link < 0) return;
-        const double *row = at_row(t.dincol, link, t.ld_in8);
+        const double *row = kAhead ? at_row(t.dincol, link, t.ld_in8) : row_at(t.dincol, link, t.ld_in8);
 #pragma unroll
         for (int j = 0; j < S; ++j)
-            if (t.active[j]) d[j] = __ldcs(row + 32 * j);
+            if (t.active[j]) d[j] = FORM == kGivenGroupsHot ? __ldg(row + 32 * j) : __ldcs(row + 32 * j);
     };
-    constexpr bool kAhead = WIN_SMEM || !LONG;
     auto read = [&](int i, double (&d)[kGivenAhead][S]) {
         if (!kAhead || i >= n_ev) return;
         const int4 e = reinterpret_cast<const int4 *>(sev + i)[0];  // user, slot, pred_begin, pred_end
@@ -650,7 +656,9 @@ __device__ __forceinline__ void stage_given(const KArgs &a, const EvRec *sev, co
         for (int k = 0; k < kGivenAhead; ++k)
 #pragma unroll
             for (int j = 0; j < S; ++j) d[k][j] = d_next[k][j];
-        i_next = take();
+        int later = 0;  // (taken ahead, read at the end: its latency hides behind the event)
+        if constexpr (kAhead) i_next = take();
+        else if (t.lane == 0) later = take_next(ctr);
         read(i_next, d_next);
         const EvRec ev = load_ev(sev + i);
         long long lk[S], lbits[S];
@@ -671,16 +679,16 @@ __device__ __forceinline__ void stage_given(const KArgs &a, const EvRec *sev, co
         };
         auto entry = [&](int4 rec, const double (&dur)[S]) {
             double src[S];
-            source<WIN_SMEM, S, true>(t, win, rec.x, rec.y, src);
+            source<WIN_SMEM, S, kAhead>(t, win, rec.x, rec.y, src);
             relaxed(src, dur, rec.y);
         };
-        // entries p to p + kGivenAhead - 1; sources that lie off chip are read together
+        // entries p to p + kGivenAhead - 1, their sources read together
         auto entries = [&](int p, const double (&dur)[kGivenAhead][S]) {
             const int4 *recs = reinterpret_cast<const int4 *>(spred + pb + p);
             double src[kGivenAhead][S];
 #pragma unroll
             for (int k = 0; k < kGivenAhead; ++k)
-                if (p + k < np) source<WIN_SMEM, S, true>(t, win, recs[2 * k].x, recs[2 * k].y, src[k]);
+                if (p + k < np) source<WIN_SMEM, S, kAhead>(t, win, recs[2 * k].x, recs[2 * k].y, src[k]);
 #pragma unroll
             for (int k = 0; k < kGivenAhead; ++k)
                 if (p + k < np) relaxed(src[k], dur[k], recs[2 * k].y);
@@ -691,27 +699,18 @@ __device__ __forceinline__ void stage_given(const KArgs &a, const EvRec *sev, co
 #pragma unroll
                 for (int k = 0; k < kGivenAhead; ++k)
                     if (p + k < np) duration(reinterpret_cast<const int4 *>(spred + pb + p + k)->z, now[k]);
-                entries(p, now);
+                if constexpr (!WIN_SMEM && FORM != kGivenGroupsHot) {
+                    entries(p, now);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < kGivenAhead; ++k)
+                        if (p + k < np) entry(reinterpret_cast<const int4 *>(spred + pb + p + k)[0], now[k]);
+                }
             }
-        } else if constexpr (!WIN_SMEM) {
-            entries(0, d);
         } else {
 #pragma unroll
             for (int k = 0; k < kGivenAhead; ++k)
                 if (k < np) entry(reinterpret_cast<const int4 *>(spred + pb + k)[0], d[k]);
-        }
-        if constexpr (LONG && kAhead) {
-            for (int p = kGivenAhead; p < np; p += kGivenAhead) {
-                const int4 *recs = reinterpret_cast<const int4 *>(spred + pb + p);
-                double rest[kGivenAhead][S];
-#pragma unroll
-                for (int k = 0; k < kGivenAhead; ++k)
-                    if (p + k < np) duration(recs[2 * k].z, rest[k]);
-#pragma unroll
-                for (int k = 0; k < kGivenAhead; ++k)
-                    if (p + k < np) entry(recs[2 * k], rest[k]);
-            }
-        } else if constexpr (!LONG) {
             for (int k = kGivenAhead; k < np; ++k) {
                 const int4 rec = reinterpret_cast<const int4 *>(spred + pb + k)[0];
                 double dur[S];
@@ -730,17 +729,18 @@ __device__ __forceinline__ void stage_given(const KArgs &a, const EvRec *sev, co
             }
         }
         if (t.rcol && t.active[0]) {
-            double *row = at_row(t.rcol, ev.user, t.rows_ld8);
+            double *row = kAhead ? at_row(t.rcol, ev.user, t.rows_ld8) : row_at(t.rcol, ev.user, t.rows_ld8);
 #pragma unroll
             for (int j = 0; j < S; ++j)
                 if (j == 0 || t.active[j]) row[32 * j] = __longlong_as_double(lbits[j]);
         }
         if (t.ccol) {
-            int32_t *row = at_row(t.ccol, ev.user, t.ld4);
+            int32_t *row = kAhead ? at_row(t.ccol, ev.user, t.ld4) : row_at(t.ccol, ev.user, t.ld4);
 #pragma unroll
             for (int j = 0; j < S; ++j)
                 if (j == 0 || t.active[j]) row[32 * j] = cause[j];
         }
+        if constexpr (!kAhead) i_next = __shfl_sync(0xFFFFFFFFu, later, 0);
     }
 }
 
@@ -904,7 +904,7 @@ __device__ __forceinline__ void stage_events(const KArgs &a, int buf, const EvRe
 // a.blk_start stages begins -- the checkpoints a level-block recomputation
 // starts from.
 template <bool GIVEN, bool WIN_SMEM, bool STATS, bool POSITIVE, bool ADJ = false, int TS = kTablesEither,
-          bool LANE_HIST = true, int S = 1, bool LONG = false>
+          bool LANE_HIST = true, int S = 1, int FORM = kGivenAheadOnce>
 __device__ __forceinline__ bool propagate_tile(const KArgs &a, int64_t tile, double *rows, int64_t rows_ld,
                                                bool rows_tile_local, unsigned char *smem, uint64_t *bars,
                                                bool reuse, double *spill = nullptr) {
@@ -1014,7 +1014,7 @@ __device__ __forceinline__ bool propagate_tile(const KArgs &a, int64_t tile, dou
         if (meta.y >= 0) {  // records in the staging buffer (shared memory)
             const unsigned char *buf = smem + a.smem_stage_off + b * a.stage_bytes;
             if constexpr (GIVEN)
-                stage_given<WIN_SMEM, S, LONG>(a, reinterpret_cast<const EvRec *>(buf), reinterpret_cast<const PredRec *>(buf + mv.z),
+                stage_given<WIN_SMEM, S, FORM>(a, reinterpret_cast<const EvRec *>(buf), reinterpret_cast<const PredRec *>(buf + mv.z),
                                          meta.z, meta.y, ctr, t, smem);
             else
                 stage_events<WIN_SMEM, STATS, POSITIVE, ADJ, true, TS, LANE_HIST, S>(
@@ -1022,7 +1022,7 @@ __device__ __forceinline__ bool propagate_tile(const KArgs &a, int64_t tile, dou
                 meta.x, meta.y, n_pair, ctr, t, smem, grp);
         } else {  // a stage whose records exceed the buffer is read from global memory
             if constexpr (GIVEN)
-                stage_given<WIN_SMEM, S, LONG>(a, a.ev + meta.x, a.pred + meta.z, meta.z, -meta.y, ctr, t, smem);
+                stage_given<WIN_SMEM, S, FORM>(a, a.ev + meta.x, a.pred + meta.z, meta.z, -meta.y, ctr, t, smem);
             else
                 stage_events<WIN_SMEM, STATS, POSITIVE, ADJ, false, TS, LANE_HIST, S>(
                 a, b, a.ev + meta.x, a.pred + meta.z, meta.z, meta.x, -meta.y, n_pair, ctr, t, smem, grp);
@@ -1065,10 +1065,10 @@ __global__ void __launch_bounds__(768, 1) k_propagate(const KArgs a) {
 
 // The same with given durations (a.dur_in), which may be anything.
 constexpr int kGivenWarps = 32;  // most warps of a CTA, and of an SM (64 registers a thread)
-template <bool WIN_SMEM, int S, bool LONG>
+template <bool WIN_SMEM, int S, int FORM>
 __global__ void __launch_bounds__(kGivenWarps * 32, 1) k_propagate_given(const KArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
-    propagate_tile<true, WIN_SMEM, false, false, false, kTablesEither, true, S, LONG>(
+    propagate_tile<true, WIN_SMEM, false, false, false, kTablesEither, true, S, FORM>(
         a, (int64_t)blockIdx.x, a.realized ? a.realized : a.scratch, a.ld, false, smem,
         reinterpret_cast<uint64_t *>(smem + a.smem_bar_off), false);
 }
